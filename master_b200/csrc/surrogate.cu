@@ -15,7 +15,10 @@
 //   dgrad:    the forward kernel on the flipped, transposed weights
 //             Wd[ci][tap][co] = W[co][26 - tap][ci]
 //   wgrad:    D[(tap,co)][ci] = sum_u dY[u - off(tap)][co] X[u][ci]
-// M tiles of 128 rows, operands staged in shared memory by cp.async in a
+// Edges of 16 and more (every layer of the network on boxes of 64 and more)
+// take conv_plane.cuh forward, which stages each voxel plane once; the kernels
+// here serve smaller edges, other channel counts and the weight gradient: M tiles of
+// 128 rows, operands gathered tap by tap in shared memory by cp.async in a
 // three-stage ring, one elected thread issuing the MMAs, completion tracked
 // by tcgen05.commit on an mbarrier per stage.  The epilogue (bias, ReLU, the
 // ReLU mask of a gradient, bf16 rounding) runs on the TMEM read-back.
@@ -42,6 +45,12 @@ constexpr int kRowBytes = 16;
 constexpr int kATileBytes = kChunks * 128 * kRowBytes;  // 128 rows
 
 __device__ unsigned g_error;  // set when a bounded wait ran out
+
+}  // namespace sg
+
+#include "conv_plane.cuh"
+
+namespace sg {
 
 struct Vol {
     const bf16 *p;
@@ -763,6 +772,59 @@ int grid_for(long long n, int block) {
     return (int)(g < 1 ? 1 : g);
 }
 
+int sm_count() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+// The plane kernels' tiles are 16 x 8 voxels.
+constexpr int kPlaneEdge = 16;
+
+// Output channels per CTA and planes per item of conv_plane_kernel: the split
+// with the least estimated time, in cycles of an SM.  A plane costs the
+// largest of its MMAs (32 cycles to read A, or N / 2), its staged bytes and
+// its epilogue; an item stages two planes more than it writes; every CTA
+// loads its weights once.
+template <int CIN> void plane_split(PlaneArgs &a, int cout, long long rows, int sms) {
+    const long long tiles = rows >> (a.lg + 7);
+    double best = 1e300;
+    for (int nb = 16; nb <= PlaneShape<CIN>::kMaxNb; nb += 16) {
+        if (cout % nb) continue;
+        const int nsplit = cout / nb;
+        for (int lgL = 0; lgL <= a.lg; ++lgL) {
+            const long long items = tiles << (a.lg - lgL);
+            const long long ctas = std::max(1ll, std::min<long long>(items, sms / nsplit));
+            const double mma = 9.0 * (CIN / 16) * std::max(32.0, 1.5 * nb);
+            const double plane = std::max(std::max(mma, kHalo * CIN * 2 / 25.0), 16.0 * nb);
+            const double t = (double)((items + ctas - 1) / ctas) * (((1 << lgL) + 2) * plane + 300.0) + 27.0 * CIN * nb * 2 / 40.0;
+            if (t < best) {
+                best = t;
+                a.nb = nb;
+                a.nsplit = nsplit;
+                a.lgL = lgL;
+                a.items = (int)items;
+            }
+        }
+    }
+}
+
+template <int CIN> cudaError_t launch_conv_plane(const ConvArgs &c, int cout, cudaStream_t st) {
+    using Sh = PlaneShape<CIN>;
+    PlaneArgs a{c.in.p, c.in.cs, c.in.coff, c.w, c.bias, c.out.p, c.out.cs, c.out.coff, c.mask.p, c.mask.cs, c.mask.coff,
+                c.relu, c.S, c.lg, 0, 0, 0, 0};
+    const int sms = sm_count();
+    plane_split<CIN>(a, cout, c.rows, sms);
+    const int smem = Sh::smem(a.nb);
+    cudaError_t e = cudaFuncSetAttribute(conv_plane_kernel<CIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         Sh::smem(Sh::kMaxNb));
+    if (e != cudaSuccess) return e;
+    const int grid = (int)std::min<long long>(a.items, std::max(1, sms / a.nsplit)) * a.nsplit;
+    conv_plane_kernel<CIN><<<grid, kPlaneThreads, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
 template <int N> cudaError_t launch_conv(const ConvArgs &a, cudaStream_t st) {
     using Sh = ConvShape<N>;
     cudaError_t e = cudaFuncSetAttribute(conv3_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem);
@@ -853,6 +915,16 @@ int dsmc_sg_conv3(void *stream, int batch, int S, const uint16_t *in, int in_cs,
     a.lg = lg;
     a.rows = (long long)batch << (3 * lg);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (S >= kPlaneEdge && (cout == 16 || cout == 32 || cout == 48 || cout == 64 || cout == 96)) {
+        switch (cin) {
+        case 16: return cuda_rc(launch_conv_plane<16>(a, cout, st));
+        case 32: return cuda_rc(launch_conv_plane<32>(a, cout, st));
+        case 48: return cuda_rc(launch_conv_plane<48>(a, cout, st));
+        case 64: return cuda_rc(launch_conv_plane<64>(a, cout, st));
+        case 96: return cuda_rc(launch_conv_plane<96>(a, cout, st));
+        default: break;
+        }
+    }
     switch (cout) {
     case 16: return cuda_rc(launch_conv<16>(a, st));
     case 32: return cuda_rc(launch_conv<32>(a, st));

@@ -87,6 +87,40 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(z), "r"(z), "r"(z), "r"(z)
         : "memory");
 }
+// One lane of the (converged) warp: 1 in it, 0 in the others.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t lead;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(lead));
+    return lead;
+}
+// mma_bf16 and mma_commit for a whole warp in step, issued by the lane with
+// lead != 0: the operands are then the same in every lane and the issue is
+// predicated, not branched.  The descriptors come as their low words (address
+// and leading offset) and common high words.
+__device__ __forceinline__ void mma_bf16_warp(uint32_t lead, uint32_t tmem_d, uint32_t alo, uint32_t ahi, uint32_t blo,
+                                              uint32_t bhi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 q, %0, 0;\n\t"
+        "setp.ne.b32 p, %7, 0;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 b, {%4, %5};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %6, p;\n\t}\n" ::"r"(lead),
+        "r"(tmem_d), "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit_warp(uint32_t lead, uint64_t *mbar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %0, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}\n" ::"r"(lead),
+        "r"(smem_u32(mbar))
+        : "memory");
+}
 // The mbarrier receives one arrival when every MMA this thread issued before
 // has completed (their shared-memory reads and TMEM writes are done).
 __device__ __forceinline__ void mma_commit(uint64_t *mbar) {
@@ -115,6 +149,9 @@ __device__ __forceinline__ void mbar_init(uint64_t *mbar, uint32_t count) {
 }
 __device__ __forceinline__ void mbar_fence_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t *mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *mbar, uint32_t parity) {
     uint32_t ok;
@@ -145,7 +182,13 @@ __device__ __forceinline__ void cp_async16_zfill(void *smem_dst, const void *gsr
                  "r"(src_bytes)
                  : "memory");
 }
+// The mbarrier receives this thread's arrival once every cp.async it issued
+// before has landed (the arrival is part of the barrier's count).
+__device__ __forceinline__ void cp_async_arrive(uint64_t *mbar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(mbar)) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }

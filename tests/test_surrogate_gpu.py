@@ -167,6 +167,47 @@ def test_conv_weight_gradient_matches_torch(cin, cout):
     assert rel_l2(db.cpu().numpy(), b.grad.numpy()) <= 1e-4
 
 
+@pytest.mark.parametrize("B,S,cin,cout", [(1, 16, 16, 16), (3, 16, 96, 96), (1, 16, 64, 48), (1, 32, 48, 64), (3, 32, 16, 96),
+                                          (1, 64, 32, 32), (1, 64, 48, 16), (2, 8, 48, 32)])
+def test_conv_edges_of_the_plane_kernels(B, S, cin, cout):
+    """Forward, masked input gradient and weight gradient at the smallest edge
+    of the plane kernels (16: one tile line block, every halo wraps), odd
+    batches, several planes per tile, each accumulator ring (16, 32 and 48
+    channels per block) past its first lap, and the edge below (8: the
+    per-tap kernels).  bf16 results are held to the rounding of the output
+    (2^-8) plus fp32 summation, as the module's other tests."""
+    g = torch.Generator().manual_seed(1000 * S + cin + cout)
+    x = rnd_bf16((B, S, S, S, cin), g)
+    dy = rnd_bf16((B, S, S, S, cout), g)
+    w32 = torch.randn((cout, 27, cin), generator=g) * (2.0 / (27 * cin)) ** 0.5
+    bias = torch.randn(cout, generator=g) * 0.1
+    wf = torch.empty(cout * 27 * cin, dtype=torch.int16, device=DEV)
+    wd = torch.empty_like(wf)
+    d_w32, d_x, d_dy, d_b = w32.to(DEV), x.to(DEV), dy.to(DEV), bias.to(DEV)
+    y = torch.zeros((B, S, S, S, cout), dtype=torch.bfloat16, device=DEV)
+    dx = torch.zeros((B, S, S, S, cin), dtype=torch.bfloat16, device=DEV)
+    dw = torch.zeros((cout, 27, cin), device=DEV)
+    L = lib()
+    capi.check(L.dsmc_sg_pack_weights(stream(), P(d_w32), cout, cin, P(wf), P(wd)))
+    capi.check(L.dsmc_sg_conv3(stream(), B, S, P(d_x), cin, 0, cin, P(wf), P(d_b), cout, P(y), cout, 0, 1, None, 0, 0))
+    capi.check(L.dsmc_sg_conv3(stream(), B, S, P(d_dy), cout, 0, cout, P(wd), None, cin, P(dx), cin, 0, 0, P(d_x), cin,
+                               0))
+    capi.check(L.dsmc_sg_conv3_wgrad(stream(), B, S, P(d_dy), cout, 0, cout, P(d_x), cin, 0, cin, P(dw)))
+    sync_ok()
+    # fp64 on the GPU, tap by tap (the network's largest layers take torch's CPU operator minutes)
+    xd, dyd, wb = d_x.double(), d_dy.double(), d_w32.to(torch.bfloat16).double()
+    ry, rdx, rdw = d_b.double().expand(B, S, S, S, cout).clone(), torch.zeros_like(xd), torch.zeros_like(wb)
+    for t in range(27):
+        off = (t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1)
+        ry += torch.roll(xd, tuple(-o for o in off), (1, 2, 3)) @ wb[:, t].T
+        back = torch.roll(dyd, off, (1, 2, 3))
+        rdx += back @ wb[:, t]
+        rdw[:, t] = back.reshape(-1, cout).T @ xd.reshape(-1, cin)
+    close_bf16(y, torch.relu(ry).cpu())
+    close_bf16(dx, (rdx * (xd > 0)).cpu())
+    assert rel_l2(dw.cpu().numpy(), rdw.cpu().numpy()) <= 1e-4
+
+
 def test_pool_and_upsample_forward_and_backward():
     g = torch.Generator().manual_seed(11)
     B, S, Cc = 2, 16, 32
