@@ -16,8 +16,8 @@
 //             Wd[ci][tap][co] = W[co][26 - tap][ci]
 //   wgrad:    D[(tap,co)][ci] = sum_u dY[u - off(tap)][co] X[u][ci]
 // Edges of 16 and more (every layer of the network on boxes of 64 and more)
-// take conv_plane.cuh forward, which stages each voxel plane once; the kernels
-// here serve smaller edges, other channel counts and the weight gradient: M tiles of
+// take conv_plane.cuh and wgrad_plane.cuh, which stage each voxel plane once;
+// the kernels here serve smaller edges and other channel counts: M tiles of
 // 128 rows, operands gathered tap by tap in shared memory by cp.async in a
 // three-stage ring, one elected thread issuing the MMAs, completion tracked
 // by tcgen05.commit on an mbarrier per stage.  The epilogue (bias, ReLU, the
@@ -49,6 +49,7 @@ __device__ unsigned g_error;  // set when a bounded wait ran out
 }  // namespace sg
 
 #include "conv_plane.cuh"
+#include "wgrad_plane.cuh"
 
 namespace sg {
 
@@ -825,6 +826,54 @@ template <int CIN> cudaError_t launch_conv_plane(const ConvArgs &c, int cout, cu
     return cudaGetLastError();
 }
 
+// Voxels per CTA of wgrad_kernel: about four CTAs per SM over all M tiles, at
+// least 512 voxels each.
+long long wgrad_voxels(const WgradArgs &a) {
+    const int mtiles = (27 * a.cout + 127) / 128;
+    long long per = (a.rows * mtiles) / (148 * 4);
+    per = ((per + 63) / 64) * 64;
+    if (per < 512) per = 512;
+    return std::min(per, a.rows);
+}
+
+// One launch over the input channels [ci0, ci0 + ciblocks * CIB).
+template <int CIB> cudaError_t launch_wgrad_plane(const WgradArgs &w, int ci0, int ciblocks, cudaStream_t st) {
+    using Sh = PlaneWgradShape<CIB>;
+    PlaneWgradArgs a{w.dy.p, w.dy.cs, w.dy.coff, w.x.p, w.x.cs, w.x.coff, w.dw, w.cin, ci0, ciblocks,
+                     0, 0, w.S, w.lg, 0, 0, 1};
+    const int sms = sm_count();
+    // an accumulator takes as many additions of 16 voxels as wgrad_kernel's
+    // would: more would cost precision, fewer cost flushes
+    const long long adds = wgrad_voxels(w) / 16;
+    // the widest block of output channels, unless a CTA would then see far
+    // fewer additions where they are many and the fp32 sums' rounding counts
+    for (a.cob = 48; a.cob > 16; a.cob -= 16)
+        if (w.cout % a.cob == 0 &&
+            (adds < 1500 || w.rows / 16 / std::max(1, sms / (ciblocks * (w.cout / a.cob))) >= adds * 3 / 4))
+            break;
+    a.coblocks = w.cout / a.cob;
+    const int groups = ciblocks * a.coblocks;
+    const int ctas = std::max(1, sms / groups);
+    // planes per item: 16, fewer while items are short of two per CTA
+    const long long tiles = w.rows >> (w.lg + 7);
+    a.lgL = std::min(4, w.lg);
+    while (a.lgL > 1 && (tiles << (w.lg - a.lgL)) < 2 * ctas) --a.lgL;
+    a.items = (int)(tiles << (w.lg - a.lgL));
+    a.flush = (int)std::max(1ll, adds / (8 << a.lgL));
+    cudaError_t e = cudaFuncSetAttribute(wgrad_plane_kernel<CIB>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::smem(48));
+    if (e != cudaSuccess) return e;
+    const int grid = (int)std::min<long long>(a.items, ctas) * groups;
+    wgrad_plane_kernel<CIB><<<grid, kPlaneThreads, Sh::smem(a.cob), st>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_wgrad_planes(const WgradArgs &w, cudaStream_t st) {
+    const int b32 = w.cin / 32;
+    cudaError_t e = b32 ? launch_wgrad_plane<32>(w, 0, b32, st) : cudaSuccess;
+    if (e == cudaSuccess && w.cin % 32) e = launch_wgrad_plane<16>(w, 32 * b32, 1, st);
+    return e;
+}
+
 template <int N> cudaError_t launch_conv(const ConvArgs &a, cudaStream_t st) {
     using Sh = ConvShape<N>;
     cudaError_t e = cudaFuncSetAttribute(conv3_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem);
@@ -851,11 +900,7 @@ template <int N> cudaError_t launch_wgrad(const WgradArgs &a0, cudaStream_t st) 
     if (e != cudaSuccess) return e;
     WgradArgs a = a0;
     const int mtiles = (27 * a.cout + 127) / 128;
-    // about four CTAs per SM over all M tiles, at least 512 voxels each
-    long long per = (a.rows * mtiles) / (148 * 4);
-    per = ((per + 63) / 64) * 64;
-    if (per < 512) per = 512;
-    if (per > a.rows) per = a.rows;
+    const long long per = wgrad_voxels(a);
     a.kv = per;
     const long long ks = (a.rows + per - 1) / per;
     dim3 grid(mtiles, (unsigned)ks);
@@ -955,6 +1000,8 @@ int dsmc_sg_conv3_wgrad(void *stream, int batch, int S, const uint16_t *dy, int 
     a.rows = (long long)batch << (3 * lg);
     a.kv = 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (S >= kPlaneEdge && (cin == 16 || cin == 32 || cin == 48 || cin == 64 || cin == 96))
+        return cuda_rc(launch_wgrad_planes(a, st));
     switch (cin) {
     case 16: return cuda_rc(launch_wgrad<16>(a, st));
     case 32: return cuda_rc(launch_wgrad<32>(a, st));
