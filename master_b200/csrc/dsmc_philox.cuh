@@ -75,6 +75,11 @@ struct DrawStream {
         }
         ++k;
     }
+    // Continue at draw k_.
+    DSMC_HD void seek(uint32_t k_) {
+        k = k_;
+        if (k & 1u) philox4x32_10(id, step, tag, k >> 1, key0, key1, w);
+    }
     DSMC_HD double uniform64() {
         uint32_t a, b;
         words(a, b);
@@ -84,8 +89,9 @@ struct DrawStream {
     DSMC_HD float uniform32() {
         uint32_t a, b;
         words(a, b);
-        return ((float)(a >> 9) + 0.5f) * (1.0f / 8388608.0f);
+        return unit32(a);
     }
+    static DSMC_HD float unit32(uint32_t a) { return ((float)(a >> 9) + 0.5f) * (1.0f / 8388608.0f); }
     template <class T> DSMC_HD T uniform();
 };
 template <> DSMC_HD double DrawStream::uniform<double>() { return uniform64(); }

@@ -113,6 +113,60 @@ __device__ __forceinline__ bool cl_normal(real v_norm_in, real factor, real max_
     return false;
 }
 
+// cl_normal for the lanes of a warp whose bit is set in `todo`, the trials of
+// one lane's sampler spread over the warp: trial k takes the stream's draws
+// 3k, 3k + 1 and 3k + 2 after the ones used so far, so 32 consecutive trials
+// run at once and the first accepted one is the sampler's.  The same outcome
+// and stream position as cl_normal.  A lane alone runs the slowest of its
+// warp's samplers trial by trial (a fast particle needs hundreds: 20 of them
+// at twice the wall's thermal speed and alpha_n = 0.8 take a thousand turns
+// to all be through).  All lanes call; `ok` and `out` are set on the todo
+// lanes.
+__device__ __forceinline__ void cl_normal_warp(unsigned todo, float v_norm_in, float factor, float max_v_out,
+                                               float sqrt_an_over_2, float sqrt_1m_an, float sqrt_1m_an_over_an,
+                                               DrawStream &rs, bool &ok, float &out) {
+    const int lane = threadIdx.x & 31;
+    max_v_out /= factor;
+    v_norm_in /= factor;
+    for (; todo; todo &= todo - 1u) {
+        const int src = __ffs(todo) - 1;
+        const float vn = __shfl_sync(0xffffffffu, v_norm_in, src), vmax = __shfl_sync(0xffffffffu, max_v_out, src);
+        const float std_dev = __shfl_sync(0xffffffffu, sqrt_an_over_2, src);
+        const float s1 = __shfl_sync(0xffffffffu, sqrt_1m_an, src), s2 = __shfl_sync(0xffffffffu, sqrt_1m_an_over_an, src);
+        const float mu = s1 * vn;
+        DrawStream r;
+        r.key0 = __shfl_sync(0xffffffffu, rs.key0, src);
+        r.key1 = __shfl_sync(0xffffffffu, rs.key1, src);
+        r.id = __shfl_sync(0xffffffffu, rs.id, src);
+        r.step = __shfl_sync(0xffffffffu, rs.step, src);
+        r.tag = __shfl_sync(0xffffffffu, rs.tag, src);
+        const uint32_t k0 = __shfl_sync(0xffffffffu, rs.k, src);
+        bool found = false;
+        float res = 0.0f;
+        uint32_t used = DSMC_CL_TRIALS;  // trials up to and including the accepted one
+        for (uint32_t t0 = 0; t0 < DSMC_CL_TRIALS && !found; t0 += 32) {
+            const uint32_t trial = t0 + (uint32_t)lane;
+            r.seek(k0 + 3u * trial);
+            const float v_out = std_dev * gauss_draw<float>(r) + mu;
+            const float u = r.uniform<float>();
+            const float arg = 2.0f * s2 * vn * v_out;
+            const float b = v_out * exp(-arg) * bessel_i0_as<float>(arg) / vmax;
+            const unsigned hit = __ballot_sync(0xffffffffu, b >= u && trial < DSMC_CL_TRIALS);
+            if (hit) {
+                const int w = __ffs(hit) - 1;
+                res = __shfl_sync(0xffffffffu, v_out, w);
+                used = t0 + (uint32_t)w + 1u;
+                found = true;
+            }
+        }
+        if (lane == src) {
+            ok = found;
+            out = res * factor;
+            rs.seek(k0 + 3u * used);
+        }
+    }
+}
+
 // ---- sampler profiles -------------------------------------------------------
 // The calling warp's copy of the system's profile sums.
 __device__ __forceinline__ double *profile_copy(const SysDev &g) {
@@ -224,13 +278,10 @@ struct Split32 {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             float x = fmaf(w[d], tau, o[d]);
-            if (x >= 1.0f || x < 0.0f) {
-                float f = floorf(x);
-                c[d] += (int)f;
-                x -= f;
-                if (x >= 1.0f) x = one_minus_ulp();
-            }
-            o[d] = x;
+            const float f = (x >= 1.0f) | (x < 0.0f) ? floorf(x) : 0.0f;
+            c[d] += (int)f;
+            x -= f;
+            o[d] = x >= 1.0f ? one_minus_ulp() : x;
         }
     }
 
@@ -250,18 +301,17 @@ struct Split32 {
         for (int a = 0; a < 3; ++a) {
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
+                // (no early out: the six faces' divisions run side by side)
                 const float t = ((float)(s - dc[a]) - o[a]) / w[a];
-                if (!(t > 0.0f && t < best)) continue;
                 const int b1 = (a + 1) % 3, b2 = (a + 2) % 3;
                 const float h1 = fmaf(w[b1], t, (float)dc[b1] + o[b1]);
                 const float h2 = fmaf(w[b2], t, (float)dc[b2] + o[b2]);
                 // fp32 hit points on an edge can round just outside the face
                 const float eps = 1e-6f;
-                if (h1 >= -eps && h1 <= 1.0f + eps && h2 >= -eps && h2 <= 1.0f + eps) {
-                    best = t;
-                    axis = a;
-                    side = s;
-                }
+                const bool hit = (t > 0.0f) & (t < best) & (h1 >= -eps) & (h1 <= 1.0f + eps) & (h2 >= -eps) & (h2 <= 1.0f + eps);
+                best = hit ? t : best;
+                axis = hit ? a : axis;
+                side = hit ? s : side;
             }
         }
         if (axis < 0) return -1.0f;
@@ -287,52 +337,90 @@ struct Split32 {
         return false;
     }
 
+    // A wall voxel's normal and tangents, and a velocity's components in them.
+    struct WallFrame {
+        float n[3], a[3], b[3];
+        __device__ __forceinline__ void compose(float vn, float vt1, float vt2, float v[3]) const {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) v[d] = vn * n[d] + vt1 * a[d] + vt2 * b[d];
+        }
+    };
+    static __device__ __forceinline__ WallFrame load_frame(const SysDev &g, uint32_t vlin) {
+        WallFrame f;
+        const float *np = g.nrm + 3 * (size_t)vlin, *ap = g.t1 + 3 * (size_t)vlin, *bp = g.t2 + 3 * (size_t)vlin;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            f.n[d] = __ldg(np + d);
+            f.a[d] = __ldg(ap + d);
+            f.b[d] = __ldg(bp + d);
+        }
+        return f;
+    }
+    static __device__ __forceinline__ WallFrame wall_frame(const SysDev &g, uint32_t vlin, const float v[3], float &vni,
+                                                           float &vt1i, float &vt2i) {
+        const WallFrame f = load_frame(g, vlin);
+        vni = v[0] * f.n[0] + v[1] * f.n[1] + v[2] * f.n[2];
+        vt1i = v[0] * f.a[0] + v[1] * f.a[1] + v[2] * f.a[2];
+        vt2i = v[0] * f.b[0] + v[1] * f.b[1] + v[2] * f.b[2];
+        return f;
+    }
+    // ColliderCercignaniLampis::collide once the normal component is drawn:
+    // the tangential components, then the velocity.
+    static __device__ __forceinline__ void cl_finish(const SysDev &g, const WallFrame &f, float vn, float vt1i, float vt2i,
+                                                     float v[3], DrawStream &rs) {
+        const float sigma = 1.0f - sqrtf(1.0f - g.alpha_t_f);
+        const float vt1 = gauss_draw<float>(rs) * sqrtf(g.alpha_t_f) * g.wall_s_f + vt1i * (1.0f - sigma);
+        const float vt2 = gauss_draw<float>(rs) * sqrtf(g.alpha_t_f) * g.wall_s_f + vt2i * (1.0f - sigma);
+        f.compose(vn, vt1, vt2, v);
+    }
+
     // The wall model's collide: ColliderThermal::collide
     // (dsmc/colliderthermal.cpp:13-46), ColliderSpecular::collide or
     // ColliderCercignaniLampis::collide.  Returns error bits.
     static __device__ __forceinline__ unsigned reflect(const SysDev &g, uint32_t vlin, float v[3], DrawStream &rs) {
         if (g.wall_model != DSMC_WALL_THERMAL) {
-            const float *np = g.nrm + 3 * (size_t)vlin, *ap = g.t1 + 3 * (size_t)vlin, *bp = g.t2 + 3 * (size_t)vlin;
-            const float n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2);
-            const float a0 = __ldg(ap), a1 = __ldg(ap + 1), a2 = __ldg(ap + 2);
-            const float b0 = __ldg(bp), b1 = __ldg(bp + 1), b2 = __ldg(bp + 2);
-            const float vni = v[0] * n0 + v[1] * n1 + v[2] * n2;
-            const float vt1i = v[0] * a0 + v[1] * a1 + v[2] * a2;
-            const float vt2i = v[0] * b0 + v[1] * b1 + v[2] * b2;
-            float vn, vt1, vt2;
+            float vni, vt1i, vt2i, vn;
+            const WallFrame f = wall_frame(g, vlin, v, vni, vt1i, vt2i);
             if (g.wall_model == DSMC_WALL_SPECULAR) {
-                vn = -vni;
-                vt1 = vt1i;
-                vt2 = vt2i;
-            } else {
-                const float factor = sqrtf(2.0f) * g.wall_s_f;
-                if (!cl_normal<float>(vni, factor, g.cl_vmax_f, g.sqrt_an_over_2_f, g.sqrt_1m_an_f,
-                                      g.sqrt_1m_an_over_an_f, rs, vn))
-                    return DSMC_EBIT_WALL;
-                const float sigma = 1.0f - sqrtf(1.0f - g.alpha_t_f);
-                vt1 = gauss_draw<float>(rs) * sqrtf(g.alpha_t_f) * g.wall_s_f + vt1i * (1.0f - sigma);
-                vt2 = gauss_draw<float>(rs) * sqrtf(g.alpha_t_f) * g.wall_s_f + vt2i * (1.0f - sigma);
+                f.compose(-vni, vt1i, vt2i, v);
+                return 0;
             }
-            v[0] = vn * n0 + vt1 * a0 + vt2 * b0;
-            v[1] = vn * n1 + vt1 * a1 + vt2 * b1;
-            v[2] = vn * n2 + vt1 * a2 + vt2 * b2;
+            const float factor = sqrtf(2.0f) * g.wall_s_f;
+            if (!cl_normal<float>(vni, factor, g.cl_vmax_f, g.sqrt_an_over_2_f, g.sqrt_1m_an_f, g.sqrt_1m_an_over_an_f,
+                                  rs, vn))
+                return DSMC_EBIT_WALL;
+            cl_finish(g, f, vn, vt1i, vt2i, v, rs);
             return 0;
         }
-        const float s = g.wall_s_f;
-        const float vn = s * sqrtf(-2.0f * logf(rs.uniform32()));
-        float u = rs.uniform32();
-        float c = rs.uniform32();
-        const float g1 = sqrtf(-2.0f * logf(1.0f - u)) * cosf(6.283185307f * c);
-        u = rs.uniform32();
-        c = rs.uniform32();
-        const float g2 = sqrtf(-2.0f * logf(1.0f - u)) * cosf(6.283185307f * c);
-        const float vt1 = s * g1, vt2 = s * g2;
-        const float *n = g.nrm + 3 * (size_t)vlin;
-        const float *a = g.t1 + 3 * (size_t)vlin;
-        const float *b = g.t2 + 3 * (size_t)vlin;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) v[d] = vn * __ldg(n + d) + vt1 * __ldg(a + d) + vt2 * __ldg(b + d);
+        float vt[3];
+        thermal_draw(g, rs, vt);
+        load_frame(g, vlin).compose(vt[0], vt[1], vt[2], v);
         return 0;
+    }
+
+    // ColliderThermal::collide's draws: the normal and tangential components
+    // of the velocity a particle leaves the wall with.
+    static __device__ __forceinline__ void thermal_draw(const SysDev &g, DrawStream &rs, float out[3]) {
+        // the stream's next five draws from three Philox blocks, evaluated side
+        // by side (drawn one after the other the blocks' chains add up)
+        uint32_t b0[4], b1[4], b2[4];
+        const uint32_t blk = rs.k >> 1;
+        philox4x32_10(rs.id, rs.step, rs.tag, blk, rs.key0, rs.key1, b0);
+        philox4x32_10(rs.id, rs.step, rs.tag, blk + 1u, rs.key0, rs.key1, b1);
+        philox4x32_10(rs.id, rs.step, rs.tag, blk + 2u, rs.key0, rs.key1, b2);
+        const bool odd = rs.k & 1u;
+        const float u0 = DrawStream::unit32(odd ? b0[2] : b0[0]), u1 = DrawStream::unit32(odd ? b1[0] : b0[2]);
+        const float c1 = DrawStream::unit32(odd ? b1[2] : b1[0]), u2 = DrawStream::unit32(odd ? b2[0] : b1[2]);
+        const float c2 = DrawStream::unit32(odd ? b2[2] : b2[0]);
+        rs.k += 5u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rs.w[i] = b2[i];  // the block of the next draw if that is an odd one
+        const float s = g.wall_s_f;
+        out[0] = s * sqrtf(-2.0f * logf(u0));
+        const float g1 = sqrtf(-2.0f * logf(1.0f - u1)) * cosf(6.283185307f * c1);
+        const float g2 = sqrtf(-2.0f * logf(1.0f - u2)) * cosf(6.283185307f * c2);
+        out[1] = s * g1;
+        out[2] = s * g2;
     }
 
     // MoleculeMover::move_molecule (dsmc/moleculemover.cpp:50-126) with its
@@ -458,9 +546,16 @@ struct Split32 {
     // instead of one divergent path after another.  The same arithmetic in
     // the same order per particle as move_general.  All lanes call; inactive
     // lanes only keep the loop company.
+    //
+    // What bounds it is one flight's serial chain (a flight of ten reflections
+    // lasts longer than the rest of the kernel), so the chain's parts overlap:
+    // the wall's frame is loaded when its voxel is found, before the facet
+    // arithmetic and the next lookup; a diffuse wall's draws (Philox, log,
+    // cos) are made while a lookup is in flight.  They are used, and the
+    // stream moved past them, only if the flight does reflect.
     static __device__ __forceinline__ void move_general_warp(const SysDev &g, Particle &p, uint32_t step,
                                                              MoveTally &t, bool active) {
-        enum { S_START, S_FIRST, S_BISECT, S_FACET, S_REFLECT, S_DONE };
+        enum { S_START, S_FIRST, S_BISECT, S_FACET, S_REFLECT, S_CL, S_RESEED, S_DONE };
         DrawStream rs;
         rs.init(g.seed, p.id, step, DSMC_TAG_MOVE);
         float w[3] = {p.v[0] * g.inv_vox_f[0], p.v[1] * g.inv_vox_f[1], p.v[2] * g.inv_vox_f[2]};
@@ -470,15 +565,18 @@ struct Split32 {
         int c0[3] = {0, 0, 0}, cb[3] = {0, 0, 0};
         float o0[3] = {0.0f, 0.0f, 0.0f};
         int state = active ? S_START : S_DONE;
+        const bool diffuse = g.wall_model == DSMC_WALL_THERMAL;
+        WallFrame frame = {};
+        float drawn[3] = {0.0f, 0.0f, 0.0f};  // the next reflection's components, once made
+        DrawStream after = rs;                // the stream past them
+        bool have = false;
         while (__any_sync(0xffffffffu, state != S_DONE)) {
             bool look = false;
-            while (state != S_DONE && !look) {
+            while (state < S_CL && !look) {
                 if (state == S_START) {
                     if (here != DSMC_VOX_EMPTY) {
-                        ++t.reseeds;
-                        if (!reseed(g, p, rs)) t.err |= DSMC_EBIT_RESEED;
                         here = DSMC_VOX_EMPTY;
-                        state = S_DONE;
+                        state = S_RESEED;
                     } else {
 #pragma unroll
                         for (int a = 0; a < 3; ++a) {
@@ -506,9 +604,7 @@ struct Split32 {
                         count = 0;
                         state = S_FACET;
                     } else if (++count > 100) {
-                        ++t.reseeds;
-                        if (!reseed(g, p, rs)) t.err |= DSMC_EBIT_RESEED;
-                        state = S_DONE;
+                        state = S_RESEED;
                     } else if (vt == DSMC_VOX_WALL) {
                         tau *= 0.5f;
                         advance(p.c, p.o, w, -tau);
@@ -527,13 +623,12 @@ struct Split32 {
                     if (vt != DSMC_VOX_BOUNDARY) {
                         state = S_REFLECT;
                     } else if (++count > 100) {
-                        ++t.reseeds;
-                        if (!reseed(g, p, rs)) t.err |= DSMC_EBIT_RESEED;
-                        state = S_DONE;
+                        state = S_RESEED;
                     } else {
                         cb[0] = p.c[0];
                         cb[1] = p.c[1];
                         cb[2] = p.c[2];
+                        if (diffuse) frame = load_frame(g, voxel_linear(g, cb[0], cb[1], cb[2]));
 #pragma unroll
                         for (int a = 0; a < 3; ++a) {
                             p.c[a] = c0[a];
@@ -547,9 +642,7 @@ struct Split32 {
                         const float tf = facet_time(dc, p.o, w, axis, side);
                         if (tf < 0.0f) {
                             t.err |= DSMC_EBIT_FACET;
-                            ++t.reseeds;
-                            if (!reseed(g, p, rs)) t.err |= DSMC_EBIT_RESEED;
-                            state = S_DONE;
+                            state = S_RESEED;
                         } else {
                             tau = tf;
                             advance(p.c, p.o, w, tau);
@@ -574,7 +667,17 @@ struct Split32 {
                 } else {  // S_REFLECT
                     here = vt;
                     dt -= tau;
-                    t.err |= reflect(g, voxel_linear(g, cb[0], cb[1], cb[2]), p.v, rs);
+                    if (g.wall_model == DSMC_WALL_CL) {
+                        state = S_CL;  // its sampler runs on the whole warp
+                        continue;
+                    }
+                    if (diffuse) {
+                        frame.compose(drawn[0], drawn[1], drawn[2], p.v);
+                        rs = after;
+                        have = false;
+                    } else {
+                        t.err |= reflect(g, voxel_linear(g, cb[0], cb[1], cb[2]), p.v, rs);
+                    }
                     ++t.wall_hits;
 #pragma unroll
                     for (int d = 0; d < 3; ++d) w[d] = p.v[d] * g.inv_vox_f[d];
@@ -587,6 +690,41 @@ struct Split32 {
                 }
             }
             if (look) vt = voxel_type(g, p.c[0], p.c[1], p.c[2]);
+            if (state == S_RESEED) {
+                ++t.reseeds;
+                if (!reseed(g, p, rs)) t.err |= DSMC_EBIT_RESEED;
+                state = S_DONE;
+            }
+            if (diffuse && state != S_DONE && !have) {
+                after = rs;
+                thermal_draw(g, after, drawn);
+                have = true;
+            }
+            const unsigned cl = __ballot_sync(0xffffffffu, state == S_CL);
+            if (cl) {
+                const bool mine = state == S_CL;
+                WallFrame f;
+                float vni = 0.0f, vt1i = 0.0f, vt2i = 0.0f, vn = 0.0f;
+                bool ok = false;
+                if (mine) f = wall_frame(g, voxel_linear(g, cb[0], cb[1], cb[2]), p.v, vni, vt1i, vt2i);
+                cl_normal_warp(cl, vni, sqrtf(2.0f) * g.wall_s_f, g.cl_vmax_f, g.sqrt_an_over_2_f, g.sqrt_1m_an_f,
+                               g.sqrt_1m_an_over_an_f, rs, ok, vn);
+                if (mine) {
+                    if (ok)
+                        cl_finish(g, f, vn, vt1i, vt2i, p.v, rs);
+                    else
+                        t.err |= DSMC_EBIT_WALL;
+                    ++t.wall_hits;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) w[d] = p.v[d] * g.inv_vox_f[d];
+                    if (!(dt > 1e-5f && depth < 10)) {
+                        state = S_DONE;
+                    } else {
+                        ++depth;
+                        state = S_START;
+                    }
+                }
+            }
         }
         if (active) {
             p.flag = here != DSMC_VOX_EMPTY;

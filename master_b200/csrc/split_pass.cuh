@@ -1265,8 +1265,14 @@ __global__ void __launch_bounds__(32 * P_WARPS, 5) place_movers_kernel(const __g
     counts_publish(P, tsys, cnt, false);
 }
 
-// The general mover for every listed wall flight, one per thread, then the
-// placement.  The last block ends the pass: it advances the step and halts
+// The general mover for every listed wall flight, one per lane, then the
+// placement.  Bound by the longest flight's serial chain (ten reflections of
+// about 3 us each) and, with many flights, by the divergence of a warp's.
+// Measured, us per step before and after the claims sized to the grid, the
+// overlapped draws and frames and the warp-shared Cercignani-Lampis trials:
+// 64^3 (2e3 flights) 42 -> 35, 128^3 (1.8e4) 61 -> 49, with CL walls of
+// alpha_n = 0.8 524 -> 104, 256^3 (1.5e5) 93 -> 87.  Held to fewer registers
+// (128, 102, 85 for 4, 5, 6 blocks per SM) it spills: 37, 40 and 44 us at 64^3.  The last block ends the pass: it advances the step and halts
 // the pipeline if anything spilled or failed.
 __global__ void __launch_bounds__(32 * W_WARPS) place_walls_kernel(const __grid_constant__ PassParams P) {
     const int lane = threadIdx.x & 31;
@@ -1279,15 +1285,20 @@ __global__ void __launch_bounds__(32 * W_WARPS) place_walls_kernel(const __grid_
     MoveCounts cnt;
     counts_reset(cnt);
     int tsys = -1;
-    // warps claim 32 entries at a time: flights differ widely in length, so
-    // a warp that finishes early takes more
+    // Warps claim entries from a counter: flights differ widely in length, so
+    // a warp that finishes early takes more.  A claim is 32 entries, or fewer
+    // when the list would not fill the grid's warps: a turn of the flights'
+    // state machine runs every state that some lane is in, so a warp of few
+    // lanes finishes its flights sooner.
+    const unsigned nw = gridDim.x * W_WARPS;
+    const unsigned claim = min(32u, max(1u, (nwalls + nw - 1u) / nw));
     for (;;) {
         unsigned i0 = 0;
-        if (lane == 0) i0 = atomicAdd(&P.status->walls_taken, 32u);
+        if (lane == 0) i0 = atomicAdd(&P.status->walls_taken, claim);
         i0 = __shfl_sync(0xffffffffu, i0, 0);
         if (i0 >= nwalls) break;
         const unsigned i = i0 + lane;
-        const bool valid = i < nwalls;
+        const bool valid = (unsigned)lane < claim && i < nwalls;
         const int2 e = valid ? P.parts.walls[i] : make_int2(0, -1);  // {slot, source cell}
         const int esys = valid ? P.cells.meta[e.y].w : -1;
         const int csys = common_system(valid, esys);

@@ -9,6 +9,7 @@ import pytest
 
 from master_b200 import capi
 from master_b200.system import System
+from master_b200.workloads import Workload, simulators_per_cell_weight
 from test_parity_gpu import load_case
 
 pytestmark = pytest.mark.gpu
@@ -179,3 +180,25 @@ def test_non_finite_state_is_refused_and_the_system_keeps_its_particles(precisio
     assert err & capi.EBIT_FATAL == 0
     r3, v3 = S.get_particles()
     assert np.isfinite(r3).all() and np.isfinite(v3).all() and S.tallies().step == 3
+
+
+@pytest.mark.parametrize("n,per_cell,dt_si,model,alpha_n", [
+    (16, 20, 1e-11, 0, 0.0), (16, 20, 1e-11, 2, 0.5), (16, 20, 5e-11, 1, 0.0), (32, 20, 2e-11, 2, 0.8),
+    (34, 20, 5e-11, 0, 0.0), (64, 60, 1e-10, 0, 0.0), (64, 60, 1e-10, 2, 1.0)])
+def test_wall_flights_few_and_many(n, per_cell, dt_si, model, alpha_n):
+    """place_walls with a handful of wall flights (claims of one entry per
+    warp) up to more than its grid holds at 32 a warp, under each wall model;
+    the Cercignani-Lampis sampler, whose trials the warp shares, at an
+    accommodation where it takes many trials and where it takes few.  Bit for
+    bit the stage kernels, which run one flight per lane and one trial at a
+    time."""
+    w = Workload("walls", n=n, radius_voxels=3.0, porosity=0.6, geometry_seed=5, cells=n // 2,
+                 atoms_per_molecule=simulators_per_cell_weight(2.5e24, 0.1, 2, per_cell), dt_si=dt_si)
+    g = w.geometry()
+    s = w.settings(rng_seed=11, statistics_interval=10 ** 9)
+    s.surface_model = model
+    if model == 2:
+        s.alpha_n, s.alpha_t = alpha_n, 0.8
+    A, B = System(s, g), System(s, g)
+    run_both(A, B, 3)
+    assert A.tallies().wall_collisions > 0
