@@ -10,10 +10,23 @@
 namespace dsmc {
 namespace split32 {
 
+// Cells per chunk for a persistent grid of `warps` warps taking chunks at a
+// fixed stride: 32 (one table row or lane per cell) gives some warps one chunk
+// more than the rest, and none to most of them when there are few cells, so
+// the chunk is cut until every warp has the same number of them.
+static PassParams with_chunk(const PassParams &P, long long warps) {
+    PassParams Q = P;
+    const long long C = P.cells.num_cells;
+    const long long rounds = std::max(1ll, (C + 32 * warps - 1) / (32 * warps));
+    Q.chunk = (int)std::max(1ll, (C + rounds * warps - 1) / (rounds * warps));
+    return Q;
+}
+
 // The production pass (split_pass.cuh): collide_cells, move_cells with the
 // smallest ring that holds the largest cell, place_movers, place_walls.
 template <int R> static cudaError_t launch_move_ring(const PassParams &P, int grid, cudaStream_t st) {
-    pass3::move_cells_kernel<R><<<grid, 32 * pass3::M_WARPS, pass3::move_smem_bytes<R>(), st>>>(P);
+    pass3::move_cells_kernel<R><<<grid, 32 * pass3::M_WARPS, pass3::move_smem_bytes<R>(), st>>>(
+        with_chunk(P, (long long)grid * pass3::M_WARPS));
     return cudaGetLastError();
 }
 template <int R> static int move_ring_blocks() {
@@ -97,10 +110,12 @@ int fused_grids(int smem_cap, int num_sms, int grids[5], int ring, int max_bps[5
 }
 
 // collide_cells with the chunk counter when each warp has many chunks
-static void launch_collide_cells(const PassParams &P, int grid, cudaStream_t st) {
+static void launch_collide_cells(const PassParams &P0, int grid, cudaStream_t st) {
+    PassParams P = with_chunk(P0, (long long)grid * pass3::C_WARPS);
     const long long nchunks = (P.cells.num_cells + 31) / 32;
     const bool counter = P.claim == 2 ||
                          (P.claim == 0 && nchunks >= (long long)pass3::CLAIM_MIN_CHUNKS_PER_WARP * grid * pass3::C_WARPS);
+    if (counter) P.chunk = 32;
     if (counter)
         pass3::collide_cells_kernel<true><<<grid, 32 * pass3::C_WARPS, 0, st>>>(P);
     else
@@ -114,7 +129,8 @@ cudaError_t launch_fused(const PassParams &P, const int grids[5], cudaStream_t s
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         if (P.do_sample) {  // sampled steps only: the host knows the cadence
-            pass3::sample_cells_kernel<<<grids[4], 32 * pass3::C_WARPS, 0, st>>>(P);
+            pass3::sample_cells_kernel<<<grids[4], 32 * pass3::C_WARPS, 0, st>>>(
+                with_chunk(P, (long long)grids[4] * pass3::C_WARPS));
             e = cudaGetLastError();
             if (e != cudaSuccess) return e;
         }
@@ -129,7 +145,8 @@ cudaError_t launch_fused(const PassParams &P, const int grids[5], cudaStream_t s
     }
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[2], st);
-    pass3::place_movers_kernel<<<grids[2], 32 * pass3::P_WARPS, 0, st>>>(P);
+    pass3::place_movers_kernel<<<grids[2], 32 * pass3::P_WARPS, 0, st>>>(
+        with_chunk(P, (long long)grids[2] * pass3::P_WARPS));
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[3], st);
@@ -144,7 +161,8 @@ cudaError_t launch_collide(const PassParams &P, const int grids[5], cudaStream_t
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (P.do_sample) {
-        pass3::sample_cells_kernel<<<grids[4], 32 * pass3::C_WARPS, 0, st>>>(P);
+        pass3::sample_cells_kernel<<<grids[4], 32 * pass3::C_WARPS, 0, st>>>(
+                with_chunk(P, (long long)grids[4] * pass3::C_WARPS));
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

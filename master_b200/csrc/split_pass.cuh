@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(32 * C_WARPS) collide_cells_kernel(const __gri
     CollideSmem &W = smem[threadIdx.x >> 5];
     float4 *Bin = reinterpret_cast<float4 *>(P.parts.B[P.cur]);
 
-    const int C = P.cells.num_cells;
-    const int nchunks = (C + 31) >> 5;
+    const int C = P.cells.num_cells, CH = P.chunk;
+    const int nchunks = (C + CH - 1) / CH;
     unsigned col = 0, cand = 0;  // this lane's counts for system tsys
     int tsys = -1;
 
@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(32 * C_WARPS) collide_cells_kernel(const __gri
     for (int ch = blockIdx.x * C_WARPS + (threadIdx.x >> 5); ch < nchunks;
          ch = CLAIM ? nw + claim_take(nxt) : ch + nw) {
         if (CLAIM) nxt = claim_issue(&P.status->collide_taken, lane);  // the next chunk, in flight meanwhile
-        const int first = ch * 32;
-        const bool mine = lane < C - first;
+        const int first = ch * CH;
+        const bool mine = lane < min(CH, C - first);
         const int a = first + lane;
         int4 m = make_int4(0, 0, 0, -1);
         unsigned nb = 0, nt = 0;
@@ -490,15 +490,15 @@ __global__ void __launch_bounds__(32 * C_WARPS) sample_cells_kernel(const __grid
     // of squares
     const int slot = lane >> 2;
     const int mcol = (lane & 3) == 0 && slot < 6 ? 1 + slot : lane == 1 ? 0 : -1;
-    const int C = P.cells.num_cells;
-    const int nchunks = (C + 31) >> 5;
+    const int C = P.cells.num_cells, CH = P.chunk;
+    const int nchunks = (C + CH - 1) / CH;
     const int nwarps = gridDim.x * C_WARPS;
     for (int ch = blockIdx.x * C_WARPS + (threadIdx.x >> 5); ch < nchunks; ch += nwarps) {
-        const int a = ch * 32 + lane;
+        const int a = ch * CH + lane;
         int4 m = make_int4(0, 0, 0, -1);
         unsigned nb = 0, nt = 0;
         bool smp = false;
-        if (a < C) {
+        if (lane < CH && a < C) {
             m = P.cells.meta[a];
             input_counts(P, a, m, nb, nt);
             const SysDev &g = P.sys[m.w];
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(32 * C_WARPS) sample_cells_kernel(const __grid
         }
         for (unsigned todo = __ballot_sync(0xffffffffu, smp); todo; todo &= todo - 1u) {
             const int c = __ffs(todo) - 1;
-            const int ac = ch * 32 + c;
+            const int ac = ch * CH + c;
             const int sys = __shfl_sync(0xffffffffu, m.w, c);
             const int cb = __shfl_sync(0xffffffffu, m.x, c), cc = __shfl_sync(0xffffffffu, m.y, c);
             const int cnb = (int)__shfl_sync(0xffffffffu, nb, c), cnt = (int)__shfl_sync(0xffffffffu, nt, c);
@@ -803,15 +803,15 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
     uint4 *Aout = reinterpret_cast<uint4 *>(P.parts.A[P.cur ^ 1]);
     float4 *Bout = reinterpret_cast<float4 *>(P.parts.B[P.cur ^ 1]);
 
-    const int C = P.cells.num_cells;
-    const int nchunks = (C + 31) >> 5;
+    const int C = P.cells.num_cells, CH = P.chunk;
+    const int nchunks = (C + CH - 1) / CH;
     const int wstride = gridDim.x * M_WARPS;
     const int chunk0 = blockIdx.x * M_WARPS + wib;
 
     auto load_tab = [&](int b, int ch) {
         MoveTab &T = W.tab[b];
-        const int first = ch * 32;
-        const int ncell = ch < nchunks ? min(32, C - first) : 0;
+        const int first = ch * CH;
+        const int ncell = ch < nchunks ? min(CH, C - first) : 0;
         if (lane == 0) {
             T.first = first;
             T.ncell = ncell;
@@ -878,7 +878,7 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
             if (head >= R) head -= R;
             used += n;
             ++ahead;
-            if (++ii == 32) {
+            if (++ii == CH) {
                 ++it;
                 ii = 0;
             }
@@ -889,7 +889,7 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
         const MoveTab &T = W.tab[ct & 1];
         if (ci >= T.ncell) {
             if (T.ncell > 0) write_tab(ct & 1, nfs_mine);
-            if (T.ncell < 32) break;  // that was the warp's last chunk
+            if (T.ncell < CH) break;  // that was the warp's last chunk
             __syncwarp();
             load_tab(ct & 1, chunk0 + (ct + 2) * wstride);
             __syncwarp();
@@ -1189,11 +1189,11 @@ __global__ void __launch_bounds__(32 * P_WARPS, 5) place_movers_kernel(const __g
     counts_reset(cnt);
     int tsys = -1;
 
-    const int C = P.cells.num_cells;
-    const int nchunks = (C + 31) >> 5;
+    const int C = P.cells.num_cells, CH = P.chunk;
+    const int nchunks = (C + CH - 1) / CH;
     for (int ch = blockIdx.x * P_WARPS + (threadIdx.x >> 5); ch < nchunks; ch += gridDim.x * P_WARPS) {
-        const int first = ch * 32;
-        const bool mine = lane < C - first;
+        const int first = ch * CH;
+        const bool mine = lane < min(CH, C - first);
         // lane i: the movers of cell i sit in output slots [gap, gap + cnt)
         int gap = 0, mv = 0, sys = -1;
         if (mine) {
