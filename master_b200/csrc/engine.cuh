@@ -117,11 +117,10 @@ __device__ __forceinline__ bool cl_normal(real v_norm_in, real factor, real max_
 // one lane's sampler spread over the warp: trial k takes the stream's draws
 // 3k, 3k + 1 and 3k + 2 after the ones used so far, so 32 consecutive trials
 // run at once and the first accepted one is the sampler's.  The same outcome
-// and stream position as cl_normal.  A lane alone runs the slowest of its
-// warp's samplers trial by trial (a fast particle needs hundreds: 20 of them
-// at twice the wall's thermal speed and alpha_n = 0.8 take a thousand turns
-// to all be through).  All lanes call; `ok` and `out` are set on the todo
-// lanes.
+// and stream position as cl_normal.  (One lane per sampler, a warp waits for
+// its slowest: at alpha_n = 0.8 a particle at three times the wall's thermal
+// speed needs 240 trials on average.)  All lanes call; `ok` and `out` are set
+// on the todo lanes.
 __device__ __forceinline__ void cl_normal_warp(unsigned todo, float v_norm_in, float factor, float max_v_out,
                                                float sqrt_an_over_2, float sqrt_1m_an, float sqrt_1m_an_over_an,
                                                DrawStream &rs, bool &ok, float &out) {

@@ -5,7 +5,7 @@
 //
 //   collide_cells  Cell::prepare + Cell::collide (dsmc/cell.cpp:42-111) of
 //                  every cell.
-//                  Per chunk of 32 consecutive cells lane i selects for cell
+//                  Per chunk of (up to 32) consecutive cells lane i selects for cell
 //                  i; the warp ranks each colliding cell's particles by id
 //                  (the reference's member order) into shared memory, then
 //                  every lane runs the candidate loop of its own cell.
