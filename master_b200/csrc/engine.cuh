@@ -35,9 +35,23 @@ __device__ __forceinline__ int wrap_index(int c, int n) {
 }
 
 __device__ __forceinline__ uint32_t voxel_linear(const SysDev &g, int i, int j, int k) {
-    return ((uint32_t)wrap_index(i, g.n[0]) * (uint32_t)g.n[1] + (uint32_t)wrap_index(j, g.n[1])) *
-               (uint32_t)g.n[2] +
-           (uint32_t)wrap_index(k, g.n[2]);
+    // at most one box length outside, as nearly always: no branches (they
+    // stand in every flight's chain)
+    int c[3] = {i, j, k};
+    bool far = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int n = g.n[d];
+        c[d] += c[d] < 0 ? n : 0;
+        c[d] -= c[d] >= n ? n : 0;
+        far |= (unsigned)c[d] >= (unsigned)n;
+    }
+    if (far) {
+        c[0] = wrap_index(i, g.n[0]);
+        c[1] = wrap_index(j, g.n[1]);
+        c[2] = wrap_index(k, g.n[2]);
+    }
+    return ((uint32_t)c[0] * (uint32_t)g.n[1] + (uint32_t)c[1]) * (uint32_t)g.n[2] + (uint32_t)c[2];
 }
 
 __device__ __forceinline__ int voxel_type(const SysDev &g, int i, int j, int k) {
@@ -561,6 +575,7 @@ struct Split32 {
         float dt = g.dt_f, tau = 0.0f;
         int here = p.flag ? DSMC_VOX_WALL : DSMC_VOX_EMPTY;
         int depth = 0, count = 0, vt = DSMC_VOX_EMPTY;
+        uint32_t lin = 0, wlin = 0;  // the last lookup's voxel, the wall's
         int c0[3] = {0, 0, 0}, cb[3] = {0, 0, 0};
         float o0[3] = {0.0f, 0.0f, 0.0f};
         int state = active ? S_START : S_DONE;
@@ -627,7 +642,8 @@ struct Split32 {
                         cb[0] = p.c[0];
                         cb[1] = p.c[1];
                         cb[2] = p.c[2];
-                        if (diffuse) frame = load_frame(g, voxel_linear(g, cb[0], cb[1], cb[2]));
+                        wlin = lin;
+                        if (diffuse) frame = load_frame(g, wlin);
 #pragma unroll
                         for (int a = 0; a < 3; ++a) {
                             p.c[a] = c0[a];
@@ -675,7 +691,7 @@ struct Split32 {
                         rs = after;
                         have = false;
                     } else {
-                        t.err |= reflect(g, voxel_linear(g, cb[0], cb[1], cb[2]), p.v, rs);
+                        t.err |= reflect(g, wlin, p.v, rs);
                     }
                     ++t.wall_hits;
 #pragma unroll
@@ -688,7 +704,10 @@ struct Split32 {
                     }
                 }
             }
-            if (look) vt = voxel_type(g, p.c[0], p.c[1], p.c[2]);
+            if (look) {
+                lin = voxel_linear(g, p.c[0], p.c[1], p.c[2]);
+                vt = __ldg(g.vox + lin);
+            }
             if (state == S_RESEED) {
                 ++t.reseeds;
                 if (!reseed(g, p, rs)) t.err |= DSMC_EBIT_RESEED;
@@ -705,7 +724,7 @@ struct Split32 {
                 WallFrame f;
                 float vni = 0.0f, vt1i = 0.0f, vt2i = 0.0f, vn = 0.0f;
                 bool ok = false;
-                if (mine) f = wall_frame(g, voxel_linear(g, cb[0], cb[1], cb[2]), p.v, vni, vt1i, vt2i);
+                if (mine) f = wall_frame(g, wlin, p.v, vni, vt1i, vt2i);
                 cl_normal_warp(cl, vni, sqrtf(2.0f) * g.wall_s_f, g.cl_vmax_f, g.sqrt_an_over_2_f, g.sqrt_1m_an_f,
                                g.sqrt_1m_an_over_an_f, rs, ok, vn);
                 if (mine) {
@@ -1080,7 +1099,12 @@ struct Fp64 {
             ++t.wall_hits;
             if (!(dt > 1e-5 && depth < 10)) break;
         }
-        // MoleculeMover::apply_periodic_boundary_conditions (dsmc/moleculemover.h:29-38)
+        wrap(g, p, t);
+        return true;
+    }
+
+    // MoleculeMover::apply_periodic_boundary_conditions (dsmc/moleculemover.h:29-38)
+    static __device__ __forceinline__ void wrap(const SysDev &g, Particle &p, MoveTally &t) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             if (p.r[d] >= g.L[d]) {
@@ -1092,6 +1116,23 @@ struct Fp64 {
             }
             if (!isfinite(p.r[d]) || !isfinite(p.v[d])) t.err |= DSMC_EBIT_NAN;
         }
+    }
+
+    // move()'s outcome when the first flight is all there is: from an empty
+    // voxel to an empty voxel.  False, p untouched, otherwise.  Both ends'
+    // lookups are in flight together.
+    static __device__ __forceinline__ bool move_open(const SysDev &g, Particle &p, MoveTally &t) {
+        int u[3], w[3];
+        double r[3] = {p.r[0], p.r[1], p.r[2]};
+        voxel_of(g, r, u);
+        do_move(r, p.v, g.dt);
+        voxel_of(g, r, w);
+        const int v0 = voxel_type(g, u[0], u[1], u[2]);
+        const int v1 = voxel_type(g, w[0], w[1], w[2]);
+        if (v0 != DSMC_VOX_EMPTY || v1 >= DSMC_VOX_WALL) return false;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) p.r[d] = r[d];
+        wrap(g, p, t);
         return true;
     }
 
@@ -1259,20 +1300,6 @@ template <class Prec> struct StageVel {
     }
 };
 
-template <class Prec>
-__device__ void ntc_collide(const SysDev &g, int cell_global_index, uint32_t step, int n, double coeff,
-                            double &vr_max, double &rest, WarpStage<Prec> &st, unsigned long long &collisions,
-                            unsigned long long &candidates) {
-    const int pairs = ntc_select(coeff, n, vr_max, rest);
-    if (n < 2 || pairs <= 0) return;
-    StageVel<Prec> vel;
-    vel.vx = st.vx;
-    vel.vy = st.vy;
-    vel.vz = st.vz;
-    ntc_run<typename Prec::real>(g.seed, cell_global_index, step, n, pairs, vr_max, vel, st.perm, collisions);
-    candidates += (unsigned long long)pairs;
-}
-
 struct WarpTally {
     unsigned long long collisions, candidates, wall_hits, reseeds, moved, stranded;
     long long cross[3];
@@ -1324,6 +1351,105 @@ __device__ __forceinline__ void flush_tally(const PassParams &P, WarpTally &w, i
     w.err = 0;
 }
 
+// Warp-aggregated counting-sort insert of one particle per valid lane into the
+// top slots of cell `key` (its meta row km is loaded while the atomic is in
+// flight).  All lanes call.
+template <class Prec>
+__device__ __forceinline__ void insert_particle(const PassParams &P, const typename Prec::Particle &p, bool valid,
+                                                unsigned key, unsigned &err) {
+    typedef typename Prec::RecA RecA;
+    typedef typename Prec::RecB RecB;
+    const int lane = threadIdx.x & 31;
+    unsigned *top_out = P.cells.top[P.cout];
+    const unsigned peers = __match_any_sync(0xffffffffu, valid ? key : 0xffffffffu);
+    const int leader = __ffs(peers) - 1;
+    const unsigned lower = peers & ((1u << lane) - 1u);
+    unsigned slot0 = 0;
+    if (valid && lane == leader) slot0 = atomicAdd(&top_out[key], (unsigned)__popc(peers));
+    const int4 km = valid ? P.cells.meta[key] : make_int4(0, 0, 0, 0);
+    slot0 = __shfl_sync(0xffffffffu, slot0, leader);
+    bool spilled = false;
+    if (valid) {
+        const unsigned k = slot0 + (unsigned)__popc(lower);
+        RecA ra;
+        RecB rb;
+        Prec::pack(p, ra, rb);
+        // a top slot may not reach the slots the cell's owner can
+        // fill from the bottom (at most its input occupancy)
+        const unsigned room = P.top_only ? (unsigned)km.y
+                                         : (unsigned)km.y - min((unsigned)km.y,
+                                                                P.cells.bot[P.cin][key] + P.cells.top[P.cin][key]);
+        if (k < room) {
+            const unsigned dst = (unsigned)(km.x + km.y) - 1u - k;
+            reinterpret_cast<RecA *>(P.parts.A[P.cur ^ 1])[dst] = ra;
+            reinterpret_cast<RecB *>(P.parts.B[P.cur ^ 1])[dst] = rb;
+        } else {
+            spilled = true;
+            const unsigned si = atomicAdd(&P.status->spill, 1u);
+            if (si < P.parts.spill_cap) {
+                SpillRec &sr = P.parts.spill[si];
+                if (sizeof(typename Prec::real) == 8) {
+                    sr.ra = *reinterpret_cast<const double4 *>(&ra);
+                    sr.rb = *reinterpret_cast<const double4 *>(&rb);
+                } else {
+                    sr.a = *reinterpret_cast<const uint4 *>(&ra);
+                    sr.b = *reinterpret_cast<const uint4 *>(&rb);
+                }
+                sr.cell = (int)key;
+            } else {
+                err |= DSMC_EBIT_SPILL_FULL;
+            }
+        }
+    }
+    // spilled slots are given back, so the counter ends at the
+    // number of particles actually placed in the top segment
+    const unsigned over = __ballot_sync(0xffffffffu, spilled) & peers;
+    if (valid && lane == leader && over) atomicSub(&top_out[key], (unsigned)__popc(over));
+}
+
+// The cell a moved particle belongs to; one that ended inside solid whose cell
+// has no free volume stays with its source cell (the reference aborts there,
+// dsmc/system.h:134-142; the particle's next move re-seeds it,
+// dsmc/moleculemover.cpp:57-60).
+template <class Prec>
+__device__ __forceinline__ unsigned moved_cell(const SysDev &g, const typename Prec::Particle &p, int src, unsigned &err,
+                                               unsigned long long &stranded) {
+    const int ac = __ldg(g.cell_map + Prec::cell_global(g, p));
+    if (ac >= 0) return (unsigned)ac;
+    err |= DSMC_EBIT_STRANDED;
+    ++stranded;
+    return (unsigned)src;
+}
+
+// End of a pass: the last block to finish advances the step and halts the
+// pipeline if anything spilled or failed.  All threads call.
+__device__ __forceinline__ void end_pass(const PassParams &P) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned done = atomicAdd(&P.status->blocks_done, 1u);
+        if (done == gridDim.x - 1) {
+            __threadfence();
+            if (P.advance_step) atomicAdd(&P.status->step, 1u);
+            if (atomicAdd(&P.status->spill, 0u) != 0u || (atomicAdd(&P.status->error, 0u) & DSMC_EBIT_FATAL) != 0u)
+                atomicExch(&P.status->halted, 1u);
+            atomicExch(&P.status->walls, 0u);
+            atomicExch(&P.status->walls_taken, 0u);
+            atomicExch(&P.status->blocks_done, 0u);
+        }
+    }
+}
+
+// The cell pass.  MODE_FUSED (the whole step) moves the flights that end in an
+// empty voxel and lists the others, a few in a thousand, for
+// pass_walls_kernel: with the general mover inline one lane's reflections kept
+// its warp's other cells waiting, and the kernel ran at half the resident
+// warps.  Members are staged and ranked only in cells that collide or sample,
+// and the next cell's header is loaded ahead.  At 3.9e5 particles in fp64 a step
+// went from 121 to 103 us: 53 here (bound by the chain of a cell: header,
+// records, both voxel lookups, cell map, counter) and 47 for the longest wall
+// flight.  With the collide's arithmetic out of line (80 registers, 24 resident
+// warps instead of 16) the pass took 63 us.
 template <class Prec, int MODE>
 __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
     typedef typename Prec::real real;
@@ -1345,13 +1471,10 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
 
     const RecA *Ain = reinterpret_cast<const RecA *>(P.parts.A[P.cur]);
     const RecB *Bin = reinterpret_cast<const RecB *>(P.parts.B[P.cur]);
-    RecA *Aout = reinterpret_cast<RecA *>(P.parts.A[P.cur ^ 1]);
-    RecB *Bout = reinterpret_cast<RecB *>(P.parts.B[P.cur ^ 1]);
     RecA *Aio = reinterpret_cast<RecA *>(P.parts.A[P.cur]);
     RecB *Bio = reinterpret_cast<RecB *>(P.parts.B[P.cur]);
     const unsigned *bot_in = P.cells.bot[P.cin];
     const unsigned *top_in = P.cells.top[P.cin];
-    unsigned *top_out = P.cells.top[P.cout];
 
     WarpTally wt;
     wt.collisions = wt.candidates = wt.wall_hits = wt.reseeds = wt.moved = wt.stranded = 0;
@@ -1361,16 +1484,29 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
 
     const int C = P.cells.num_cells;
     const int stride = gridDim.x * warps_per_block;
-    for (int a = blockIdx.x * warps_per_block + warp_in_block; a < C; a += stride) {
-        const int4 meta = P.cells.meta[a];
+    int a = blockIdx.x * warps_per_block + warp_in_block;
+    int4 meta = make_int4(0, 0, 0, 0);
+    unsigned nb = 0, nt = 0;
+    auto header = [&](int c, int4 &m, unsigned &b, unsigned &t) {
+        if (c < C) {
+            m = P.cells.meta[c];
+            b = bot_in[c];
+            t = top_in[c];
+        }
+    };
+    header(a, meta, nb, nt);
+    for (; a < C; a += stride) {
+        int4 next_meta = make_int4(0, 0, 0, 0);
+        unsigned next_nb = 0, next_nt = 0;
+        header(a + stride, next_meta, next_nb, next_nt);
+        nb = min(nb, (unsigned)meta.y);
+        nt = min(nt, (unsigned)meta.y - nb);
         const int sys = meta.w;
         if (sys != wt.sys) {
             if (wt.sys >= 0) flush_tally(P, wt, lane);
             wt.sys = sys;
         }
         const SysDev &g = P.sys[sys];
-        const unsigned nb = min(bot_in[a], (unsigned)meta.y);
-        const unsigned nt = min(top_in[a], (unsigned)meta.y - nb);
         int n = (int)(nb + nt);
         if (n > P.smem_cap) {
             wt.err |= DSMC_EBIT_SMEM;
@@ -1379,10 +1515,18 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
         const bool collide = P.do_collide && MODE != MODE_SORT;
         bool sample = P.do_sample && MODE != MODE_SORT && g.sample_interval > 0 && step > 0 &&
                       (step % (uint32_t)g.sample_interval) == 0 && step >= (uint32_t)g.sample_begin;
-        const bool need_order = collide || sample;
+        // Cell::prepare, on every lane; the candidate pairs run below
+        double4 cs = make_double4(0, 0, 0, 0);
+        int pairs = 0;
+        if (collide) {
+            cs = P.cells.state[a];
+            pairs = ntc_select(cs.z, n, cs.x, cs.y);
+            if (n < 2) pairs = 0;
+        }
+        const bool staged = pairs > 0 || sample;  // members needed in id order
 
         // Stage velocities (and ids) in shared memory.
-        if (MODE != MODE_SORT) {
+        if (staged) {
             for (int s = lane; s < n; s += 32) {
                 real v[3];
                 uint32_t id;
@@ -1393,8 +1537,6 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
                 st.id[s] = id;
             }
             __syncwarp();
-        }
-        if (need_order) {
             // Members in id order: rank = number of smaller ids.
             for (int s = lane; s < n; s += 32) {
                 const uint32_t mine = st.id[s];
@@ -1404,14 +1546,18 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
             }
             __syncwarp();
         }
-        if (collide) {
-            if (lane == 0) {
-                double4 cs = P.cells.state[a];
-                ntc_collide<Prec>(g, meta.z, step, n, cs.z, cs.x, cs.y, st, wt.collisions, wt.candidates);
-                P.cells.state[a] = cs;
+        if (collide && lane == 0) {
+            if (pairs > 0) {
+                StageVel<Prec> vel;
+                vel.vx = st.vx;
+                vel.vy = st.vy;
+                vel.vz = st.vz;
+                ntc_run<real>(g.seed, meta.z, step, n, pairs, cs.x, vel, st.perm, wt.collisions);
+                wt.candidates += (unsigned long long)pairs;
             }
-            __syncwarp();
+            P.cells.state[a] = cs;
         }
+        if (staged) __syncwarp();
         if (sample) {
             double m[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             for (int r0 = 0; r0 < n; r0 += 32) {  // y-binned profiles, member by member
@@ -1463,12 +1609,13 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
             const bool valid = s < n;
             Particle p;
             unsigned key = 0xffffffffu;
+            bool wall = false;
             const unsigned addr = cell_slot(meta.x, meta.y, nb, nt, (unsigned)s);
             if (valid) {
                 RecA ra = Ain[addr];
                 RecB rb = Bin[addr];
                 Prec::unpack(ra, rb, p);
-                if (MODE != MODE_SORT) {
+                if (staged) {
                     p.v[0] = st.vx[s];
                     p.v[1] = st.vy[s];
                     p.v[2] = st.vz[s];
@@ -1481,7 +1628,13 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
                     mt.wall_hits = mt.reseeds = 0;
                     mt.cross[0] = mt.cross[1] = mt.cross[2] = 0;
                     mt.err = 0;
-                    const bool left_voxel = Prec::move(g, p, move_step, mt);
+                    if (MODE == MODE_FUSED) {
+                        wall = !Prec::move_open(g, p, mt);
+                        if (!wall) key = moved_cell<Prec>(g, p, a, mt.err, wt.stranded);
+                    } else {
+                        const bool left_voxel = Prec::move(g, p, move_step, mt);
+                        key = left_voxel ? moved_cell<Prec>(g, p, a, mt.err, wt.stranded) : (unsigned)a;
+                    }
                     wt.wall_hits += mt.wall_hits;
                     wt.reseeds += mt.reseeds;
                     wt.cross[0] += mt.cross[0];
@@ -1489,19 +1642,26 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
                     wt.cross[2] += mt.cross[2];
                     wt.err |= mt.err;
                     wt.moved += 1;
-                    const int ac = left_voxel ? __ldg(g.cell_map + Prec::cell_global(g, p)) : a;
-                    if (ac < 0) {
-                        // The reference aborts here (dsmc/system.h:134-142); the
-                        // particle sits in solid and its next move re-seeds it
-                        // (dsmc/moleculemover.cpp:57-60), so keep it in this cell.
-                        wt.err |= DSMC_EBIT_STRANDED;
-                        ++wt.stranded;
-                        key = (unsigned)a;
-                    } else {
-                        key = (unsigned)ac;
-                    }
                 } else {
                     key = (unsigned)a;
+                }
+            }
+            if (MODE == MODE_FUSED) {
+                // wall flights: the record, accelerated, goes back to its
+                // input slot, the slot to the list
+                const unsigned wm = __ballot_sync(0xffffffffu, wall);
+                if (wm) {
+                    unsigned at = 0;
+                    if (lane == __ffs(wm) - 1) at = atomicAdd(&P.status->walls, (unsigned)__popc(wm));
+                    at = __shfl_sync(0xffffffffu, at, __ffs(wm) - 1) + (unsigned)__popc(wm & ((1u << lane) - 1u));
+                    if (wall) {
+                        RecA ra;
+                        RecB rb;
+                        Prec::pack(p, ra, rb);
+                        Bio[addr] = rb;
+                        if (at < P.parts.walls_cap) P.parts.walls[at] = make_int2((int)addr, a);
+                        else wt.err |= DSMC_EBIT_SPILL_FULL;  // cannot happen: one entry per slot at most
+                    }
                 }
             }
             if (MODE == MODE_INPLACE) {
@@ -1516,70 +1676,78 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
                     if (P.do_move || collide) Bio[addr] = rb;
                 }
             } else {
-                // Warp-aggregated counting-sort insert into the new cell's top slots.
-                const unsigned peers = __match_any_sync(0xffffffffu, key);
-                const int leader = __ffs(peers) - 1;
-                const unsigned lower = peers & ((1u << lane) - 1u);
-                unsigned slot0 = 0;
-                if (valid && lane == leader) slot0 = atomicAdd(&top_out[key], (unsigned)__popc(peers));
-                slot0 = __shfl_sync(0xffffffffu, slot0, leader);
-                bool spilled = false;
-                if (valid) {
-                    const unsigned k = slot0 + (unsigned)__popc(lower);
-                    RecA ra;
-                    RecB rb;
-                    Prec::pack(p, ra, rb);
-                    const int4 km = key == (unsigned)a ? meta : P.cells.meta[key];
-                    // a top slot may not reach the slots the cell's owner can
-                    // fill from the bottom (at most its input occupancy)
-                    const unsigned room =
-                        P.top_only ? (unsigned)km.y
-                                   : (unsigned)km.y - min((unsigned)km.y, bot_in[key] + top_in[key]);
-                    if (k < room) {
-                        const unsigned dst = (unsigned)(km.x + km.y) - 1u - k;
-                        Aout[dst] = ra;
-                        Bout[dst] = rb;
-                    } else {
-                        spilled = true;
-                        const unsigned si = atomicAdd(&P.status->spill, 1u);
-                        if (si < P.parts.spill_cap) {
-                            SpillRec &sr = P.parts.spill[si];
-                            if (sizeof(real) == 8) {
-                                sr.ra = *reinterpret_cast<const double4 *>(&ra);
-                                sr.rb = *reinterpret_cast<const double4 *>(&rb);
-                            } else {
-                                sr.a = *reinterpret_cast<const uint4 *>(&ra);
-                                sr.b = *reinterpret_cast<const uint4 *>(&rb);
-                            }
-                            sr.cell = (int)key;
-                        } else {
-                            wt.err |= DSMC_EBIT_SPILL_FULL;
-                        }
-                    }
-                }
-                // spilled slots are given back, so the counter ends at the
-                // number of particles actually placed in the top segment
-                const unsigned over = __ballot_sync(0xffffffffu, spilled) & peers;
-                if (valid && lane == leader && over) atomicSub(&top_out[key], (unsigned)__popc(over));
+                insert_particle<Prec>(P, p, valid && !wall, key, wt.err);
             }
+        }
+        meta = next_meta;
+        nb = next_nb;
+        nt = next_nt;
+    }
+    if (wt.sys >= 0) flush_tally(P, wt, lane);
+    if (MODE != MODE_FUSED) end_pass(P);  // a fused pass ends with its wall flights
+}
+
+// The general mover for the wall flights that a fused pass listed, then their
+// placement and the pass's end.  Claims as place_walls_kernel's.
+constexpr int G_WARPS = 4;
+template <class Prec> __global__ void __launch_bounds__(32 * G_WARPS) pass_walls_kernel(PassParams P) {
+    typedef typename Prec::RecA RecA;
+    typedef typename Prec::RecB RecB;
+    const int lane = threadIdx.x & 31;
+    const volatile Status *vs = P.status;
+    if (vs->halted) return;
+    const uint32_t move_step = vs->step + 1;
+    const unsigned nwalls = min(vs->walls, P.parts.walls_cap);
+    const RecA *Ain = reinterpret_cast<const RecA *>(P.parts.A[P.cur]);
+    const RecB *Bin = reinterpret_cast<const RecB *>(P.parts.B[P.cur]);
+    WarpTally wt;
+    wt.collisions = wt.candidates = wt.wall_hits = wt.reseeds = wt.moved = wt.stranded = 0;
+    wt.cross[0] = wt.cross[1] = wt.cross[2] = 0;
+    wt.err = 0;
+    wt.sys = -1;
+    const unsigned nw = gridDim.x * G_WARPS;
+    const unsigned claim = min(32u, max(1u, (nwalls + nw - 1u) / nw));
+    for (;;) {
+        unsigned i0 = 0;
+        if (lane == 0) i0 = atomicAdd(&P.status->walls_taken, claim);
+        i0 = __shfl_sync(0xffffffffu, i0, 0);
+        if (i0 >= nwalls) break;
+        const unsigned i = i0 + lane;
+        const bool valid = (unsigned)lane < claim && i < nwalls;
+        const int2 e = valid ? P.parts.walls[i] : make_int2(0, -1);  // {input slot, source cell}
+        const int esys = valid ? P.cells.meta[e.y].w : -1;
+        // one system at a time: a warp's counts go to one system's tally
+        for (unsigned todo = __ballot_sync(0xffffffffu, valid); todo;) {
+            const int sys = __shfl_sync(0xffffffffu, esys, __ffs(todo) - 1);
+            const bool mine = valid && esys == sys;
+            todo &= ~__ballot_sync(0xffffffffu, mine);
+            if (sys != wt.sys) {
+                if (wt.sys >= 0) flush_tally(P, wt, lane);
+                wt.sys = sys;
+            }
+            typename Prec::Particle p;
+            unsigned key = 0;
+            if (mine) {
+                const SysDev &g = P.sys[sys];
+                Prec::unpack(Ain[e.x], Bin[e.x], p);
+                MoveTally mt;
+                mt.wall_hits = mt.reseeds = 0;
+                mt.cross[0] = mt.cross[1] = mt.cross[2] = 0;
+                mt.err = 0;
+                Prec::move(g, p, move_step, mt);
+                key = moved_cell<Prec>(g, p, e.y, mt.err, wt.stranded);
+                wt.wall_hits += mt.wall_hits;
+                wt.reseeds += mt.reseeds;
+                wt.cross[0] += mt.cross[0];
+                wt.cross[1] += mt.cross[1];
+                wt.cross[2] += mt.cross[2];
+                wt.err |= mt.err;
+            }
+            insert_particle<Prec>(P, p, mine, key, wt.err);
         }
     }
     if (wt.sys >= 0) flush_tally(P, wt, lane);
-
-    // End of pass: the last block to finish advances the step and halts the
-    // pipeline if anything spilled or failed.
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned done = atomicAdd(&P.status->blocks_done, 1u);
-        if (done == gridDim.x - 1) {
-            __threadfence();
-            if (P.advance_step) atomicAdd(&P.status->step, 1u);
-            if (atomicAdd(&P.status->spill, 0u) != 0u || (atomicAdd(&P.status->error, 0u) & DSMC_EBIT_FATAL) != 0u)
-                atomicExch(&P.status->halted, 1u);
-            atomicExch(&P.status->blocks_done, 0u);
-        }
-    }
+    end_pass(P);
 }
 
 }  // namespace dsmc

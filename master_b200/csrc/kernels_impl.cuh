@@ -2,6 +2,8 @@
 // translation unit defines DSMC_PREC (the policy) and DSMC_PREC_NS (the
 // namespace the launchers are placed in).
 #pragma once
+#include <algorithm>
+
 #include "engine.cuh"
 #include "kernels.h"
 
@@ -324,12 +326,25 @@ __global__ void k_cell_energy(const CellArrays cells, const ParticleArrays parts
 // ---- launchers --------------------------------------------------------------
 static size_t stage_bytes(int cap) { return WarpStage<Prec>::bytes(cap); }
 
+// The wall flights of a fused pass: a grid of the most resident blocks.
+static cudaError_t launch_pass_walls(const PassParams &P, cudaStream_t st) {
+    int dev = 0, sms = 0, nb = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pass_walls_kernel<Prec>, 32 * G_WARPS, 0);
+    if (e != cudaSuccess) return e;
+    pass_walls_kernel<Prec><<<std::max(1, nb * sms), 32 * G_WARPS, 0, st>>>(P);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_pass(int mode, const PassParams &P, int grid, int block, cudaStream_t st) {
     const size_t smem = stage_bytes(P.smem_cap) * (block / 32);
     switch (mode) {
         case MODE_FUSED:
             pass_kernel<Prec, MODE_FUSED><<<grid, block, smem, st>>>(P);
-            break;
+            if (cudaError_t e = cudaGetLastError()) return e;
+            return launch_pass_walls(P, st);
         case MODE_INPLACE:
             pass_kernel<Prec, MODE_INPLACE><<<grid, block, smem, st>>>(P);
             break;
