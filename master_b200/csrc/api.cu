@@ -115,7 +115,7 @@ struct dsmc_ctx {
     size_t slots = 0;
     int smem_cap = 32;
     // particles
-    DevBuf<unsigned char> A0, A1, B0, B1;
+    DevBuf<unsigned char> rec[2];    // {A, B} records of each buffer
     DevBuf<SpillRec> spill;
     unsigned spill_cap = 1u << 16;
     DevBuf<int2> walls;       // wall-flight list of the production pass (one entry per slot at most)
@@ -211,10 +211,10 @@ CellArrays cell_arrays(dsmc_ctx *ctx) {
 
 ParticleArrays particle_arrays(dsmc_ctx *ctx) {
     ParticleArrays p;
-    p.A[0] = ctx->A0.p;
-    p.A[1] = ctx->A1.p;
-    p.B[0] = ctx->B0.p;
-    p.B[1] = ctx->B1.p;
+    for (int b = 0; b < 2; ++b) {
+        p.A[b] = ctx->rec[b].p;
+        p.B[b] = ctx->rec[b].p ? ctx->rec[b].p + ctx->rec_half() : nullptr;
+    }
     p.spill = ctx->spill.p;
     p.spill_cap = ctx->spill_cap;
     p.walls = ctx->walls.p;
@@ -286,10 +286,8 @@ int relayout(dsmc_ctx *ctx, long long total) {
     ctx->smem_cap = (int)((maxcap + 31u) & ~31u);
     ctx->slots = slots;
     const size_t half = ctx->rec_half();
-    CK(ctx->A0.ensure_grow(slots * half));
-    CK(ctx->A1.ensure_grow(slots * half));
-    CK(ctx->B0.ensure_grow(slots * half));
-    CK(ctx->B1.ensure_grow(slots * half));
+    CK(ctx->rec[0].ensure_grow(2 * slots * half));
+    CK(ctx->rec[1].ensure_grow(2 * slots * half));
     CK(ctx->key.ensure_grow(slots));
     CK(ctx->walls.ensure_grow(std::max<size_t>(slots, 1)));
     if (C) {
@@ -353,7 +351,7 @@ static int stage_present_set(dsmc_ctx *ctx, long long extra, const std::vector<c
     CK(cudaMemsetAsync(ctx->hist.p, 0, std::max(ctx->num_cells, 1) * sizeof(unsigned), ctx->stream));
     CK(cudaMemsetAsync(ctx->cursor.p, 0, sizeof(unsigned long long), ctx->stream));
     *staged = 0;
-    if (ctx->A0.p && ctx->num_cells) {
+    if (ctx->rec[0].p && ctx->num_cells) {
         for (size_t s = 0; s < ctx->systems.size(); ++s) {
             if (skipped(s)) continue;
             SysHost &h = *ctx->systems[s];
@@ -1701,7 +1699,7 @@ int dsmc_tallies_get(dsmc_ctx *ctx, int sys_id, dsmc_tallies *t) {
     // MeasureEnergy / MeasureTemperature (dsmc/statisticalproperty.cpp:21-71)
     // from the current velocities, summed per cell and then in cell order.
     const int C = h.active_end - h.active_begin;
-    if (C > 0 && ctx->A0.p) {
+    if (C > 0 && ctx->rec[0].p) {
         // kept by the context: a sampler reading this every few steps
         // allocates once, not on every read
         DevBuf<double> &ce = ctx->cell_energy;

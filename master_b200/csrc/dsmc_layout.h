@@ -16,13 +16,18 @@
 // and the set the pass clears for the pass after next), so no count a pass
 // reads is written during it.
 //
-// Record formats (structure of arrays, 16-byte vectors):
+// Record formats: slot s of a buffer holds the pair {A, B} side by side (A at
+// element 2s of an array of either's size, B at 2s + 1), so that a particle is
+// one 32-byte sector (split precision) and a cell's members one run of memory:
+// the members fill a third of the slots, and with A and B in arrays of their
+// own DRAM opened twice the rows for half the bytes each.
 //   split precision:  A = uint4 {voxel (i | j<<11 | k<<22), ox, oy, oz (fp32 bits)}
 //                     B = float4 {vx, vy, vz, id (u32 bits)}
 //                     ox,oy,oz in [0,1) voxel units; v in reduced units.
 //   fp64 reference:   A = double4 {rx, ry, rz, id}   B = double4 {vx, vy, vz, 0}
 //                     the reference's own representation (dsmc/system.h:74-75).
 #pragma once
+#include <stddef.h>
 #include <stdint.h>
 #include <vector_types.h>
 
@@ -47,6 +52,14 @@
 #define DSMC_VOX_K(p) ((int)((p) >> 22))
 
 namespace dsmc {
+
+// Element of slot s in a buffer's A (and, from B's base, B) elements.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline size_t rec_at(long long s) {
+    return 2 * (size_t)s;
+}
 
 // Slot address of the s-th occupied particle of a cell (bottom, then top).
 #ifdef __CUDACC__
@@ -153,8 +166,8 @@ struct CellArrays {
 };
 
 struct ParticleArrays {
-    void *A[2];
-    void *B[2];
+    void *A[2];                // element rec_at(s): slot s's A record
+    void *B[2];                // the same memory one element on: its B record
     SpillRec *spill;
     unsigned spill_cap;
     int2 *walls;               // production pass: {output slot, source cell} of flights that meet a wall

@@ -1381,8 +1381,8 @@ __device__ __forceinline__ void insert_particle(const PassParams &P, const typen
                                                                 P.cells.bot[P.cin][key] + P.cells.top[P.cin][key]);
         if (k < room) {
             const unsigned dst = (unsigned)(km.x + km.y) - 1u - k;
-            reinterpret_cast<RecA *>(P.parts.A[P.cur ^ 1])[dst] = ra;
-            reinterpret_cast<RecB *>(P.parts.B[P.cur ^ 1])[dst] = rb;
+            reinterpret_cast<RecA *>(P.parts.A[P.cur ^ 1])[rec_at(dst)] = ra;
+            reinterpret_cast<RecB *>(P.parts.B[P.cur ^ 1])[rec_at(dst)] = rb;
         } else {
             spilled = true;
             const unsigned si = atomicAdd(&P.status->spill, 1u);
@@ -1530,7 +1530,7 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
             for (int s = lane; s < n; s += 32) {
                 real v[3];
                 uint32_t id;
-                Prec::stage_load(Ain, Bin, cell_slot(meta.x, meta.y, nb, nt, s), v, id);
+                Prec::stage_load(Ain, Bin, rec_at(cell_slot(meta.x, meta.y, nb, nt, s)), v, id);
                 st.vx[s] = v[0];
                 st.vy[s] = v[1];
                 st.vz[s] = v[2];
@@ -1568,7 +1568,7 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
                 if (ok) {
                     const int s = st.perm[r];
                     vz = (double)st.vz[s];
-                    bin = profile_bin(g, Prec::y_of(g, Ain[cell_slot(meta.x, meta.y, nb, nt, s)]));
+                    bin = profile_bin(g, Prec::y_of(g, Ain[rec_at(cell_slot(meta.x, meta.y, nb, nt, s))]));
                 }
                 profile_add_warp(g, ok, bin, 1.0, vz, 0.5 * g.mass * vz * vz);
                 if (ok) profile_vx(g, (double)st.vx[st.perm[r]]);
@@ -1612,8 +1612,8 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
             bool wall = false;
             const unsigned addr = cell_slot(meta.x, meta.y, nb, nt, (unsigned)s);
             if (valid) {
-                RecA ra = Ain[addr];
-                RecB rb = Bin[addr];
+                RecA ra = Ain[rec_at(addr)];
+                RecB rb = Bin[rec_at(addr)];
                 Prec::unpack(ra, rb, p);
                 if (staged) {
                     p.v[0] = st.vx[s];
@@ -1658,7 +1658,7 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
                         RecA ra;
                         RecB rb;
                         Prec::pack(p, ra, rb);
-                        Bio[addr] = rb;
+                        Bio[rec_at(addr)] = rb;
                         if (at < P.parts.walls_cap) P.parts.walls[at] = make_int2((int)addr, a);
                         else wt.err |= DSMC_EBIT_SPILL_FULL;  // cannot happen: one entry per slot at most
                     }
@@ -1670,10 +1670,10 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
                     RecB rb;
                     Prec::pack(p, ra, rb);
                     if (P.do_move) {
-                        Aio[addr] = ra;
+                        Aio[rec_at(addr)] = ra;
                         P.cells.key[addr] = key;
                     }
-                    if (P.do_move || collide) Bio[addr] = rb;
+                    if (P.do_move || collide) Bio[rec_at(addr)] = rb;
                 }
             } else {
                 insert_particle<Prec>(P, p, valid && !wall, key, wt.err);
@@ -1729,7 +1729,7 @@ template <class Prec> __global__ void __launch_bounds__(32 * G_WARPS) pass_walls
             unsigned key = 0;
             if (mine) {
                 const SysDev &g = P.sys[sys];
-                Prec::unpack(Ain[e.x], Bin[e.x], p);
+                Prec::unpack(Ain[rec_at(e.x)], Bin[rec_at(e.x)], p);
                 MoveTally mt;
                 mt.wall_hits = mt.reseeds = 0;
                 mt.cross[0] = mt.cross[1] = mt.cross[2] = 0;

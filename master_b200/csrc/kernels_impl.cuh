@@ -179,7 +179,7 @@ __global__ void k_field_accumulate(const SysDev *sys, int s, const CellArrays ce
         for (unsigned q = lane; q < nb + nt; q += 32) {
             Particle p;
             const unsigned addr = cell_slot(m.x, m.y, nb, nt, q);
-            Prec::unpack(Ain[addr], Bin[addr], p);
+            Prec::unpack(Ain[rec_at(addr)], Bin[rec_at(addr)], p);
             double rr[3];
             Maker<Prec>::position(g, p, rr);
             int c[3];
@@ -219,8 +219,8 @@ __global__ void k_gather(const CellArrays cells, const ParticleArrays parts, int
         }
         for (unsigned s = lane; s < n; s += 32) {
             const unsigned addr = cell_slot(m.x, m.y, nb, nt, s);
-            A[at + s] = Ain[addr];
-            B[at + s] = Bin[addr];
+            A[at + s] = Ain[rec_at(addr)];
+            B[at + s] = Bin[rec_at(addr)];
             key[at + s] = a;
         }
         if (lane == 0 && n) atomicAdd(&hist[a], n);
@@ -260,8 +260,8 @@ __global__ void k_insert(const CellArrays cells, const ParticleArrays parts, int
             atomicOr(err, DSMC_EBIT_SPILL_FULL);
             continue;
         }
-        Aout[m.x + slot] = A[i];
-        Bout[m.x + slot] = B[i];
+        Aout[rec_at(m.x + (long long)slot)] = A[i];
+        Bout[rec_at(m.x + (long long)slot)] = B[i];
     }
 }
 
@@ -282,7 +282,7 @@ __global__ void k_to_fp64(const SysDev *sys, int s, const CellArrays cells, cons
         for (unsigned q = lane; q < nb + nt; q += 32) {
             Particle p;
             const unsigned addr = cell_slot(m.x, m.y, nb, nt, q);
-            Prec::unpack(Ain[addr], Bin[addr], p);
+            Prec::unpack(Ain[rec_at(addr)], Bin[rec_at(addr)], p);
             const long long i = (long long)p.id - (long long)id_base;
             if (i < 0 || i >= cap) {
                 atomicOr(err, DSMC_EBIT_CELL);
@@ -314,7 +314,7 @@ __global__ void k_cell_energy(const CellArrays cells, const ParticleArrays parts
         const unsigned nt = min(cells.top[cin][a], (unsigned)m.y - nb);
         double e = 0;
         for (unsigned q = lane; q < nb + nt; q += 32) {
-            const RecB b = Bin[cell_slot(m.x, m.y, nb, nt, q)];
+            const RecB b = Bin[rec_at(cell_slot(m.x, m.y, nb, nt, q))];
             const double x = (double)b.x, y = (double)b.y, z = (double)b.z;
             e += x * x + y * y + z * z;
         }

@@ -67,6 +67,25 @@ __device__ __forceinline__ void cp_async_wait(int pending) {
     }
 }
 
+// A particle record {A, B} of slot s in one 32-byte access.  (With A and B in
+// arrays of their own a mover took four sectors, each half used, and
+// place_movers 174 us at 256^3; now 108.)
+__device__ __forceinline__ void load_record(const void *A, long long s, uint4 &a, float4 &b) {
+    uint32_t r[8];
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "l"(reinterpret_cast<const uint4 *>(A) + rec_at(s))
+                 : "memory");
+    a = make_uint4(r[0], r[1], r[2], r[3]);
+    b = make_float4(__uint_as_float(r[4]), __uint_as_float(r[5]), __uint_as_float(r[6]), __uint_as_float(r[7]));
+}
+__device__ __forceinline__ void store_record(void *A, long long s, const uint4 &a, const float4 &b) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(reinterpret_cast<uint4 *>(A) + rec_at(s)),
+                 "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(__float_as_uint(b.x)), "r"(__float_as_uint(b.y)),
+                 "r"(__float_as_uint(b.z)), "r"(__float_as_uint(b.w))
+                 : "memory");
+}
+
 // Input occupancy of active cell a (clamped to its capacity).
 __device__ __forceinline__ void input_counts(const PassParams &P, int a, const int4 &m, unsigned &nb, unsigned &nt) {
     nb = min(P.cells.bot[P.cin][a], (unsigned)m.y);
@@ -122,13 +141,13 @@ struct RankVel {
     float4 *b;
     const int *perm;
     __device__ __forceinline__ void get(int r, float &x, float &y, float &z) const {
-        const float4 v = b[perm[r]];
+        const float4 v = b[rec_at(perm[r])];
         x = v.x;
         y = v.y;
         z = v.z;
     }
     __device__ __forceinline__ void set(int r, float x, float y, float z) const {
-        float *q = reinterpret_cast<float *>(b + perm[r]);
+        float *q = reinterpret_cast<float *>(b + rec_at(perm[r]));
         q[0] = x;
         q[1] = y;
         q[2] = z;
@@ -141,13 +160,13 @@ struct IdentityPerm {
 struct SlotVel {
     float4 *b;
     __device__ __forceinline__ void get(int s, float &x, float &y, float &z) const {
-        const float4 v = b[s];
+        const float4 v = b[rec_at(s)];
         x = v.x;
         y = v.y;
         z = v.z;
     }
     __device__ __forceinline__ void set(int s, float x, float y, float z) const {
-        float *q = reinterpret_cast<float *>(b + s);
+        float *q = reinterpret_cast<float *>(b + rec_at(s));
         q[0] = x;
         q[1] = y;
         q[2] = z;
@@ -292,7 +311,7 @@ __global__ void __launch_bounds__(32 * C_WARPS) collide_cells_kernel(const __gri
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int f = f0 + 32 * u;
-                    v[u] = f < total ? __float_as_uint(Bin[W.slot[f]].w) : 0u;
+                    v[u] = f < total ? __float_as_uint(Bin[rec_at(W.slot[f])].w) : 0u;
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
@@ -467,8 +486,6 @@ __global__ void __launch_bounds__(32 * C_WARPS) sample_cells_kernel(const __grid
     const volatile Status *vs = P.status;
     if (vs->halted) return;
     const uint32_t step = vs->step;
-    const float4 *Bin = reinterpret_cast<const float4 *>(P.parts.B[P.cur]);
-    const uint4 *Ain = reinterpret_cast<const uint4 *>(P.parts.A[P.cur]);
     unsigned *H = hist[threadIdx.x >> 5];
     for (int b = lane; b < SHIST; b += 32) H[b] = 0;
     __syncwarp();
@@ -532,11 +549,13 @@ __global__ void __launch_bounds__(32 * C_WARPS) sample_cells_kernel(const __grid
                 double x = 0, y = 0, z = 0;
                 if (ok) {
                     const int sl = member_slot(cb, cc, cnb, cnt, q);
-                    const float4 b = Bin[sl];
+                    uint4 ra;
+                    float4 b;
+                    load_record(P.parts.A[P.cur], sl, ra, b);
                     x = b.x;
                     y = b.y;
                     z = b.z;
-                    bin = profile_bin(g, Split32::y_of(g, Ain[sl]));
+                    bin = profile_bin(g, Split32::y_of(g, ra));
                     v[0] += x;
                     v[1] += y;
                     v[2] += z;
@@ -585,14 +604,24 @@ constexpr int M_WARPS = 4;
 constexpr int DEPTH = 4;  // cells staged ahead of the one in work
 
 struct MoveTab {
-    int base[32], cap[32];
-    unsigned nb[32], nt[32];
-    int sys[32];
+    int4 t[32];  // {first slot, slots, bottom | top << 16 occupancy, system}: one load per cell
     int first, ncell;
+    __device__ __forceinline__ static int nb(const int4 &c) { return c.z & 0xffff; }
+    __device__ __forceinline__ static int nt(const int4 &c) { return (int)((unsigned)c.z >> 16); }
 };
+// The staging ring: records of 32 bytes, the halves of every other group of
+// four swapped so that eight lanes' 16-byte reads of one half of consecutive
+// records fall into different banks.
 template <int R> struct MoveSmem {
-    uint4 A[R];
-    float4 B[R];
+    uint4 rec[2 * R];
+    __device__ __forceinline__ static int at(int r, int half) { return 2 * r + (half ^ ((r >> 2) & 1)); }
+    __device__ __forceinline__ uint4 a(int r) const { return rec[at(r, 0)]; }
+    __device__ __forceinline__ float4 b(int r) const { return *reinterpret_cast<const float4 *>(&rec[at(r, 1)]); }
+    __device__ __forceinline__ uint32_t id(int r) const { return rec[at(r, 1)].w; }
+    __device__ __forceinline__ void set(int r, const uint4 &ra, const float4 &rb) {
+        rec[at(r, 0)] = ra;
+        *reinterpret_cast<float4 *>(&rec[at(r, 1)]) = rb;
+    }
     MoveTab tab[2];
     uint16_t pref[R + 2];  // two-pass placement: stayers before each member
 };
@@ -620,34 +649,36 @@ __device__ __forceinline__ bool first_flight(const SysDev &g, Split32::Particle 
 
 // A system's constants of the first flight, held in registers.
 struct FlightConst {
-    float inv_vox[3], dt, accel;
-    int flow_dir;
+    float inv_vox[3], dt, accel[3];  // accel: the flow axis's accel_dt_f, 0 on the others
 };
 __device__ __forceinline__ FlightConst flight_const(const SysDev &g) {
     FlightConst k;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) k.inv_vox[d] = g.inv_vox_f[d];
+    for (int d = 0; d < 3; ++d) {
+        k.inv_vox[d] = g.inv_vox_f[d];
+        k.accel[d] = g.flow_dir == d ? g.accel_dt_f : 0.0f;
+    }
     k.dt = g.dt_f;
-    k.accel = g.accel_dt_f;
-    k.flow_dir = g.flow_dir;
     return k;
 }
 // first_flight on the packed record itself: the voxel index is never
 // unpacked (a stayer changes only its offsets, a mover only its velocity).
-// Bit for bit what unpack + first_flight + pack give.
+// The values that unpack + first_flight + pack give.  [0, 1) is tested on the
+// bits: of the floats, exactly those from 0 to below 1 are below 0x3f800000 as
+// unsigned numbers (negative ones and NaNs are above).
 __device__ __forceinline__ bool first_flight_raw(const FlightConst &k, uint4 &a, float4 &b) {
-    b.x = k.flow_dir == 0 ? b.x + k.accel : b.x;
-    b.y = k.flow_dir == 1 ? b.y + k.accel : b.y;
-    b.z = k.flow_dir == 2 ? b.z + k.accel : b.z;
-    if (a.y >> 31) return false;  // the voxel is not empty: general mover
-    const float x0 = fmaf(b.x * k.inv_vox[0], k.dt, __uint_as_float(a.y));
-    const float x1 = fmaf(b.y * k.inv_vox[1], k.dt, __uint_as_float(a.z));
-    const float x2 = fmaf(b.z * k.inv_vox[2], k.dt, __uint_as_float(a.w));
-    const bool stay = (x0 >= 0.0f) & (x0 < 1.0f) & (x1 >= 0.0f) & (x1 < 1.0f) & (x2 >= 0.0f) & (x2 < 1.0f);
+    b.x += k.accel[0];
+    b.y += k.accel[1];
+    b.z += k.accel[2];
+    const uint32_t x0 = __float_as_uint(fmaf(b.x * k.inv_vox[0], k.dt, __uint_as_float(a.y)));
+    const uint32_t x1 = __float_as_uint(fmaf(b.y * k.inv_vox[1], k.dt, __uint_as_float(a.z)));
+    const uint32_t x2 = __float_as_uint(fmaf(b.z * k.inv_vox[2], k.dt, __uint_as_float(a.w)));
+    // (the flag of a particle whose voxel is not empty, the general mover's, is a.y's sign bit)
+    const bool stay = (max(max(x0, x1), x2) < 0x3f800000u) & ((int)a.y >= 0);
     if (stay) {
-        a.y = __float_as_uint(x0);
-        a.z = __float_as_uint(x1);
-        a.w = __float_as_uint(x2);
+        a.y = x0;
+        a.z = x1;
+        a.w = x2;
     }
     return stay;
 }
@@ -658,7 +689,7 @@ __device__ __forceinline__ bool first_flight_raw(const FlightConst &k, uint4 &a,
 // Returns the number of stayers.  All lanes call.
 template <int R, int NR>
 __device__ __forceinline__ unsigned place_sorted(const FlightConst &fc, const MoveSmem<R> &W, int tail, int base,
-                                                 int n, int nb, uint4 *Aout, float4 *Bout, int lane) {
+                                                 int n, int nb, void *out, int lane) {
     const unsigned below = (1u << lane) - 1u;
     uint4 ra[NR];
     float4 rb[NR];
@@ -673,8 +704,8 @@ __device__ __forceinline__ unsigned place_sorted(const FlightConst &fc, const Mo
         if (valid) {
             int r = tail + q;
             if (r >= R) r -= R;
-            ra[k] = W.A[r];
-            rb[k] = W.B[r];
+            ra[k] = W.a(r);
+            rb[k] = W.b(r);
             stay[k] = first_flight_raw(fc, ra[k], rb[k]);
         }
         id[k] = valid ? __float_as_uint(rb[k].w) : 0xffffffffu;
@@ -710,8 +741,7 @@ __device__ __forceinline__ unsigned place_sorted(const FlightConst &fc, const Mo
             const unsigned dst =
                 stay[k] ? (unsigned)base + (q < nb ? fs_before + (unsigned)__popc(fast[k] & bm[k] & below) : pb[k]) + add[k]
                         : (unsigned)(base + n) - 1u - mv_before - (unsigned)__popc(slow[k] & below);
-            Aout[dst] = ra[k];
-            Bout[dst] = rb[k];
+            store_record(out, dst, ra[k], rb[k]);
         }
         fs_before += (unsigned)__popc(fast[k] & bm[k]);
         mv_before += (unsigned)__popc(slow[k]);
@@ -728,7 +758,7 @@ __device__ __forceinline__ unsigned place_sorted(const FlightConst &fc, const Mo
 // nfs[k]: stayers of cell k.  All lanes call.
 template <int R>
 __device__ __forceinline__ void place_pair(const FlightConst &fc, const MoveSmem<R> &W, int tail, const int base[2],
-                                          const int n[2], const int nb[2], uint4 *Aout, float4 *Bout, int lane,
+                                          const int n[2], const int nb[2], void *out, int lane,
                                           unsigned nfs[2]) {
     const unsigned below = (1u << lane) - 1u;
     uint4 ra[2];
@@ -746,8 +776,8 @@ __device__ __forceinline__ void place_pair(const FlightConst &fc, const MoveSmem
         if (valid) {
             int r = tl[k] + lane;
             if (r >= R) r -= R;
-            ra[k] = W.A[r];
-            rb[k] = W.B[r];
+            ra[k] = W.a(r);
+            rb[k] = W.b(r);
             stay[k] = first_flight_raw(fc, ra[k], rb[k]);
         }
         id[k] = valid ? __float_as_uint(rb[k].w) : 0xffffffffu;
@@ -778,13 +808,15 @@ __device__ __forceinline__ void place_pair(const FlightConst &fc, const MoveSmem
             const unsigned dst =
                 stay[k] ? (unsigned)base[k] + (lane < nb[k] ? (unsigned)__popc(fast[k] & bm[k] & below) : pb[k]) + add[k]
                         : (unsigned)(base[k] + n[k]) - 1u - (unsigned)__popc(slow[k] & below);
-            Aout[dst] = ra[k];
-            Bout[dst] = rb[k];
+            store_record(out, dst, ra[k], rb[k]);
         }
         nfs[k] = (unsigned)__popc(fast[k]);
     }
 }
 
+// 64 B per particle; at 256^3 (3.15e7 particles) 566 us with A and B apart and
+// five table words per cell, 549 us (3.7 TB/s) so.  Bound by its instructions
+// (about 400 per pair of cells, 0.5 issued per cycle and scheduler).
 // At most 128 registers (four blocks per SM): the compiler then keeps both
 // cells of a pair in flight; left to itself it may pick 96 and five blocks,
 // which measured slower.
@@ -798,10 +830,8 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
     if (vs->halted) return;
 
     MoveSmem<R> &W = reinterpret_cast<MoveSmem<R> *>(smem_raw)[wib];
-    const uint4 *Ain = reinterpret_cast<const uint4 *>(P.parts.A[P.cur]);
-    const float4 *Bin = reinterpret_cast<const float4 *>(P.parts.B[P.cur]);
-    uint4 *Aout = reinterpret_cast<uint4 *>(P.parts.A[P.cur ^ 1]);
-    float4 *Bout = reinterpret_cast<float4 *>(P.parts.B[P.cur ^ 1]);
+    const uint4 *in = reinterpret_cast<const uint4 *>(P.parts.A[P.cur]);
+    void *out = P.parts.A[P.cur ^ 1];
 
     const int C = P.cells.num_cells, CH = P.chunk;
     const int nchunks = (C + CH - 1) / CH;
@@ -824,11 +854,7 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
             if (nb + nt > (unsigned)R) atomicOr(&P.status->error, DSMC_EBIT_SMEM);  // the host sizes R above every cap
             // top slots free for arrivals this pass: above the input occupancy
             P.cells.room[a] = make_int2(m.x + m.y, m.y - (int)(nb + nt));
-            T.base[lane] = m.x;
-            T.cap[lane] = m.y;
-            T.nb[lane] = nb;
-            T.nt[lane] = nt;
-            T.sys[lane] = m.w;
+            T.t[lane] = make_int4(m.x, m.y, (int)(nb | nt << 16), m.w);  // (cells hold at most R <= 512)
         }
     };
     // Lane i publishes cell i's bottom occupancy and clears the set the next
@@ -862,16 +888,16 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
         while (ahead <= DEPTH && it <= ct + 1) {
             const MoveTab &T = W.tab[it & 1];
             if (ii >= T.ncell) return;
-            const int nb = (int)T.nb[ii], nt = (int)T.nt[ii];
+            const int4 c = T.t[ii];
+            const int nb = MoveTab::nb(c), nt = MoveTab::nt(c);
             const int n = min(nb + nt, R);
             if (used + n > R) return;
-            const int base = T.base[ii], cap = T.cap[ii];
-            for (int q = lane; q < n; q += 32) {
-                const int slot = member_slot(base, cap, nb, nt, q);
+            const int base = c.x, cap = c.y;
+            for (int h = lane; h < 2 * n; h += 32) {  // half h & 1 of member h >> 1
+                const int q = h >> 1;
                 int r = head + q;
                 if (r >= R) r -= R;
-                cp_async16(&W.A[r], Ain + slot);
-                cp_async16(&W.B[r], Bin + slot);
+                cp_async16(&W.rec[MoveSmem<R>::at(r, h & 1)], in + rec_at(member_slot(base, cap, nb, nt, q)) + (h & 1));
             }
             cp_async_commit();
             head += n;
@@ -898,16 +924,16 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
             continue;
         }
         stage_ahead();  // the cell in work is staged once this returns
+        const int4 c0 = T.t[ci], c1 = T.t[min(ci + 1, 31)];
+        const int pnb[2] = {MoveTab::nb(c0), MoveTab::nb(c1)};
+        const int pn[2] = {pnb[0] + MoveTab::nt(c0), pnb[1] + MoveTab::nt(c1)};
         // Two small cells of one system with sorted bottoms go together.
-        if (P.sorted_in && ahead >= 2 && ci + 1 < T.ncell && T.sys[ci + 1] == T.sys[ci] &&
-            T.sys[ci] == tsys && T.nb[ci] + T.nt[ci] <= 32u && T.nb[ci + 1] + T.nt[ci + 1] <= 32u) {
+        if (P.sorted_in && ahead >= 2 && ci + 1 < T.ncell && c1.w == c0.w && c0.w == tsys && pn[0] <= 32 && pn[1] <= 32) {
             cp_async_wait(ahead - 2);
             __syncwarp();
-            const int pn[2] = {(int)(T.nb[ci] + T.nt[ci]), (int)(T.nb[ci + 1] + T.nt[ci + 1])};
-            const int pnb[2] = {(int)T.nb[ci], (int)T.nb[ci + 1]};
-            const int pbase[2] = {T.base[ci], T.base[ci + 1]};
+            const int pbase[2] = {c0.x, c1.x};
             unsigned nfs[2];
-            place_pair<R>(fc, W, tail, pbase, pn, pnb, Aout, Bout, lane, nfs);
+            place_pair<R>(fc, W, tail, pbase, pn, pnb, out, lane, nfs);
             if (lane == ci) nfs_mine = nfs[0];
             if (lane == ci + 1) nfs_mine = nfs[1];
             const int m = pn[0] + pn[1];
@@ -923,9 +949,9 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
         cp_async_wait(ahead - 1);
         __syncwarp();
 
-        const int n = min((int)(T.nb[ci] + T.nt[ci]), R);
-        const int base = T.base[ci];
-        const int sys = T.sys[ci];
+        const int n = min(pn[0], R);
+        const int base = c0.x;
+        const int sys = c0.w;
         if (sys != tsys) {
             if (lane == 0 && tsys >= 0 && moved) atomicAdd(&P.tally[tsys].particle_steps, (unsigned long long)moved);
             moved = 0;
@@ -934,12 +960,12 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
         }
         const SysDev &g = P.sys[sys];
 
-        const int nb = min((int)T.nb[ci], n);
+        const int nb = min(pnb[0], n);
         auto ring = [&](int q) {
             const int r = tail + q;
             return r >= R ? r - R : r;
         };
-        auto rid = [&](int q) { return __float_as_uint(W.B[ring(q)].w); };
+        auto rid = [&](int q) { return W.id(ring(q)); };
         bool viol = false;
         if (!P.sorted_in)
             for (int q = lane; q + 1 < nb; q += 32) viol |= !(rid(q) < rid(q + 1));
@@ -949,9 +975,9 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
         // Stayers go to the bottom segment in id order, movers to the gap.
         unsigned n_fs;
         if (sorted && n <= 32) {
-            n_fs = place_sorted<R, 1>(fc, W, tail, base, n, nb, Aout, Bout, lane);
+            n_fs = place_sorted<R, 1>(fc, W, tail, base, n, nb, out, lane);
         } else if (sorted && n <= 64) {
-            n_fs = place_sorted<R, 2>(fc, W, tail, base, n, nb, Aout, Bout, lane);
+            n_fs = place_sorted<R, 2>(fc, W, tail, base, n, nb, out, lane);
         } else {
             // pass 1: every member's flight; the record goes back into the
             // ring and pref[q] counts the stayers before member q
@@ -963,9 +989,12 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
                 if (valid) {
                     const int r = ring(q);
                     Particle p;
-                    Split32::unpack(W.A[r], W.B[r], p);
+                    Split32::unpack(W.a(r), W.b(r), p);
                     stay = first_flight(g, p);
-                    Split32::pack(p, W.A[r], W.B[r]);
+                    uint4 ra;
+                    float4 rb;
+                    Split32::pack(p, ra, rb);
+                    W.set(r, ra, rb);
                 }
                 const unsigned fast = __ballot_sync(0xffffffffu, valid && stay);
                 if (valid) W.pref[q] = (uint16_t)(S + (unsigned)__popc(fast & below));
@@ -1003,8 +1032,7 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
                     } else {
                         dst = (unsigned)(base + n) - 1u - ((unsigned)q - W.pref[q]);
                     }
-                    Aout[dst] = W.A[r];
-                    Bout[dst] = W.B[r];
+                    store_record(out, dst, W.a(r), W.b(r));
                 }
             }
             n_fs = S;
@@ -1097,8 +1125,7 @@ __device__ __forceinline__ void insert_top(const PassParams &P, const Split32::P
         Split32::pack(p, ra, rb);
         if (j < (unsigned)rt.y) {
             const unsigned dst = (unsigned)rt.x - 1u - j;
-            reinterpret_cast<uint4 *>(P.parts.A[P.cur ^ 1])[dst] = ra;
-            reinterpret_cast<float4 *>(P.parts.B[P.cur ^ 1])[dst] = rb;
+            store_record(P.parts.A[P.cur ^ 1], dst, ra, rb);
         } else {
             spilled = true;
             const unsigned si = atomicAdd(&P.status->spill, 1u);
@@ -1182,8 +1209,7 @@ __global__ void __launch_bounds__(32 * P_WARPS, 5) place_movers_kernel(const __g
     PlaceSmem &W = smem[threadIdx.x >> 5];
     if (lane == 0) W.qn = 0;
     __syncwarp();
-    const uint4 *Aout = reinterpret_cast<const uint4 *>(P.parts.A[P.cur ^ 1]);
-    const float4 *Bout = reinterpret_cast<const float4 *>(P.parts.B[P.cur ^ 1]);
+    const void *out = P.parts.A[P.cur ^ 1];
 
     MoveCounts cnt;
     counts_reset(cnt);
@@ -1241,7 +1267,10 @@ __global__ void __launch_bounds__(32 * P_WARPS, 5) place_movers_kernel(const __g
             bool done = false, place = false, leave = false;
             unsigned key = 0;
             if (valid) {
-                Split32::unpack(Aout[slot], Bout[slot], p);
+                uint4 ra;
+                float4 rb;
+                load_record(out, slot, ra, rb);
+                Split32::unpack(ra, rb, p);
                 const SysDev &g = P.sys[psys];
                 done = Split32::move_open(g, p, mt);
                 if (done) place = new_cell(g, p, src, key, leave, cnt, mt.err);
@@ -1280,8 +1309,7 @@ __global__ void __launch_bounds__(32 * W_WARPS) place_walls_kernel(const __grid_
     if (vs->halted) return;
     const uint32_t move_step = vs->step + 1;
     const unsigned nwalls = min(vs->walls, P.parts.walls_cap);
-    const uint4 *Aout = reinterpret_cast<const uint4 *>(P.parts.A[P.cur ^ 1]);
-    const float4 *Bout = reinterpret_cast<const float4 *>(P.parts.B[P.cur ^ 1]);
+    const void *out = P.parts.A[P.cur ^ 1];
     MoveCounts cnt;
     counts_reset(cnt);
     int tsys = -1;
@@ -1316,7 +1344,12 @@ __global__ void __launch_bounds__(32 * W_WARPS) place_walls_kernel(const __grid_
         // the lanes of a warp share their system unless it is mixed; a mixed
         // warp moves its lanes one system at a time
         const int s0 = esys;
-        if (valid) Split32::unpack(Aout[e.x], Bout[e.x], p);
+        if (valid) {
+            uint4 ra;
+            float4 rb;
+            load_record(out, e.x, ra, rb);
+            Split32::unpack(ra, rb, p);
+        }
         for (unsigned todo = __ballot_sync(0xffffffffu, valid); todo;) {
             const int sys = __shfl_sync(0xffffffffu, s0, __ffs(todo) - 1);
             const bool mine = valid && s0 == sys;
@@ -1357,8 +1390,6 @@ __global__ void __launch_bounds__(32 * W_WARPS) place_walls_kernel(const __grid_
 __global__ void put_records_kernel(const SysDev *sys, int s, const CellArrays cells, const ParticleArrays parts,
                                    int cur, int cin, long long n, const uint4 *rec, Status *status) {
     const SysDev &g = sys[s];
-    uint4 *A = reinterpret_cast<uint4 *>(parts.A[cur]);
-    float4 *B = reinterpret_cast<float4 *>(parts.B[cur]);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const uint4 ra = rec[2 * i];
         const uint4 rbits = rec[2 * i + 1];
@@ -1379,8 +1410,7 @@ __global__ void put_records_kernel(const SysDev *sys, int s, const CellArrays ce
         const unsigned j = atomicAdd(&cells.top[cin][ac], 1u);
         if (nb + j < (unsigned)m.y) {
             const unsigned dst = (unsigned)(m.x + m.y) - 1u - j;
-            A[dst] = ra;
-            B[dst] = rb;
+            store_record(parts.A[cur], dst, ra, rb);
         } else {
             atomicSub(&cells.top[cin][ac], 1u);
             const unsigned si = atomicAdd(&status->spill, 1u);
