@@ -1259,7 +1259,8 @@ __device__ __forceinline__ void ntc_loop(Draws &rs, int n, int pairs, double &vr
         const real ub = rs.template uniform<real>();
         int ip0, ip1;
         ntc_pick(ua, ub, n, ip0, ip1);
-        const int s0 = perm[ip0], s1 = perm[ip1];
+        int s0, s1;
+        perm.pick(ip0, ip1, s0, s1);
         real ax, ay, az, bx, by, bz;
         vel.get(s0, ax, ay, az);
         vel.get(s1, bx, by, bz);
@@ -1277,12 +1278,20 @@ __device__ __forceinline__ void ntc_loop(Draws &rs, int n, int pairs, double &vr
     }
     vr_max = crm;
 }
+// Member slots by id rank.
+struct RankTable {
+    const uint16_t *slot;
+    __device__ __forceinline__ void pick(int r0, int r1, int &s0, int &s1) const {
+        s0 = slot[r0];
+        s1 = slot[r1];
+    }
+};
 template <class real, class Vel>
 __device__ void ntc_run(uint64_t seed, int cell_global_index, uint32_t step, int n, int pairs, double &vr_max,
                         Vel vel, const uint16_t *perm, unsigned long long &collisions) {
     DrawStream rs;
     rs.init(seed, (uint32_t)cell_global_index, step, DSMC_TAG_COLLIDE);
-    ntc_loop<real>(rs, n, pairs, vr_max, vel, perm, collisions);
+    ntc_loop<real>(rs, n, pairs, vr_max, vel, RankTable{perm}, collisions);
 }
 
 template <class Prec> struct StageVel {

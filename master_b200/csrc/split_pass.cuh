@@ -6,9 +6,8 @@
 //   collide_cells  Cell::prepare + Cell::collide (dsmc/cell.cpp:42-111) of
 //                  every cell.
 //                  Per chunk of (up to 32) consecutive cells lane i selects for cell
-//                  i; the warp ranks each colliding cell's particles by id
-//                  (the reference's member order) into shared memory, then
-//                  every lane runs the candidate loop of its own cell.
+//                  i and runs its candidate loop; the members' order is the
+//                  id order (the reference's).
 //                  Velocities are updated in place in the input buffer.
 //   sample_cells   On sampled steps only (the reference's cadence,
 //                  dsmc/statisticssampler.cpp:45-66): every cell's fp64
@@ -132,8 +131,8 @@ struct CollideSmem {
     uint32_t ids[PCAP];  // batch members: ids and slots, cell by cell
     int slot[PCAP];
     int perm[PCAP];      // batch members by id rank within each cell (warp-ranked cells)
-    int apos[32 * (NTMAX + 1)];   // lane i: its cell's arrivals in id order: merged rank
-    int aslot[32 * (NTMAX + 1)];  //   and slot (rows of NTMAX + 1: no bank conflicts)
+    uint32_t aid[32 * (NTMAX + 1)];  // lane i: its cell's arrivals in id order: id
+    int aslot[32 * (NTMAX + 1)];     //   and slot (rows of NTMAX + 1: no bank conflicts)
 };
 
 // Velocities of one cell's members in the input buffer, by id rank.
@@ -154,7 +153,10 @@ struct RankVel {
     }
 };
 struct IdentityPerm {
-    __device__ __forceinline__ int operator[](int i) const { return i; }
+    __device__ __forceinline__ void pick(int r0, int r1, int &s0, int &s1) const {
+        s0 = r0;
+        s1 = r1;
+    }
 };
 // Velocities of a cell's members by slot.
 struct SlotVel {
@@ -172,20 +174,46 @@ struct SlotVel {
         q[2] = z;
     }
 };
-// Slot of the member of id rank r in a cell whose bottom segment is sorted:
-// an arrival if one has merged rank r, else the bottom member r minus the
-// arrivals below.
+// Slots of the members of two id ranks in a cell whose bottom segment is
+// sorted.  With the bottom ids b[k] (nothing below 0, everything at nb and
+// above) and the arrivals' ids t[j] in order, arrival j has rank p_j =
+// #{b < t[j]} + j, so p_j < r exactly if b[r - j - 1] > t[j], and p_j <= r if
+// b[r - j] > t[j]: rank r is settled by the nt + 1 bottom members up to
+// position r, without the other members' ids.
 struct PickPerm {
-    const int *apos, *aslot;
-    int nt, base;
-    __device__ __forceinline__ int operator[](int r) const {
-        int below = 0;
-        for (int j = 0; j < nt; ++j) {
-            const int p = apos[j];
-            if (p == r) return aslot[j];
-            below += p < r;
+    const float4 *B;
+    const uint32_t *aid;
+    const int *aslot;
+    int nt, nb, base;
+    __device__ __forceinline__ uint32_t bottom(int k) const {
+        return k < 0 ? 0u : k >= nb ? 0xffffffffu : __float_as_uint(B[rec_at(base + k)].w);
+    }
+    __device__ __forceinline__ int resolve(int r, uint32_t b0, uint32_t b1, uint32_t b2) const {
+        uint32_t at = b0, below = b1;  // b[r - j], b[r - j - 1]
+        int j = 0;
+        for (; j < nt; ++j) {
+            const uint32_t t = aid[j];
+            if (!(below > t)) return at > t ? aslot[j] : base + (r - j);
+            at = below;
+            below = j == 0 ? b2 : bottom(r - j - 2);
         }
-        return base + (r - below);
+        return base + (r - j);
+    }
+    __device__ __forceinline__ void pick(int r0, int r1, int &s0, int &s1) const {
+        // both ranks' first three bottom ids in flight together (two arrivals)
+        uint32_t x0 = 0, x1 = 0, x2 = 0, y0 = 0, y1 = 0, y2 = 0;
+        if (nt > 0) {
+            x0 = bottom(r0);
+            x1 = bottom(r0 - 1);
+            y0 = bottom(r1);
+            y1 = bottom(r1 - 1);
+        }
+        if (nt > 1) {
+            x2 = bottom(r0 - 2);
+            y2 = bottom(r1 - 2);
+        }
+        s0 = resolve(r0, x0, x1, x2);
+        s1 = resolve(r1, y0, y1, y2);
     }
 };
 
@@ -205,11 +233,16 @@ __device__ __forceinline__ void publish_collide(const PassParams &P, int sys, un
     }
 }
 
+// Bound by the latency of a lane's chain: header, arrivals' ids, the picks'
+// bottom ids and velocities per candidate.  us per step, with every member's id
+// of a colliding cell loaded and ranked, and so: 64^3 18.0 -> 17.1, 128^3 58 ->
+// 35, 256^3 267 -> 153.  Five blocks per SM (96 registers): six spill (80
+// registers; 172 us at 256^3), four have too few warps (179 us).
 // CLAIM: chunks beyond each warp's first come from the counter (chosen by
 // the launcher when there are many chunks per warp; a fixed stride measured
 // faster with few: packed_64 and packed_128).
 template <bool CLAIM>
-__global__ void __launch_bounds__(32 * C_WARPS) collide_cells_kernel(const __grid_constant__ PassParams P) {
+__global__ void __launch_bounds__(32 * C_WARPS, 5) collide_cells_kernel(const __grid_constant__ PassParams P) {
     __shared__ CollideSmem smem[C_WARPS];
     const int lane = threadIdx.x & 31;
     const volatile Status *vs = P.status;
@@ -261,9 +294,45 @@ __global__ void __launch_bounds__(32 * C_WARPS) collide_cells_kernel(const __gri
             tsys = csys;
         }
 
-        // Rank the colliding cells' members by id, a batch at a time, and
-        // run the batch's candidate loops one cell per lane.
-        unsigned todo = __ballot_sync(0xffffffffu, pairs > 0);
+        // Cells with a sorted bottom and few arrivals, as nearly all: each lane
+        // sorts its cell's arrivals by id and runs its candidate loop.
+        const bool lp = pairs > 0 && P.sorted_in && (int)nt <= NTMAX;
+        if (lp) {
+            uint32_t *aid = W.aid + lane * (NTMAX + 1);
+            int *as = W.aslot + lane * (NTMAX + 1);
+            const int t0 = m.x + m.y - (int)nt;
+            for (int j = 0; j < (int)nt; ++j) aid[j] = __float_as_uint(Bin[rec_at(t0 + j)].w);
+            for (int j = 0; j < (int)nt; ++j) {
+                const uint32_t id = aid[j];
+                int i = j - 1;
+                while (i >= 0 && aid[i] > id) {
+                    aid[i + 1] = aid[i];
+                    as[i + 1] = as[i];
+                    --i;
+                }
+                aid[i + 1] = id;
+                as[i + 1] = t0 + j;
+            }
+            DrawStream rs;
+            rs.init(P.sys[sys].seed, (uint32_t)m.z, step, DSMC_TAG_COLLIDE);
+            unsigned long long c_ = 0;
+            SlotVel vel;
+            vel.b = Bin;
+            PickPerm pick;
+            pick.B = Bin;
+            pick.aid = aid;
+            pick.aslot = as;
+            pick.nt = (int)nt;
+            pick.nb = (int)nb;
+            pick.base = m.x;
+            ntc_loop<float>(rs, n, pairs, vr, vel, pick, c_);
+            col += (unsigned)c_;
+            cand += (unsigned)pairs;
+        }
+        // The others (unsorted bottoms after a repack or the stage kernels,
+        // many arrivals): rank their members by id, a batch at a time, and run
+        // the batch's candidate loops one cell per lane.
+        unsigned todo = __ballot_sync(0xffffffffu, pairs > 0 && !lp);
         while (todo) {
             // the batch: colliding cells, in order, whose members fit PCAP
             unsigned ready = 0;
@@ -318,41 +387,8 @@ __global__ void __launch_bounds__(32 * C_WARPS) collide_cells_kernel(const __gri
                     if (f0 + 32 * u < total) W.ids[f0 + 32 * u] = v[u];
             }
             __syncwarp();
-            // Cells with a sorted bottom and few arrivals: each lane sorts its
-            // cell's arrivals and finds their merged ranks by binary search.
-            const bool lp = rb && P.sorted_in && (int)nt <= NTMAX;
-            if (lp) {
-                uint32_t *ids = W.ids + start;
-                int *sl = W.slot + start;
-                const int b = (int)nb;
-                for (int j = b + 1; j < n; ++j) {
-                    const uint32_t id = ids[j];
-                    const int s = sl[j];
-                    int i = j - 1;
-                    while (i >= b && ids[i] > id) {
-                        ids[i + 1] = ids[i];
-                        sl[i + 1] = sl[i];
-                        --i;
-                    }
-                    ids[i + 1] = id;
-                    sl[i + 1] = s;
-                }
-                int *ap = W.apos + lane * (NTMAX + 1), *as = W.aslot + lane * (NTMAX + 1);
-                for (int j = 0; j < (int)nt; ++j) {
-                    const uint32_t id = ids[b + j];
-                    int lo = 0, hi = b;
-                    while (lo < hi) {
-                        const int mid = (lo + hi) >> 1;
-                        if (ids[mid] < id) lo = mid + 1;
-                        else hi = mid;
-                    }
-                    ap[j] = lo + j;
-                    as[j] = sl[b + j];
-                }
-            }
-            // The other cells: id ranks by the warp, cell by cell.
-            const unsigned wr = ready & ~__ballot_sync(0xffffffffu, lp);
-            for (unsigned t2 = wr; t2; t2 &= t2 - 1u) {
+            // id ranks by the warp, cell by cell
+            for (unsigned t2 = ready; t2; t2 &= t2 - 1u) {
                 const int c = __ffs(t2) - 1;
                 const int off = __shfl_sync(0xffffffffu, start, c);
                 const int nc = __shfl_sync(0xffffffffu, n, c);
@@ -414,21 +450,10 @@ __global__ void __launch_bounds__(32 * C_WARPS) collide_cells_kernel(const __gri
                 DrawStream rs;
                 rs.init(g.seed, (uint32_t)m.z, step, DSMC_TAG_COLLIDE);
                 unsigned long long c_ = 0;
-                if (lp) {
-                    SlotVel vel;
-                    vel.b = Bin;
-                    PickPerm pick;
-                    pick.apos = W.apos + lane * (NTMAX + 1);
-                    pick.aslot = W.aslot + lane * (NTMAX + 1);
-                    pick.nt = (int)nt;
-                    pick.base = m.x;
-                    ntc_loop<float>(rs, n, pairs, vr, vel, pick, c_);
-                } else {
-                    RankVel vel;
-                    vel.b = Bin;
-                    vel.perm = W.perm + start;
-                    ntc_loop<float>(rs, n, pairs, vr, vel, IdentityPerm(), c_);
-                }
+                RankVel vel;
+                vel.b = Bin;
+                vel.perm = W.perm + start;
+                ntc_loop<float>(rs, n, pairs, vr, vel, IdentityPerm(), c_);
                 col += (unsigned)c_;
                 cand += (unsigned)pairs;
             }
