@@ -354,8 +354,10 @@ struct Split32 {
     struct WallFrame {
         float n[3], a[3], b[3];
         __device__ __forceinline__ void compose(float vn, float vt1, float vt2, float v[3]) const {
+            // rounding spelled out: a caller's -vn folded into the sum would
+            // change which product is rounded
 #pragma unroll
-            for (int d = 0; d < 3; ++d) v[d] = vn * n[d] + vt1 * a[d] + vt2 * b[d];
+            for (int d = 0; d < 3; ++d) v[d] = fmaf(vt2, b[d], fmaf(vn, n[d], __fmul_rn(vt1, a[d])));
         }
     };
     static __device__ __forceinline__ WallFrame load_frame(const SysDev &g, uint32_t vlin) {
