@@ -405,7 +405,7 @@ int dsmc_ctx_set_capacity(dsmc_ctx *ctx, double factor, int pad);
  * Launch shape of the timestep pass: pipelined = 1 when the split-precision
  * production pass (collide_cells, move_cells, place_movers, place_walls) runs
  * dsmc_step (0: the generic cell pass, e.g. fp64 contexts), the grid and
- * block of move_cells, and its per-warp staging ring in particles. */
+ * block of move_cells, and the particles of a group that its warps stage. */
 int dsmc_pass_info(dsmc_ctx *ctx, int *pipelined, int *grid, int *block, int *stage_capacity);
 
 /* Launch tuning of the production pass, for the autotuner
@@ -414,8 +414,8 @@ int dsmc_pass_info(dsmc_ctx *ctx, int *pipelined, int *grid, int *block, int *st
  * collide_cells, move_cells, place_movers, place_walls and sample_cells, each
  * a persistent grid (0: the most that are resident, the default; larger
  * values are clamped to it); ring: move_cells' shared-memory staging ring in
- * particles per warp (0: the smallest that holds the largest cell; larger
- * rings trade resident blocks for staging depth); collide_claim: how
+ * particles per warp and staged group of cells (0: 128, or the smallest that
+ * holds the largest cell; larger ones trade resident blocks for staging depth); collide_claim: how
  * collide_cells' warps take chunks of 32 cells after their first (0: a
  * pass-wide counter when each warp has four chunks or more, else a fixed
  * stride; 1: always the stride; 2: always the counter).  Any setting gives

@@ -58,10 +58,11 @@ template <class K> static int static_blocks(K kernel, int threads) {
     return nb;
 }
 
-// Ring slots per warp of move_cells for cells of at most `smem_cap` slots
+// Records of the groups that move_cells' warps stage, for cells of at most
+// `smem_cap` slots (128 at least)
 // (0: no ring is large enough, or a cell could exceed the collide batch).
 int fused_capacity(int smem_cap) {
-    static const int rings[] = {64, 96, 128, 160, 192, 224, 256, 320, 384, 448, 512};
+    static const int rings[] = {128, 160, 192, 224, 256, 320, 384, 448, 512};
     if (smem_cap > pass3::PCAP) return 0;
     for (int r : rings)
         if (smem_cap <= r) return r;
@@ -69,7 +70,7 @@ int fused_capacity(int smem_cap) {
 }
 
 int ring_for(int smem_cap, int ring) {
-    static const int rings[] = {64, 96, 128, 160, 192, 224, 256, 320, 384, 448, 512};
+    static const int rings[] = {128, 160, 192, 224, 256, 320, 384, 448, 512};
     const int need = fused_capacity(smem_cap);
     if (need <= 0) return 0;
     const int want = std::max(need, ring);
@@ -82,7 +83,7 @@ int max_ring() { return 512; }
 
 int fused_block() { return 32 * pass3::M_WARPS; }
 
-#define DSMC_MOVE_RINGS(X) X(64) X(96) X(128) X(160) X(192) X(224) X(256) X(320) X(384) X(448) X(512)
+#define DSMC_MOVE_RINGS(X) X(128) X(160) X(192) X(224) X(256) X(320) X(384) X(448) X(512)
 
 int fused_grids(int smem_cap, int num_sms, int grids[5], int ring, int max_bps[5]) {
     int bm = 0;

@@ -20,7 +20,8 @@
 //                  not moved, go to the gap just above: slots
 //                  [base + stayers, base + n_in) hold exactly the cell's
 //                  movers.  Particle records stream through a per-warp
-//                  shared-memory ring with 16-byte cp.async copies.
+//                  shared-memory ring with bulk copies, a group of cells
+//                  ahead of the one in work.
 //   place_movers   A mover whose flight ends in an empty voxel completes it
 //                  and takes a top slot of its new cell (warp-aggregated
 //                  atomics; the spill list when the cell is full).  Flights
@@ -48,22 +49,39 @@ namespace pass3 {
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// 16-byte global -> shared copy, cached in L2 only (both addresses 16-byte
-// aligned: slots are uint4/float4 records).
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+// Bulk copies global -> shared of this block (addresses and size multiples of
+// 16 bytes), completing on an mbarrier.
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// Waits until at most `pending` of this thread's newest commit groups are
-// still in flight (more than 4 is treated as 4, which waits longer).
-__device__ __forceinline__ void cp_async_wait(int pending) {
-    switch (pending) {
-        case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-        case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-        case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-        case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-        default: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_fence_init() {
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Waits for the phase of the given parity; false when the (far too long)
+// limit ran out.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
+    for (unsigned i = 0; i < (1u << 22); ++i) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (done) return true;
     }
+    return false;
 }
 
 // A particle record {A, B} of slot s in one 32-byte access.  (With A and B in
@@ -626,7 +644,6 @@ __global__ void __launch_bounds__(32 * C_WARPS) sample_cells_kernel(const __grid
 // ---- move_cells -------------------------------------------------------------
 
 constexpr int M_WARPS = 4;
-constexpr int DEPTH = 4;  // cells staged ahead of the one in work
 
 struct MoveTab {
     int4 t[32];  // {first slot, slots, bottom | top << 16 occupancy, system}: one load per cell
@@ -634,44 +651,26 @@ struct MoveTab {
     __device__ __forceinline__ static int nb(const int4 &c) { return c.z & 0xffff; }
     __device__ __forceinline__ static int nt(const int4 &c) { return (int)((unsigned)c.z >> 16); }
 };
-// The staging ring: records of 32 bytes, the halves of every other group of
-// four swapped so that eight lanes' 16-byte reads of one half of consecutive
-// records fall into different banks.
 template <int R> struct MoveSmem {
-    uint4 rec[2 * R];
-    __device__ __forceinline__ static int at(int r, int half) { return 2 * r + (half ^ ((r >> 2) & 1)); }
-    __device__ __forceinline__ uint4 a(int r) const { return rec[at(r, 0)]; }
-    __device__ __forceinline__ float4 b(int r) const { return *reinterpret_cast<const float4 *>(&rec[at(r, 1)]); }
-    __device__ __forceinline__ uint32_t id(int r) const { return rec[at(r, 1)].w; }
+    static constexpr int H = R < 256 ? R : 256;  // records of a staged group
+    static constexpr int T = 2 * H;              // two groups
+    uint4 rec[2 * T];  // records of 32 bytes
+    __device__ __forceinline__ uint4 a(int r) const { return rec[2 * r]; }
+    __device__ __forceinline__ float4 b(int r) const { return *reinterpret_cast<const float4 *>(&rec[2 * r + 1]); }
+    __device__ __forceinline__ uint32_t id(int r) const { return rec[2 * r + 1].w; }
     __device__ __forceinline__ void set(int r, const uint4 &ra, const float4 &rb) {
-        rec[at(r, 0)] = ra;
-        *reinterpret_cast<float4 *>(&rec[at(r, 1)]) = rb;
+        rec[2 * r] = ra;
+        *reinterpret_cast<float4 *>(&rec[2 * r + 1]) = rb;
     }
+    uint64_t bar[2];   // a half's copies
     MoveTab tab[2];
     uint16_t pref[R + 2];  // two-pass placement: stayers before each member
 };
 
-// accelerate, then the first flight when it stays inside the particle's
-// empty voxel (the reference's outcome: r += v dt lands in an empty voxel,
+// accelerate, then the first flight when it stays inside the particle's empty
+// voxel (the reference's outcome: r += v dt lands in an empty voxel,
 // dsmc/moleculemover.cpp:74-77); false leaves the particle accelerated.
-__device__ __forceinline__ bool first_flight(const SysDev &g, Split32::Particle &p) {
-    Split32::accelerate(g, p);
-    if (p.flag) return false;
-    float x[3];
-    bool stay = true;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        x[d] = fmaf(p.v[d] * g.inv_vox_f[d], g.dt_f, p.o[d]);
-        stay &= (x[d] >= 0.0f) & (x[d] < 1.0f);
-    }
-    if (stay) {
-        p.o[0] = x[0];
-        p.o[1] = x[1];
-        p.o[2] = x[2];
-    }
-    return stay;
-}
-
+//
 // A system's constants of the first flight, held in registers.
 struct FlightConst {
     float inv_vox[3], dt, accel[3];  // accel: the flow axis's accel_dt_f, 0 on the others
@@ -709,30 +708,20 @@ __device__ __forceinline__ bool first_flight_raw(const FlightConst &k, uint4 &a,
 }
 
 // One cell of at most 32 * NR members whose bottom segment is sorted by id,
-// held in registers (member q = 32 k + lane in p[k]): flight of every member,
-// then stayers to the bottom segment in id order and movers to the gap.
-// Returns the number of stayers.  All lanes call.
-template <int R, int NR>
-__device__ __forceinline__ unsigned place_sorted(const FlightConst &fc, const MoveSmem<R> &W, int tail, int base,
-                                                 int n, int nb, void *out, int lane) {
+// held in registers (member q = 32 k + lane in ra[k], rb[k]): flight of every
+// member, then stayers to the bottom segment in id order and movers to the
+// gap.  Returns the number of stayers.  All lanes call.
+template <int NR>
+__device__ __forceinline__ unsigned place_sorted(const FlightConst &fc, uint4 (&ra)[NR], float4 (&rb)[NR], int base, int n,
+                                                 int nb, void *out, int lane) {
     const unsigned below = (1u << lane) - 1u;
-    uint4 ra[NR];
-    float4 rb[NR];
     bool stay[NR];
     uint32_t id[NR];
     unsigned fast[NR], slow[NR], bm[NR], add[NR], pb[NR];
 #pragma unroll
     for (int k = 0; k < NR; ++k) {
-        const int q = 32 * k + lane;
-        const bool valid = q < n;
-        stay[k] = false;
-        if (valid) {
-            int r = tail + q;
-            if (r >= R) r -= R;
-            ra[k] = W.a(r);
-            rb[k] = W.b(r);
-            stay[k] = first_flight_raw(fc, ra[k], rb[k]);
-        }
+        const bool valid = 32 * k + lane < n;
+        stay[k] = first_flight_raw(fc, ra[k], rb[k]);
         id[k] = valid ? __float_as_uint(rb[k].w) : 0xffffffffu;
         fast[k] = __ballot_sync(0xffffffffu, valid && stay[k]);
         slow[k] = __ballot_sync(0xffffffffu, valid && !stay[k]);
@@ -743,22 +732,27 @@ __device__ __forceinline__ unsigned place_sorted(const FlightConst &fc, const Mo
     // each arrival i: staying arrivals below every member, bottom stayers
     // below the arrival
     for (int i = nb; i < n; ++i) {
-        const int li = i & 31;
-        const bool hi = NR > 1 && i >= 32;
-        const uint32_t t = __shfl_sync(0xffffffffu, hi ? id[NR - 1] : id[0], li);
-        const unsigned ts = ((hi ? fast[NR - 1] : fast[0]) >> li) & 1u;
+        const int li = i & 31, ki = i >> 5;
+        uint32_t src = id[0];
+        unsigned fk = fast[0];
+#pragma unroll
+        for (int k = 1; k < NR; ++k) {
+            src = ki == k ? id[k] : src;
+            fk = ki == k ? fast[k] : fk;
+        }
+        const uint32_t t = __shfl_sync(0xffffffffu, src, li);
+        const unsigned ts = (fk >> li) & 1u;
         unsigned bl = 0;
 #pragma unroll
         for (int k = 0; k < NR; ++k) {
             add[k] += ts && t < id[k];
             bl += (unsigned)__popc(fast[k] & bm[k] & __ballot_sync(0xffffffffu, id[k] < t));
         }
-        if (lane == li) {
-            if (hi) pb[NR - 1] = bl;
-            else pb[0] = bl;
-        }
+#pragma unroll
+        for (int k = 0; k < NR; ++k)
+            if (lane == li && ki == k) pb[k] = bl;
     }
-    unsigned fs_before = 0, mv_before = 0;  // bottom stayers and movers of the earlier chunks
+    unsigned fs_before = 0, mv_before = 0, nfs = 0;  // bottom stayers and movers of the earlier chunks; stayers
 #pragma unroll
     for (int k = 0; k < NR; ++k) {
         const int q = 32 * k + lane;
@@ -770,41 +764,25 @@ __device__ __forceinline__ unsigned place_sorted(const FlightConst &fc, const Mo
         }
         fs_before += (unsigned)__popc(fast[k] & bm[k]);
         mv_before += (unsigned)__popc(slow[k]);
+        nfs += (unsigned)__popc(fast[k]);
     }
-    unsigned nfs = 0;
-#pragma unroll
-    for (int k = 0; k < NR; ++k) nfs += (unsigned)__popc(fast[k]);
     return nfs;
 }
 
-// Two consecutive cells of at most 32 members each with sorted bottom
-// segments and one system: place_sorted<R, 1> for both, written as one
-// straight-line body so that the two cells' dependency chains interleave.
-// nfs[k]: stayers of cell k.  All lanes call.
-template <int R>
-__device__ __forceinline__ void place_pair(const FlightConst &fc, const MoveSmem<R> &W, int tail, const int base[2],
-                                          const int n[2], const int nb[2], void *out, int lane,
-                                          unsigned nfs[2]) {
+// Two cells of at most 32 members each with sorted bottom segments and one
+// system: place_sorted<1> for both, written as one straight-line body so that
+// the two cells' dependency chains interleave.  nfs[k]: stayers of cell k.
+// All lanes call.
+__device__ __forceinline__ void place_pair(const FlightConst &fc, uint4 (&ra)[2], float4 (&rb)[2], const int base[2],
+                                          const int n[2], const int nb[2], void *out, int lane, unsigned nfs[2]) {
     const unsigned below = (1u << lane) - 1u;
-    uint4 ra[2];
-    float4 rb[2];
     bool stay[2];
     uint32_t id[2];
     unsigned fast[2], slow[2], bm[2], add[2], pb[2];
-    int t1 = tail + n[0];
-    if (t1 >= R) t1 -= R;
-    const int tl[2] = {tail, t1};
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const bool valid = lane < n[k];
-        stay[k] = false;
-        if (valid) {
-            int r = tl[k] + lane;
-            if (r >= R) r -= R;
-            ra[k] = W.a(r);
-            rb[k] = W.b(r);
-            stay[k] = first_flight_raw(fc, ra[k], rb[k]);
-        }
+        stay[k] = first_flight_raw(fc, ra[k], rb[k]);
         id[k] = valid ? __float_as_uint(rb[k].w) : 0xffffffffu;
         fast[k] = __ballot_sync(0xffffffffu, valid && stay[k]);
         slow[k] = __ballot_sync(0xffffffffu, valid && !stay[k]);
@@ -839,16 +817,102 @@ __device__ __forceinline__ void place_pair(const FlightConst &fc, const MoveSmem
     }
 }
 
-// 64 B per particle; at 256^3 (3.15e7 particles) 566 us with A and B apart and
-// five table words per cell, 549 us (3.7 TB/s) so.  Bound by its instructions
-// (about 400 per pair of cells, 0.5 issued per cycle and scheduler).
-// At most 128 registers (four blocks per SM): the compiler then keeps both
-// cells of a pair in flight; left to itself it may pick 96 and five blocks,
-// which measured slower.
+// A cell whose n records are staged at record r0: any size, any order of the
+// bottom segment, in two passes.  Returns the number of stayers.  All lanes
+// call.
+template <int R>
+__device__ __noinline__ unsigned place_staged(int sorted_in, FlightConst fc, MoveSmem<R> &W, int r0, int base, int n, int nb,
+                                              void *out, int lane) {
+    auto rid = [&](int q) { return W.id(r0 + q); };
+    bool viol = false;
+    if (!sorted_in)
+        for (int q = lane; q + 1 < nb; q += 32) viol |= !(rid(q) < rid(q + 1));
+    const bool sorted = !__any_sync(0xffffffffu, viol);
+    if (sorted && n <= 128) {
+        uint4 ra[4];
+        float4 rb[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int r = r0 + max(min(32 * k + lane, n - 1), 0);
+            ra[k] = W.a(r);
+            rb[k] = W.b(r);
+        }
+        return place_sorted<4>(fc, ra, rb, base, n, nb, out, lane);
+    }
+    const unsigned below = (1u << lane) - 1u;
+    // pass 1: every member's flight; the record goes back and pref[q] counts
+    // the stayers before member q
+    unsigned S = 0;
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        const int q = c0 + lane;
+        const bool valid = q < n;
+        bool stay = false;
+        if (valid) {
+            uint4 ra = W.a(r0 + q);
+            float4 rb = W.b(r0 + q);
+            stay = first_flight_raw(fc, ra, rb);
+            W.set(r0 + q, ra, rb);
+        }
+        const unsigned fast = __ballot_sync(0xffffffffu, valid && stay);
+        if (valid) W.pref[q] = (uint16_t)(S + (unsigned)__popc(fast & below));
+        S += (unsigned)__popc(fast);
+    }
+    if (lane == 0) W.pref[n] = (uint16_t)S;
+    __syncwarp();
+    // pass 2: stayers in id order, movers below the top of the gap
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        const int q = c0 + lane;
+        if (q < n) {
+            const uint32_t id = rid(q);
+            unsigned dst;
+            if (W.pref[q + 1] > W.pref[q]) {
+                unsigned pos;
+                if (sorted) {
+                    int lb = q;  // bottom members below this id
+                    if (q >= nb) {
+                        int lo = 0, hi = nb;
+                        while (lo < hi) {
+                            const int mid = (lo + hi) >> 1;
+                            if (rid(mid) < id) lo = mid + 1;
+                            else hi = mid;
+                        }
+                        lb = lo;
+                    }
+                    pos = W.pref[lb];
+                    for (int i = nb; i < n; ++i) pos += (W.pref[i + 1] > W.pref[i]) && rid(i) < id;
+                } else {
+                    pos = 0;
+                    for (int i = 0; i < n; ++i) pos += (W.pref[i + 1] > W.pref[i]) && rid(i) < id;
+                }
+                dst = (unsigned)base + pos;
+            } else {
+                dst = (unsigned)(base + n) - 1u - ((unsigned)q - W.pref[q]);
+            }
+            store_record(out, dst, W.a(r0 + q), W.b(r0 + q));
+        }
+    }
+    return S;
+}
+
+// Cells staged together: cells [ci, ci + cnt) of their chunk, at most H
+// records, or one cell larger than that (`big`: staged when its turn comes).
+struct MoveGroup {
+    int ci, cnt;  // cnt 0: none left
+    bool big, last;  // last: of its chunk
+};
+
+// Each lane stages its own cell: a bulk copy of the bottom segment and one of
+// the top, tracked by an mbarrier per half of the staging memory; a group is in
+// flight while the one before is worked on.  With 16-byte copies per lane, cell by
+// cell, the staging took a quarter of the instructions.  us per step at 64^3 /
+// 128^3 / 256^3: so staged 16.9 / 83 / 549; in groups of up to 80 records 16.4 /
+// 72 / 470, of 128 15.0 / 65 / 418 (4.8 TB/s, 0.75 of the copy rate), of 160
+// 14.6 / 63 / 430, of 192 14.6 / 62 / 448.  Loaded straight into registers a pair of cells
+// ahead, with fewer instructions still, 14.5 / 84 / 590: too few bytes in flight.
 template <int R>
 __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __grid_constant__ PassParams P) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    typedef Split32::Particle Particle;
+    constexpr int H = MoveSmem<R>::H, T2 = MoveSmem<R>::T;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const volatile Status *vs = P.status;
@@ -871,16 +935,21 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
             T.first = first;
             T.ncell = ncell;
         }
+        int4 row = make_int4(0, 0, 0, 0);
         if (lane < ncell) {
             const int a = first + lane;
             const int4 m = P.cells.meta[a];
             unsigned nb, nt;
             input_counts(P, a, m, nb, nt);
-            if (nb + nt > (unsigned)R) atomicOr(&P.status->error, DSMC_EBIT_SMEM);  // the host sizes R above every cap
+            if (nb + nt > (unsigned)R) {  // the host sizes R above every cap
+                atomicOr(&P.status->error, DSMC_EBIT_SMEM);
+                nb = nt = 0;
+            }
             // top slots free for arrivals this pass: above the input occupancy
             P.cells.room[a] = make_int2(m.x + m.y, m.y - (int)(nb + nt));
-            T.t[lane] = make_int4(m.x, m.y, (int)(nb | nt << 16), m.w);  // (cells hold at most R <= 512)
+            row = make_int4(m.x, m.y, (int)(nb | nt << 16), m.w);  // (cells hold at most R <= 512)
         }
+        T.t[lane] = row;
     };
     // Lane i publishes cell i's bottom occupancy and clears the set the next
     // pass writes.
@@ -894,183 +963,154 @@ __global__ void __launch_bounds__(32 * M_WARPS, 4) move_cells_kernel(const __gri
         }
     };
 
+    if (lane == 0) {
+        mbar_init(&W.bar[0], 1);
+        mbar_init(&W.bar[1], 1);
+        mbar_fence_init();
+    }
     load_tab(0, chunk0);
     load_tab(1, chunk0 + wstride);
     __syncwarp();
 
-    int head = 0, tail = 0, used = 0;  // ring (warp-uniform)
-    int it = 0, ii = 0;                // next cell to stage: chunk ordinal, cell in chunk
-    int ct = 0, ci = 0;                // cell in work
-    int ahead = 0;                     // cells staged, the one in work included
-    unsigned nfs_mine = 0;             // lane i: bottom occupancy of cell i of the chunk in work
-    unsigned moved = 0;                // particles moved, system tsys (warp-uniform)
-    int tsys = -1;
-    FlightConst fc = {};               // constants of system tsys
-
-    auto stage_ahead = [&]() {
-        // (it, ii) moves past a full chunk as soon as its last cell is
-        // staged, so ii >= ncell only past the warp's last cell
-        while (ahead <= DEPTH && it <= ct + 1) {
-            const MoveTab &T = W.tab[it & 1];
-            if (ii >= T.ncell) return;
-            const int4 c = T.t[ii];
-            const int nb = MoveTab::nb(c), nt = MoveTab::nt(c);
-            const int n = min(nb + nt, R);
-            if (used + n > R) return;
-            const int base = c.x, cap = c.y;
-            for (int h = lane; h < 2 * n; h += 32) {  // half h & 1 of member h >> 1
-                const int q = h >> 1;
-                int r = head + q;
-                if (r >= R) r -= R;
-                cp_async16(&W.rec[MoveSmem<R>::at(r, h & 1)], in + rec_at(member_slot(base, cap, nb, nt, q)) + (h & 1));
+    int gt = 0, gi = 0;     // the next group: chunk ordinal, first cell
+    uint32_t parity = 0;    // bit h: phase of half h's barrier
+    bool ok = true;
+    // The next group; its copies start, into half h, unless it is big.
+    auto next_group = [&](MoveGroup &g, int h) {
+        const MoveTab &T = W.tab[gt & 1];
+        const int nc = T.ncell;
+        g.cnt = 0;
+        if (gi >= nc) return;  // past the warp's last cell
+        const int4 c = T.t[lane];  // (rows past the chunk's cells are empty)
+        const int nb = MoveTab::nb(c), nt = MoveTab::nt(c), n = lane >= gi ? nb + nt : 0;
+        int incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const bool fits = lane >= gi && lane < nc && incl <= H;
+        g.ci = gi;
+        g.cnt = __popc(__ballot_sync(0xffffffffu, fits));
+        g.big = g.cnt == 0;
+        if (g.big) {
+            g.cnt = 1;
+        } else {
+            const int total = __shfl_sync(0xffffffffu, incl, gi + g.cnt - 1);
+            if (lane == 0) mbar_expect(&W.bar[h], 32u * (unsigned)total);
+            __syncwarp();
+            if (fits) {
+                uint4 *dst = &W.rec[2 * (h * H + incl - n)];
+                if (nb) bulk_load(dst, in + rec_at(c.x), 32u * (unsigned)nb, &W.bar[h]);
+                if (nt) bulk_load(dst + 2 * nb, in + rec_at(c.x + c.y - nt), 32u * (unsigned)nt, &W.bar[h]);
             }
-            cp_async_commit();
-            head += n;
-            if (head >= R) head -= R;
-            used += n;
-            ++ahead;
-            if (++ii == CH) {
-                ++it;
-                ii = 0;
-            }
+        }
+        gi += g.cnt;
+        g.last = gi == nc;
+        if (gi == CH) {
+            ++gt;
+            gi = 0;
         }
     };
 
-    while (true) {
+    int ct = 0;             // chunk in work
+    unsigned nfs_mine = 0;  // lane i: bottom occupancy of cell i of the chunk in work
+    unsigned moved = 0;     // particles moved, system tsys (warp-uniform)
+    int tsys = -1;
+    FlightConst fc = {};    // constants of system tsys
+    MoveGroup cur, nxt;
+    int half = 0;
+    next_group(cur, 0);
+    while (cur.cnt) {
         const MoveTab &T = W.tab[ct & 1];
-        if (ci >= T.ncell) {
-            if (T.ncell > 0) write_tab(ct & 1, nfs_mine);
-            if (T.ncell < CH) break;  // that was the warp's last chunk
+        int r = half * H;   // record of the cell in work
+        if (cur.big) {
+            // (nothing else is staged: the whole ring is free)
+            const int4 c = T.t[cur.ci];
+            const int nb = MoveTab::nb(c), nt = MoveTab::nt(c);
+            if (lane == 0) {
+                mbar_expect(&W.bar[half], 32u * (unsigned)(nb + nt));
+                if (nb) bulk_load(W.rec, in + rec_at(c.x), 32u * (unsigned)nb, &W.bar[half]);
+                if (nt) bulk_load(W.rec + 2 * nb, in + rec_at(c.x + c.y - nt), 32u * (unsigned)nt, &W.bar[half]);
+            }
+            __syncwarp();
+            r = 0;
+        } else {
+            next_group(nxt, half ^ 1);
+        }
+        ok &= mbar_wait(&W.bar[half], (parity >> half) & 1u);
+        parity ^= 1u << half;
+        const int end = cur.ci + cur.cnt;
+        for (int i = cur.ci; i < end;) {
+            const int4 c0 = T.t[i], c1 = T.t[min(i + 1, 31)];
+            if (c0.w != tsys) {
+                if (lane == 0 && tsys >= 0 && moved) atomicAdd(&P.tally[tsys].particle_steps, (unsigned long long)moved);
+                moved = 0;
+                tsys = c0.w;
+                fc = flight_const(P.sys[tsys]);
+            }
+            const int nb[2] = {MoveTab::nb(c0), MoveTab::nb(c1)};
+            int n[2] = {nb[0] + MoveTab::nt(c0), nb[1] + MoveTab::nt(c1)};
+            if (P.sorted_in && n[0] <= 32) {
+                // two small cells of one system go together
+                const bool two = i + 1 < end && n[1] <= 32 && c1.w == c0.w;
+                n[1] = two ? n[1] : 0;
+                const int base[2] = {c0.x, c1.x};
+                const int q[2] = {r + lane, r + n[0] + lane};
+                uint4 ra[2];
+                float4 rb[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const int at = min(q[k], T2 - 1);  // (lanes past the members read some record)
+                    ra[k] = W.a(at);
+                    rb[k] = W.b(at);
+                }
+                unsigned nfs[2];
+                place_pair(fc, ra, rb, base, n, nb, out, lane, nfs);
+                if (lane == i) nfs_mine = nfs[0];
+                if (two && lane == i + 1) nfs_mine = nfs[1];
+                r += n[0] + n[1];
+                moved += (unsigned)(n[0] + n[1]);
+                i += two ? 2 : 1;
+                continue;
+            }
+            unsigned nfs;
+            if (P.sorted_in && n[0] <= 64) {
+                uint4 ra[2];
+                float4 rb[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const int at = min(r + 32 * k + lane, T2 - 1);
+                    ra[k] = W.a(at);
+                    rb[k] = W.b(at);
+                }
+                nfs = place_sorted<2>(fc, ra, rb, c0.x, n[0], nb[0], out, lane);
+            } else {
+                nfs = place_staged<R>(P.sorted_in, fc, W, r, c0.x, n[0], nb[0], out, lane);
+                proxy_fence();  // its writes to the ring, before the next copies there
+            }
+            if (lane == i) nfs_mine = nfs;
+            r += n[0];
+            moved += (unsigned)n[0];
+            ++i;
+        }
+        __syncwarp();  // every lane is done with the group's records
+        if (cur.last) {
+            write_tab(ct & 1, nfs_mine);
             __syncwarp();
             load_tab(ct & 1, chunk0 + (ct + 2) * wstride);
             __syncwarp();
             ++ct;
-            ci = 0;
-            continue;
         }
-        stage_ahead();  // the cell in work is staged once this returns
-        const int4 c0 = T.t[ci], c1 = T.t[min(ci + 1, 31)];
-        const int pnb[2] = {MoveTab::nb(c0), MoveTab::nb(c1)};
-        const int pn[2] = {pnb[0] + MoveTab::nt(c0), pnb[1] + MoveTab::nt(c1)};
-        // Two small cells of one system with sorted bottoms go together.
-        if (P.sorted_in && ahead >= 2 && ci + 1 < T.ncell && c1.w == c0.w && c0.w == tsys && pn[0] <= 32 && pn[1] <= 32) {
-            cp_async_wait(ahead - 2);
-            __syncwarp();
-            const int pbase[2] = {c0.x, c1.x};
-            unsigned nfs[2];
-            place_pair<R>(fc, W, tail, pbase, pn, pnb, out, lane, nfs);
-            if (lane == ci) nfs_mine = nfs[0];
-            if (lane == ci + 1) nfs_mine = nfs[1];
-            const int m = pn[0] + pn[1];
-            moved += (unsigned)m;
-            __syncwarp();  // every lane is done with the cells' ring slots
-            tail += m;
-            if (tail >= R) tail -= R;
-            used -= m;
-            ahead -= 2;
-            ci += 2;
-            continue;
-        }
-        cp_async_wait(ahead - 1);
-        __syncwarp();
-
-        const int n = min(pn[0], R);
-        const int base = c0.x;
-        const int sys = c0.w;
-        if (sys != tsys) {
-            if (lane == 0 && tsys >= 0 && moved) atomicAdd(&P.tally[tsys].particle_steps, (unsigned long long)moved);
-            moved = 0;
-            tsys = sys;
-            fc = flight_const(P.sys[sys]);
-        }
-        const SysDev &g = P.sys[sys];
-
-        const int nb = min(pnb[0], n);
-        auto ring = [&](int q) {
-            const int r = tail + q;
-            return r >= R ? r - R : r;
-        };
-        auto rid = [&](int q) { return W.id(ring(q)); };
-        bool viol = false;
-        if (!P.sorted_in)
-            for (int q = lane; q + 1 < nb; q += 32) viol |= !(rid(q) < rid(q + 1));
-        const bool sorted = !__any_sync(0xffffffffu, viol);
-        const unsigned below = (1u << lane) - 1u;
-
-        // Stayers go to the bottom segment in id order, movers to the gap.
-        unsigned n_fs;
-        if (sorted && n <= 32) {
-            n_fs = place_sorted<R, 1>(fc, W, tail, base, n, nb, out, lane);
-        } else if (sorted && n <= 64) {
-            n_fs = place_sorted<R, 2>(fc, W, tail, base, n, nb, out, lane);
+        if (cur.big) {
+            half ^= 1;
+            next_group(cur, half);
         } else {
-            // pass 1: every member's flight; the record goes back into the
-            // ring and pref[q] counts the stayers before member q
-            unsigned S = 0;
-            for (int c0 = 0; c0 < n; c0 += 32) {
-                const int q = c0 + lane;
-                const bool valid = q < n;
-                bool stay = false;
-                if (valid) {
-                    const int r = ring(q);
-                    Particle p;
-                    Split32::unpack(W.a(r), W.b(r), p);
-                    stay = first_flight(g, p);
-                    uint4 ra;
-                    float4 rb;
-                    Split32::pack(p, ra, rb);
-                    W.set(r, ra, rb);
-                }
-                const unsigned fast = __ballot_sync(0xffffffffu, valid && stay);
-                if (valid) W.pref[q] = (uint16_t)(S + (unsigned)__popc(fast & below));
-                S += (unsigned)__popc(fast);
-            }
-            if (lane == 0) W.pref[n] = (uint16_t)S;
-            __syncwarp();
-            // pass 2: stayers in id order, movers below the top of the gap
-            for (int c0 = 0; c0 < n; c0 += 32) {
-                const int q = c0 + lane;
-                if (q < n) {
-                    const int r = ring(q);
-                    const uint32_t id = rid(q);
-                    unsigned dst;
-                    if (W.pref[q + 1] > W.pref[q]) {
-                        unsigned pos;
-                        if (sorted) {
-                            int lb = q;  // bottom members below this id
-                            if (q >= nb) {
-                                int lo = 0, hi = nb;
-                                while (lo < hi) {
-                                    const int mid = (lo + hi) >> 1;
-                                    if (rid(mid) < id) lo = mid + 1;
-                                    else hi = mid;
-                                }
-                                lb = lo;
-                            }
-                            pos = W.pref[lb];
-                            for (int i = nb; i < n; ++i) pos += (W.pref[i + 1] > W.pref[i]) && rid(i) < id;
-                        } else {
-                            pos = 0;
-                            for (int i = 0; i < n; ++i) pos += (W.pref[i + 1] > W.pref[i]) && rid(i) < id;
-                        }
-                        dst = (unsigned)base + pos;
-                    } else {
-                        dst = (unsigned)(base + n) - 1u - ((unsigned)q - W.pref[q]);
-                    }
-                    store_record(out, dst, W.a(r), W.b(r));
-                }
-            }
-            n_fs = S;
+            half ^= 1;
+            cur = nxt;
         }
-        if (lane == ci) nfs_mine = n_fs;
-        moved += (unsigned)n;
-        __syncwarp();  // every lane is done with the cell's ring slots
-        tail += n;
-        if (tail >= R) tail -= R;
-        used -= n;
-        --ahead;
-        ++ci;
     }
+    if (!ok) atomicOr(&P.status->error, DSMC_EBIT_SMEM);
     if (lane == 0 && tsys >= 0 && moved) atomicAdd(&P.tally[tsys].particle_steps, (unsigned long long)moved);
 }
 
@@ -1226,7 +1266,10 @@ __device__ __forceinline__ void flush_walls(const PassParams &P, PlaceSmem &W) {
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(32 * P_WARPS, 5) place_movers_kernel(const __grid_constant__ PassParams P) {
+// Bound by the latency of a mover's chain (record, voxel type, cell map, room,
+// counter, store) over as many warps as fit: at 256^3 108, 103 and 99 us with
+// five, seven and eight blocks per SM (77, 70 and 64 registers).
+__global__ void __launch_bounds__(32 * P_WARPS, 8) place_movers_kernel(const __grid_constant__ PassParams P) {
     __shared__ PlaceSmem smem[P_WARPS];
     const int lane = threadIdx.x & 31;
     const volatile Status *vs = P.status;
