@@ -353,6 +353,11 @@ struct Split32 {
     // A wall voxel's normal and tangents, and a velocity's components in them.
     struct WallFrame {
         float n[3], a[3], b[3];
+        __device__ __forceinline__ void components(const float v[3], float &vn, float &vt1, float &vt2) const {
+            vn = v[0] * n[0] + v[1] * n[1] + v[2] * n[2];
+            vt1 = v[0] * a[0] + v[1] * a[1] + v[2] * a[2];
+            vt2 = v[0] * b[0] + v[1] * b[1] + v[2] * b[2];
+        }
         __device__ __forceinline__ void compose(float vn, float vt1, float vt2, float v[3]) const {
             // rounding spelled out: a caller's -vn folded into the sum would
             // change which product is rounded
@@ -371,14 +376,6 @@ struct Split32 {
         }
         return f;
     }
-    static __device__ __forceinline__ WallFrame wall_frame(const SysDev &g, uint32_t vlin, const float v[3], float &vni,
-                                                           float &vt1i, float &vt2i) {
-        const WallFrame f = load_frame(g, vlin);
-        vni = v[0] * f.n[0] + v[1] * f.n[1] + v[2] * f.n[2];
-        vt1i = v[0] * f.a[0] + v[1] * f.a[1] + v[2] * f.a[2];
-        vt2i = v[0] * f.b[0] + v[1] * f.b[1] + v[2] * f.b[2];
-        return f;
-    }
     // ColliderCercignaniLampis::collide once the normal component is drawn:
     // the tangential components, then the velocity.
     static __device__ __forceinline__ void cl_finish(const SysDev &g, const WallFrame &f, float vn, float vt1i, float vt2i,
@@ -392,10 +389,10 @@ struct Split32 {
     // The wall model's collide: ColliderThermal::collide
     // (dsmc/colliderthermal.cpp:13-46), ColliderSpecular::collide or
     // ColliderCercignaniLampis::collide.  Returns error bits.
-    static __device__ __forceinline__ unsigned reflect(const SysDev &g, uint32_t vlin, float v[3], DrawStream &rs) {
+    static __device__ __forceinline__ unsigned reflect(const SysDev &g, const WallFrame &f, float v[3], DrawStream &rs) {
         if (g.wall_model != DSMC_WALL_THERMAL) {
             float vni, vt1i, vt2i, vn;
-            const WallFrame f = wall_frame(g, vlin, v, vni, vt1i, vt2i);
+            f.components(v, vni, vt1i, vt2i);
             if (g.wall_model == DSMC_WALL_SPECULAR) {
                 f.compose(-vni, vt1i, vt2i, v);
                 return 0;
@@ -409,7 +406,7 @@ struct Split32 {
         }
         float vt[3];
         thermal_draw(g, rs, vt);
-        load_frame(g, vlin).compose(vt[0], vt[1], vt[2], v);
+        f.compose(vt[0], vt[1], vt[2], v);
         return 0;
     }
 
@@ -448,7 +445,7 @@ struct Split32 {
     // that subtraction drifts by an ulp, which is more than the 1e-7 time
     // units the reference leaves before a face for slow particles, so the
     // sub-step's start position is kept and restored instead.
-    static __device__ __noinline__ void move_general(const SysDev &g, Particle &p, uint32_t step, MoveTally &t) {
+    static __device__ __forceinline__ void move_general(const SysDev &g, Particle &p, uint32_t step, MoveTally &t) {
         DrawStream rs;
         rs.init(g.seed, p.id, step, DSMC_TAG_MOVE);
         float w[3] = {p.v[0] * g.inv_vox_f[0], p.v[1] * g.inv_vox_f[1], p.v[2] * g.inv_vox_f[2]};
@@ -465,7 +462,8 @@ struct Split32 {
             const float o0[3] = {p.o[0], p.o[1], p.o[2]};
             float tau = dt;
             advance(p.c, p.o, w, tau);
-            int vt = voxel_type(g, p.c[0], p.c[1], p.c[2]);
+            uint32_t lin = voxel_linear(g, p.c[0], p.c[1], p.c[2]);  // the last lookup's voxel
+            int vt = __ldg(g.vox + lin);
             if (vt == DSMC_VOX_EMPTY) break;
             // Bisect back out of solid (wall) voxels until a boundary voxel.
             bool stop = false, again = false;
@@ -480,7 +478,8 @@ struct Split32 {
                 if (vt == DSMC_VOX_WALL) {
                     tau *= 0.5f;
                     advance(p.c, p.o, w, -tau);
-                    vt = voxel_type(g, p.c[0], p.c[1], p.c[2]);
+                    lin = voxel_linear(g, p.c[0], p.c[1], p.c[2]);
+                    vt = __ldg(g.vox + lin);
                 } else {
                     dt -= tau;
                     again = dt > 1e-5f && depth < 10;
@@ -491,7 +490,9 @@ struct Split32 {
             if (stop) break;
             if (again) continue;
             // Back off and stop just short of the first boundary voxel's face.
+            // (the wall's frame is loaded as soon as its voxel is known)
             int cb[3] = {p.c[0], p.c[1], p.c[2]};
+            WallFrame frame = {};
             count = 0;
             while (vt == DSMC_VOX_BOUNDARY) {
                 if (++count > 100) {
@@ -503,6 +504,7 @@ struct Split32 {
                 cb[0] = p.c[0];
                 cb[1] = p.c[1];
                 cb[2] = p.c[2];
+                frame = load_frame(g, lin);
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
                     p.c[a] = c0[a];
@@ -540,12 +542,13 @@ struct Split32 {
                         p.o[2] = oo;
                     }
                 }
-                vt = voxel_type(g, p.c[0], p.c[1], p.c[2]);
+                lin = voxel_linear(g, p.c[0], p.c[1], p.c[2]);
+                vt = __ldg(g.vox + lin);
             }
             if (stop) break;
             here = vt;
             dt -= tau;
-            t.err |= reflect(g, voxel_linear(g, cb[0], cb[1], cb[2]), p.v, rs);
+            t.err |= reflect(g, frame, p.v, rs);
             ++t.wall_hits;
 #pragma unroll
             for (int d = 0; d < 3; ++d) w[d] = p.v[d] * g.inv_vox_f[d];
@@ -562,12 +565,9 @@ struct Split32 {
     // the same order per particle as move_general.  All lanes call; inactive
     // lanes only keep the loop company.
     //
-    // What bounds it is one flight's serial chain (a flight of ten reflections
-    // lasts longer than the rest of the kernel), so the chain's parts overlap:
-    // the wall's frame is loaded when its voxel is found, before the facet
-    // arithmetic and the next lookup; a diffuse wall's draws (Philox, log,
-    // cos) are made while a lookup is in flight.  They are used, and the
-    // stream moved past them, only if the flight does reflect.
+    // For Cercignani-Lampis walls, whose sampler the whole warp runs; with the
+    // other models a flight on its own lane is through sooner (no dispatch, no
+    // turns shared with other states).
     static __device__ __forceinline__ void move_general_warp(const SysDev &g, Particle &p, uint32_t step,
                                                              MoveTally &t, bool active) {
         enum { S_START, S_FIRST, S_BISECT, S_FACET, S_REFLECT, S_CL, S_RESEED, S_DONE };
@@ -581,11 +581,6 @@ struct Split32 {
         int c0[3] = {0, 0, 0}, cb[3] = {0, 0, 0};
         float o0[3] = {0.0f, 0.0f, 0.0f};
         int state = active ? S_START : S_DONE;
-        const bool diffuse = g.wall_model == DSMC_WALL_THERMAL;
-        WallFrame frame = {};
-        float drawn[3] = {0.0f, 0.0f, 0.0f};  // the next reflection's components, once made
-        DrawStream after = rs;                // the stream past them
-        bool have = false;
         while (__any_sync(0xffffffffu, state != S_DONE)) {
             bool look = false;
             while (state < S_CL && !look) {
@@ -645,7 +640,6 @@ struct Split32 {
                         cb[1] = p.c[1];
                         cb[2] = p.c[2];
                         wlin = lin;
-                        if (diffuse) frame = load_frame(g, wlin);
 #pragma unroll
                         for (int a = 0; a < 3; ++a) {
                             p.c[a] = c0[a];
@@ -684,26 +678,7 @@ struct Split32 {
                 } else {  // S_REFLECT
                     here = vt;
                     dt -= tau;
-                    if (g.wall_model == DSMC_WALL_CL) {
-                        state = S_CL;  // its sampler runs on the whole warp
-                        continue;
-                    }
-                    if (diffuse) {
-                        frame.compose(drawn[0], drawn[1], drawn[2], p.v);
-                        rs = after;
-                        have = false;
-                    } else {
-                        t.err |= reflect(g, wlin, p.v, rs);
-                    }
-                    ++t.wall_hits;
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) w[d] = p.v[d] * g.inv_vox_f[d];
-                    if (!(dt > 1e-5f && depth < 10)) {
-                        state = S_DONE;
-                    } else {
-                        ++depth;
-                        state = S_START;
-                    }
+                    state = S_CL;  // the wall's sampler runs on the whole warp
                 }
             }
             if (look) {
@@ -715,18 +690,16 @@ struct Split32 {
                 if (!reseed(g, p, rs)) t.err |= DSMC_EBIT_RESEED;
                 state = S_DONE;
             }
-            if (diffuse && state != S_DONE && !have) {
-                after = rs;
-                thermal_draw(g, after, drawn);
-                have = true;
-            }
             const unsigned cl = __ballot_sync(0xffffffffu, state == S_CL);
             if (cl) {
                 const bool mine = state == S_CL;
                 WallFrame f;
                 float vni = 0.0f, vt1i = 0.0f, vt2i = 0.0f, vn = 0.0f;
                 bool ok = false;
-                if (mine) f = wall_frame(g, wlin, p.v, vni, vt1i, vt2i);
+                if (mine) {
+                    f = load_frame(g, wlin);
+                    f.components(p.v, vni, vt1i, vt2i);
+                }
                 cl_normal_warp(cl, vni, sqrtf(2.0f) * g.wall_s_f, g.cl_vmax_f, g.sqrt_an_over_2_f, g.sqrt_1m_an_f,
                                g.sqrt_1m_an_over_an_f, rs, ok, vn);
                 if (mine) {
@@ -814,8 +787,11 @@ struct Split32 {
                 return false;
             }
         }
-        move_general(g, p, step, t);
+        move_general_call(g, p, step, t);
         return true;
+    }
+    static __device__ __noinline__ void move_general_call(const SysDev &g, Particle &p, uint32_t step, MoveTally &t) {
+        move_general(g, p, step, t);
     }
 
     // Cell of the particle: whole voxels per cell, so cell = voxel / vpc.

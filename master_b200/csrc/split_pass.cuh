@@ -1364,12 +1364,14 @@ __global__ void __launch_bounds__(32 * P_WARPS, 8) place_movers_kernel(const __g
 
 // The general mover for every listed wall flight, one per lane, then the
 // placement.  Bound by the longest flight's serial chain (ten reflections of
-// about 3 us each) and, with many flights, by the divergence of a warp's.
-// Measured, us per step before and after the claims sized to the grid, the
-// overlapped draws and frames and the warp-shared Cercignani-Lampis trials:
-// 64^3 (2e3 flights) 42 -> 35, 128^3 (1.8e4) 61 -> 49, with CL walls of
-// alpha_n = 0.8 524 -> 104, 256^3 (1.5e5) 93 -> 87.  Held to fewer registers
-// (128, 102, 85 for 4, 5, 6 blocks per SM) it spills: 37, 40 and 44 us at 64^3.  The last block ends the pass: it advances the step and halts
+// about 2 us each) and, with many flights, by the divergence of a warp's.
+// Measured, us per step at 64^3 (2e3 flights) / 128^3 (1.8e4) / 256^3 (1.5e5):
+// a warp-wide state machine with claims of 32 42 / 61 / 93; claims sized to the
+// grid, draws and frames overlapped 35 / 47 / 78; each flight on its own lane,
+// without the machine, 27 / 35 / 65.  With Cercignani-Lampis walls (128^3,
+// alpha_n = 0.8) 524, with the trials shared by the warp 91.  Held to fewer
+// registers (128, 102, 85 for 4, 5, 6 blocks per SM) the machine spilled: 37, 40
+// and 44 us at 64^3.  The last block ends the pass: it advances the step and halts
 // the pipeline if anything spilled or failed.
 __global__ void __launch_bounds__(32 * W_WARPS) place_walls_kernel(const __grid_constant__ PassParams P) {
     const int lane = threadIdx.x & 31;
@@ -1421,7 +1423,12 @@ __global__ void __launch_bounds__(32 * W_WARPS) place_walls_kernel(const __grid_
         for (unsigned todo = __ballot_sync(0xffffffffu, valid); todo;) {
             const int sys = __shfl_sync(0xffffffffu, s0, __ffs(todo) - 1);
             const bool mine = valid && s0 == sys;
-            Split32::move_general_warp(P.sys[sys], p, move_step, mt, mine);
+            const SysDev &g = P.sys[sys];
+            if (g.wall_model == DSMC_WALL_CL)
+                Split32::move_general_warp(g, p, move_step, mt, mine);
+            else if (mine)
+                Split32::move_general(g, p, move_step, mt);
+            __syncwarp();
             todo &= ~__ballot_sync(0xffffffffu, mine);
         }
         if (valid) place = new_cell(P.sys[esys], p, e.y, key, leave, cnt, mt.err);
