@@ -208,6 +208,54 @@ def test_conv_edges_of_the_plane_kernels(B, S, cin, cout):
     assert rel_l2(dw.cpu().numpy(), rdw.cpu().numpy()) <= 1e-4
 
 
+@pytest.mark.parametrize("B,S,c,cs,off", [(1, 4, 16, 16, 0), (3, 8, 48, 64, 16), (2, 16, 128, 128, 0), (1, 16, 8, 24, 8),
+                                          (2, 8, 20, 24, 1), (1, 2, 128, 128, 0)])
+def test_bias_gradient_shapes(B, S, c, cs, off):
+    """16-byte chunks (channel counts whose chunks do and do not divide the
+    block, fewer rows than blocks, a view) and the scalar kernel (20 channels
+    at an odd offset) against fp64; fp32 sums of at most 8192 rows in blocks
+    of a few hundred: relative error below 1e-4 of the sums' scale."""
+    g = torch.Generator().manual_seed(c + S)
+    x = rnd_bf16((B, S, S, S, cs), g)
+    db = torch.ones(c, device=DEV)  # accumulated
+    d = x.to(DEV)
+    capi.check(lib().dsmc_sg_bias_grad(stream(), B, S, P(d), cs, off, c, P(db)))
+    ref = 1.0 + x[..., off:off + c].double().sum(dim=(0, 1, 2, 3))
+    scale = x[..., off:off + c].double().abs().sum(dim=(0, 1, 2, 3)).max().item()
+    assert (db.cpu().double() - ref).abs().max().item() <= 1e-4 * scale
+
+
+@pytest.mark.parametrize("B,S", [(1, 2), (3, 4), (2, 16)])
+def test_loss_and_head_backward_rows(B, S):
+    """Loss, head gradients and input gradient at few rows (fewer than a
+    warp's eight), rows that do not fill the last turn, and many; fp32
+    products summed in another order than fp64: 1e-4 of each tensor's norm,
+    the bf16 input gradient to its rounding."""
+    g = torch.Generator().manual_seed(S)
+    e = torch.relu(torch.randn((B, S, S, S, 16), generator=g)).to(torch.bfloat16)
+    wh = torch.randn((4, 16), generator=g)
+    out, tgt = torch.randn((B, S, S, S, 4), generator=g), torch.randn((B, S, S, S, 4), generator=g)
+    valid = (torch.rand((B, S, S, S), generator=g) < 0.6).to(torch.uint8)
+    cw = torch.tensor([1.0, 4.0, 1.0, 0.5])
+    coef = torch.randn(B, generator=g, dtype=torch.float64)
+    inv = 1.0 / max(1, int(valid.sum()))
+    d = [t.to(DEV) for t in (out, tgt, valid, cw, e, wh, coef)]
+    dwh, dbh = torch.zeros((4, 16), device=DEV), torch.zeros(4, device=DEV)
+    de = torch.zeros_like(d[4])
+    loss = torch.zeros(1, dtype=torch.float64, device=DEV)
+    capi.check(lib().dsmc_sg_loss_head_bwd(stream(), B, S, P(d[0]), P(d[1]), P(d[2]), P(d[3]), C.c_float(inv), P(d[4]), 16, 0,
+                                           P(d[5]), P(dwh), P(dbh), P(de), 16, 0, P(loss), P(d[6]), 1))
+    v = valid.double()[..., None]
+    diff = (out - tgt).double() * v
+    dout = 2.0 * cw.double() * diff * inv
+    dout[..., 1] += coef.reshape(B, 1, 1, 1) * v[..., 0]
+    ed = e.double()
+    assert abs(loss.item() - float((cw.double() * diff ** 2).sum() * inv)) <= 1e-5 * abs(loss.item())
+    assert rel_l2(dwh.cpu().numpy(), (dout.reshape(-1, 4).T @ ed.reshape(-1, 16)).numpy()) <= 1e-4
+    assert rel_l2(dbh.cpu().numpy(), dout.reshape(-1, 4).sum(0).numpy()) <= 1e-4
+    close_bf16(de, (dout @ wh.double()) * (ed > 0))
+
+
 def test_pool_and_upsample_forward_and_backward():
     g = torch.Generator().manual_seed(11)
     B, S, Cc = 2, 16, 32
