@@ -390,7 +390,7 @@ int flush_pending(dsmc_ctx *ctx);
 // One production pass from its cached graph, captured on first use.
 cudaError_t launch_fused_graph(dsmc_ctx *ctx, const PassParams &P) {
     const int key = P.cur | (P.cin << 1) | (P.sorted_in << 3) | (P.do_collide << 4) | (P.do_sample << 5) |
-                    (P.do_move << 6);
+                    (P.do_move << 6) | (P.any_cl << 7);
     auto it = ctx->graphs.find(key);
     if (it == ctx->graphs.end()) {
         cudaGraph_t g = nullptr;
@@ -430,6 +430,8 @@ PassParams pass_params(dsmc_ctx *ctx, int do_collide, int do_move, int do_sample
     P.advance_step = advance;
     P.ring = ctx->tune_ring;
     P.claim = ctx->tune_claim;
+    P.any_cl = 0;
+    for (const auto &s : ctx->systems) P.any_cl |= s->dev.wall_model == DSMC_WALL_CL ? 1 : 0;
     return P;
 }
 

@@ -193,6 +193,7 @@ struct PassParams {
     int advance_step;          // increment Status::step at the end of the pass
     int ring;                  // production pass: move_cells ring slots per warp (0: the smallest that fits)
     int claim;                 // production pass: collide_cells chunk claims (0 auto, 1 stride, 2 counter)
+    int any_cl;                // some system has Cercignani-Lampis walls
     int chunk;                 // production pass: cells per chunk of this launch (at most 32)
 };
 

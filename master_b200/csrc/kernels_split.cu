@@ -27,7 +27,8 @@ static PassParams with_chunk(const PassParams &P, long long warps) {
 }
 
 // The production pass (split_pass.cuh): collide_cells, move_cells with the
-// smallest ring that holds the largest cell, place_movers, place_walls.
+// smallest ring that holds the largest cell, place_movers, and place_walls
+// where place_movers lists its wall flights.
 template <int R> static cudaError_t launch_move_ring(const PassParams &P, int grid, cudaStream_t st) {
     pass3::move_cells_kernel<R><<<grid, 32 * pass3::M_WARPS, pass3::move_smem_bytes<R>(), st>>>(
         with_chunk(P, (long long)grid * pass3::M_WARPS));
@@ -95,7 +96,7 @@ int fused_grids(int smem_cap, int num_sms, int grids[5], int ring, int max_bps[5
     }
     const int bc = std::min(static_blocks(pass3::collide_cells_kernel<false>, 32 * pass3::C_WARPS),
                             static_blocks(pass3::collide_cells_kernel<true>, 32 * pass3::C_WARPS));
-    const int bp = static_blocks(pass3::place_movers_kernel, 32 * pass3::P_WARPS);
+    const int bp = static_blocks(pass3::place_movers_kernel<false>, 32 * pass3::P_WARPS);
     const int bw = static_blocks(pass3::place_walls_kernel, 32 * pass3::W_WARPS);
     const int bs = static_blocks(pass3::sample_cells_kernel, 32 * pass3::C_WARPS);
     if (bm <= 0 || bc <= 0 || bp <= 0 || bw <= 0 || bs <= 0) return 0;
@@ -150,13 +151,23 @@ cudaError_t launch_fused(const PassParams &P, const int grids[5], cudaStream_t s
     }
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[2], st);
-    pass3::place_movers_kernel<<<grids[2], 32 * pass3::P_WARPS, 0, st>>>(
-        with_chunk(P, (long long)grids[2] * pass3::P_WARPS));
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    if (ev) cudaEventRecord(ev[3], st);
-    pass3::place_walls_kernel<<<grids[3], 32 * pass3::W_WARPS, 0, st>>>(P);
-    e = cudaGetLastError();
+    // each warp its own wall flights, up to four chunks of cells per warp (its
+    // comment); half the blocks of the listing kernel fit
+    const int own_grid = std::max(1, grids[2] / 2);
+    const long long own_warps = (long long)own_grid * pass3::P_WARPS;
+    if (!P.any_cl && P.cells.num_cells <= 4 * 32 * own_warps) {
+        pass3::place_movers_kernel<true><<<own_grid, 32 * pass3::P_WARPS, 0, st>>>(with_chunk(P, own_warps));
+        e = cudaGetLastError();
+        if (ev) cudaEventRecord(ev[3], st);
+    } else {
+        pass3::place_movers_kernel<false><<<grids[2], 32 * pass3::P_WARPS, 0, st>>>(
+            with_chunk(P, (long long)grids[2] * pass3::P_WARPS));
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        if (ev) cudaEventRecord(ev[3], st);
+        pass3::place_walls_kernel<<<grids[3], 32 * pass3::W_WARPS, 0, st>>>(P);
+        e = cudaGetLastError();
+    }
     if (ev) cudaEventRecord(ev[4], st);
     return e;
 }

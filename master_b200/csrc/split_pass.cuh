@@ -1,5 +1,5 @@
-// The production timestep pass for split-precision state: four kernels per
-// step (five on sampled steps) over the active cells, which the previous pass
+// The production timestep pass for split-precision state: three or four
+// kernels per step (one more on sampled steps) over the active cells, which the previous pass
 // left sorted by cell (bottom segment + top segment of each cell's slots,
 // counts in the `cin` occupancy set).
 //
@@ -25,11 +25,12 @@
 //   place_movers   A mover whose flight ends in an empty voxel completes it
 //                  and takes a top slot of its new cell (warp-aggregated
 //                  atomics; the spill list when the cell is full).  Flights
-//                  that meet a wall go to a list of (slot, source cell)
-//                  pairs.
-//   place_walls    The general mover (bisection, facet, diffuse wall) for
-//                  the listed flights, then the same placement.  The last
-//                  block ends the pass (step counter, halting).
+//                  that meet a wall go through the general mover
+//                  (bisection, facet, wall model) and the same placement: by
+//                  the warp that found them (few cells), or from a list of
+//                  (slot, source cell) pairs by
+//   place_walls    where there are many.  The last block of the last kernel
+//                  ends the pass (step counter, halting).
 //
 // Top slots are taken from the top of the cell down and never below
 // base + n_in(cell), so they cannot meet the bottom segment or the gap.
@@ -37,9 +38,9 @@
 // Member order: move_cells writes each cell's stayers in id order, so a
 // bottom segment is normally sorted by id and only the few arrivals of the
 // top segment are out of order.  The id rank of a member (the reference's
-// cell-list order) is then its bottom position plus the arrivals below it,
-// which collide_cells and move_cells compute with one shuffle and ballot per
-// arrival.  A cell whose bottom segment is not sorted (after a repack or the
+// cell-list order) is then its bottom position plus the arrivals below it:
+// move_cells computes it with one shuffle and ballot per arrival, collide_cells
+// turns a picked rank into its member by the bottom ids next to it.  A cell whose bottom segment is not sorted (after a repack or the
 // stand-alone stage kernels) is ranked in full and leaves move_cells sorted.
 #pragma once
 #include "engine.cuh"
@@ -1120,10 +1121,10 @@ template <int R> constexpr size_t move_smem_bytes() { return sizeof(MoveSmem<R>)
 
 constexpr int P_WARPS = 4;
 constexpr int W_WARPS = 4;
-constexpr int WQ = 32;  // wall-flight entries a warp collects before appending them to the list
+constexpr int WQ = 64;  // wall flights a warp collects: 31 left over and a turn's 32 fit
 
 struct PlaceSmem {
-    int2 q[WQ];  // {output slot, system}
+    int2 q[WQ];  // {output slot, source cell}
     int qn;
 };
 
@@ -1249,31 +1250,116 @@ __device__ __forceinline__ void leave_slab(const PassParams &P, const Split32::P
     }
 }
 
-// Appends the warp's collected wall flights to the list (one atomic per
-// batch).  All lanes call.
-__device__ __forceinline__ void flush_walls(const PassParams &P, PlaceSmem &W) {
+// Takes up to 32 of the warp's collected wall flights, one per lane (true in
+// the lanes that got one).  All lanes call.
+__device__ __forceinline__ bool pop_walls(PlaceSmem &W, int2 &e) {
     const int lane = threadIdx.x & 31;
-    const int qn = W.qn;
+    const int qn = W.qn, n = min(qn, 32);
+    e = lane < n ? W.q[qn - n + lane] : make_int2(0, -1);
+    __syncwarp();
+    if (lane == 0) W.qn = qn - n;
+    __syncwarp();
+    return lane < n;
+}
+
+// Appends the valid lanes' wall flights to the list (one atomic).  All lanes call.
+__device__ __forceinline__ void list_walls(const PassParams &P, int2 e, bool valid) {
+    const int lane = threadIdx.x & 31;
+    const int n = __popc(__ballot_sync(0xffffffffu, valid));  // the first n lanes
     unsigned at = 0;
-    if (lane == 0 && qn) at = atomicAdd(&P.status->walls, (unsigned)qn);
+    if (lane == 0 && n) at = atomicAdd(&P.status->walls, (unsigned)n);
     at = __shfl_sync(0xffffffffu, at, 0);
-    if (lane < qn) {
-        if (at + lane < P.parts.walls_cap) P.parts.walls[at + lane] = W.q[lane];
+    if (valid) {
+        if (at + lane < P.parts.walls_cap) P.parts.walls[at + lane] = e;
         else atomicOr(&P.status->error, DSMC_EBIT_SPILL_FULL);  // cannot happen: one entry per slot at most
     }
-    __syncwarp();
-    if (lane == 0) W.qn = 0;
-    __syncwarp();
+}
+
+// The general mover for the listed wall flights of the valid lanes, {output
+// slot, source cell} each, then their placement.  All lanes call; tsys as
+// counts_publish's.  CL: some system may have Cercignani-Lampis walls.
+template <bool CL>
+__device__ __forceinline__ void wall_flights(const PassParams &P, uint32_t move_step, int2 e, bool valid,
+                                             MoveCounts &cnt, int &tsys) {
+    const int esys = valid ? P.cells.meta[e.y].w : -1;
+    const int csys = common_system(valid, esys);
+    if (csys != tsys) {
+        counts_publish(P, tsys, cnt, false);
+        tsys = csys;
+    }
+    Split32::Particle p;
+    MoveTally mt;
+    mt.wall_hits = mt.reseeds = 0;
+    mt.cross[0] = mt.cross[1] = mt.cross[2] = 0;
+    mt.err = 0;
+    unsigned key = 0;
+    bool place = false, leave = false;
+    if (valid) {
+        uint4 ra;
+        float4 rb;
+        load_record(P.parts.A[P.cur ^ 1], e.x, ra, rb);
+        Split32::unpack(ra, rb, p);
+    }
+    // the lanes of a warp share their system unless it is mixed; a mixed
+    // warp moves its lanes one system at a time
+    for (unsigned todo = __ballot_sync(0xffffffffu, valid); todo;) {
+        const int sys = __shfl_sync(0xffffffffu, esys, __ffs(todo) - 1);
+        const bool mine = valid && esys == sys;
+        const SysDev &g = P.sys[sys];
+        if (CL && g.wall_model == DSMC_WALL_CL)
+            Split32::move_general_warp(g, p, move_step, mt, mine);
+        else if (mine)
+            Split32::move_general(g, p, move_step, mt);
+        __syncwarp();
+        todo &= ~__ballot_sync(0xffffffffu, mine);
+    }
+    if (valid) place = new_cell(P.sys[esys], p, e.y, key, leave, cnt, mt.err);
+    insert_top(P, p, place, key, mt.err);
+    leave_slab(P, p, leave, mt.err);
+    counts_add(cnt, mt);
+    if (tsys == -2) counts_publish(P, esys, cnt, true);
+}
+
+// The last block ends the pass: it advances the step and halts the pipeline
+// if anything spilled or failed.
+__device__ __forceinline__ void end_split_pass(const PassParams &P) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned done = atomicAdd(&P.status->blocks_done, 1u);
+        if (done == gridDim.x - 1) {
+            __threadfence();
+            if (P.advance_step) atomicAdd(&P.status->step, 1u);
+            if (atomicAdd(&P.status->spill, 0u) != 0u || (atomicAdd(&P.status->error, 0u) & DSMC_EBIT_FATAL) != 0u)
+                atomicExch(&P.status->halted, 1u);
+            atomicExch(&P.status->walls, 0u);
+            atomicExch(&P.status->walls_taken, 0u);
+            atomicExch(&P.status->collide_taken, 0u);
+            atomicExch(&P.status->blocks_done, 0u);
+        }
+    }
 }
 
 // Bound by the latency of a mover's chain (record, voxel type, cell map, room,
 // counter, store) over as many warps as fit: at 256^3 108, 103 and 99 us with
 // five, seven and eight blocks per SM (77, 70 and 64 registers).
-__global__ void __launch_bounds__(32 * P_WARPS, 8) place_movers_kernel(const __grid_constant__ PassParams P) {
+//
+// OWN: a warp moves its own wall flights, 32 at a time and the rest at its end,
+// and the kernel ends the pass; otherwise they go to place_walls' list.  The
+// general mover takes 123 registers (four blocks per SM; held to 102 and 85,
+// 45.2 and 46.8 us per step against 44.9 at 64^3), which costs the placing of
+// many movers more than a launch and the list's turn-around: us per step, both
+// kernels, list -> own: 64^3 (2e4 cells) 39 -> 28, 128^3 (2e5) 60 -> 49, 160^3
+// (3.5e5) 76 -> 68 in all 226 -> 223, 192^3 (6e5) 92 -> 99, 256^3 162 -> 193.
+// Cercignani-Lampis flights are always listed: their warps share the rejection
+// trials, so equal claims matter more (64^3 69 -> 182, 128^3 119 -> 393).
+template <bool OWN>
+__global__ void __launch_bounds__(32 * P_WARPS, OWN ? 4 : 8) place_movers_kernel(const __grid_constant__ PassParams P) {
     __shared__ PlaceSmem smem[P_WARPS];
     const int lane = threadIdx.x & 31;
     const volatile Status *vs = P.status;
     if (vs->halted) return;
+    const uint32_t move_step = vs->step + 1;
     PlaceSmem &W = smem[threadIdx.x >> 5];
     if (lane == 0) W.qn = 0;
     __syncwarp();
@@ -1283,6 +1369,13 @@ __global__ void __launch_bounds__(32 * P_WARPS, 8) place_movers_kernel(const __g
     counts_reset(cnt);
     int tsys = -1;
 
+    // the flights collected so far: moved here (OWN), or appended to the list
+    auto walls = [&]() {
+        int2 e;
+        const bool valid = pop_walls(W, e);
+        if (OWN) wall_flights<false>(P, move_step, e, valid, cnt, tsys);
+        else list_walls(P, e, valid);
+    };
     const int C = P.cells.num_cells, CH = P.chunk;
     const int nchunks = (C + CH - 1) / CH;
     for (int ch = blockIdx.x * P_WARPS + (threadIdx.x >> 5); ch < nchunks; ch += gridDim.x * P_WARPS) {
@@ -1346,7 +1439,6 @@ __global__ void __launch_bounds__(32 * P_WARPS, 8) place_movers_kernel(const __g
             // flights that meet a wall stay in their slot for place_walls
             const unsigned wall = __ballot_sync(0xffffffffu, valid && !done);
             if (wall) {
-                if (W.qn + __popc(wall) > WQ) flush_walls(P, W);
                 if (valid && !done) W.q[W.qn + __popc(wall & ((1u << lane) - 1u))] = make_int2(slot, src);
                 __syncwarp();
                 if (lane == 0) W.qn += __popc(wall);
@@ -1356,10 +1448,12 @@ __global__ void __launch_bounds__(32 * P_WARPS, 8) place_movers_kernel(const __g
             leave_slab(P, p, leave, mt.err);
             counts_add(cnt, mt);
             if (tsys == -2) counts_publish(P, psys, cnt, true);
+            if (W.qn >= 32) walls();
         }
     }
-    if (W.qn) flush_walls(P, W);
+    if (W.qn) walls();
     counts_publish(P, tsys, cnt, false);
+    if (OWN) end_split_pass(P);
 }
 
 // The general mover for every listed wall flight, one per lane, then the
@@ -1371,15 +1465,13 @@ __global__ void __launch_bounds__(32 * P_WARPS, 8) place_movers_kernel(const __g
 // without the machine, 27 / 35 / 65.  With Cercignani-Lampis walls (128^3,
 // alpha_n = 0.8) 524, with the trials shared by the warp 91.  Held to fewer
 // registers (128, 102, 85 for 4, 5, 6 blocks per SM) the machine spilled: 37, 40
-// and 44 us at 64^3.  The last block ends the pass: it advances the step and halts
-// the pipeline if anything spilled or failed.
+// and 44 us at 64^3.
 __global__ void __launch_bounds__(32 * W_WARPS) place_walls_kernel(const __grid_constant__ PassParams P) {
     const int lane = threadIdx.x & 31;
     const volatile Status *vs = P.status;
     if (vs->halted) return;
     const uint32_t move_step = vs->step + 1;
     const unsigned nwalls = min(vs->walls, P.parts.walls_cap);
-    const void *out = P.parts.A[P.cur ^ 1];
     MoveCounts cnt;
     counts_reset(cnt);
     int tsys = -1;
@@ -1398,62 +1490,10 @@ __global__ void __launch_bounds__(32 * W_WARPS) place_walls_kernel(const __grid_
         const unsigned i = i0 + lane;
         const bool valid = (unsigned)lane < claim && i < nwalls;
         const int2 e = valid ? P.parts.walls[i] : make_int2(0, -1);  // {slot, source cell}
-        const int esys = valid ? P.cells.meta[e.y].w : -1;
-        const int csys = common_system(valid, esys);
-        if (csys != tsys) {
-            counts_publish(P, tsys, cnt, false);
-            tsys = csys;
-        }
-        Split32::Particle p;
-        MoveTally mt;
-        mt.wall_hits = mt.reseeds = 0;
-        mt.cross[0] = mt.cross[1] = mt.cross[2] = 0;
-        mt.err = 0;
-        unsigned key = 0;
-        bool place = false, leave = false;
-        // the lanes of a warp share their system unless it is mixed; a mixed
-        // warp moves its lanes one system at a time
-        const int s0 = esys;
-        if (valid) {
-            uint4 ra;
-            float4 rb;
-            load_record(out, e.x, ra, rb);
-            Split32::unpack(ra, rb, p);
-        }
-        for (unsigned todo = __ballot_sync(0xffffffffu, valid); todo;) {
-            const int sys = __shfl_sync(0xffffffffu, s0, __ffs(todo) - 1);
-            const bool mine = valid && s0 == sys;
-            const SysDev &g = P.sys[sys];
-            if (g.wall_model == DSMC_WALL_CL)
-                Split32::move_general_warp(g, p, move_step, mt, mine);
-            else if (mine)
-                Split32::move_general(g, p, move_step, mt);
-            __syncwarp();
-            todo &= ~__ballot_sync(0xffffffffu, mine);
-        }
-        if (valid) place = new_cell(P.sys[esys], p, e.y, key, leave, cnt, mt.err);
-        insert_top(P, p, place, key, mt.err);
-        leave_slab(P, p, leave, mt.err);
-        counts_add(cnt, mt);
-        if (tsys == -2) counts_publish(P, esys, cnt, true);
+        wall_flights<true>(P, move_step, e, valid, cnt, tsys);
     }
     counts_publish(P, tsys, cnt, false);
-
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned done = atomicAdd(&P.status->blocks_done, 1u);
-        if (done == gridDim.x - 1) {
-            __threadfence();
-            if (P.advance_step) atomicAdd(&P.status->step, 1u);
-            if (atomicAdd(&P.status->spill, 0u) != 0u || (atomicAdd(&P.status->error, 0u) & DSMC_EBIT_FATAL) != 0u)
-                atomicExch(&P.status->halted, 1u);
-            atomicExch(&P.status->walls, 0u);
-            atomicExch(&P.status->walls_taken, 0u);
-            atomicExch(&P.status->collide_taken, 0u);
-            atomicExch(&P.status->blocks_done, 0u);
-        }
-    }
+    end_split_pass(P);
 }
 
 // ---- slab exchange ----------------------------------------------------------

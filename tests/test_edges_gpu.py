@@ -202,3 +202,27 @@ def test_wall_flights_few_and_many(n, per_cell, dt_si, model, alpha_n):
     A, B = System(s, g), System(s, g)
     run_both(A, B, 3)
     assert A.tallies().wall_collisions > 0
+
+
+@pytest.mark.parametrize("cells,per_cell,dt_si,model", [(64, 3, 2e-11, 0), (64, 3, 2e-11, 1), (32, 60, 1e-10, 0), (16, 20, 1e-11, 0)])
+def test_wall_flights_own_and_listed(cells, per_cell, dt_si, model):
+    """place_movers with a quarter of an SM's blocks and with all: at 64^3
+    cells (1.6e5 active) the first lists its wall flights and the second has
+    each warp move its own; at 32^3 and 16^3 both move their own, the first with several
+    turns of 32 flights per warp.  The state is the same bit for bit."""
+    from master_b200 import autotune
+    w = Workload("walls", n=64, radius_voxels=3.0, porosity=0.6, geometry_seed=5, cells=cells,
+                 atoms_per_molecule=simulators_per_cell_weight(2.5e24, 0.1, 2, per_cell * (cells / 32.0) ** 3), dt_si=dt_si)
+    g = w.geometry()
+    s = w.settings(rng_seed=11, statistics_interval=10 ** 9)
+    s.surface_model = model
+    A, B = System(s, g), System(s, g)
+    autotune.set_tuning(A.ctx, (0, 0, 1, 0, 0))
+    for S in (A, B):
+        assert S.ctx.pass_info()["pipelined"] == 1
+        S.step(4)
+    (ra, va), (rb, vb) = A.get_particles(), B.get_particles()
+    assert np.array_equal(ra, rb) and np.array_equal(va, vb)
+    ta, tb = A.tallies(), B.tallies()
+    assert ta.wall_collisions == tb.wall_collisions > 0 and ta.collisions == tb.collisions
+    assert A.ctx.device_status()[0] & capi.EBIT_FATAL == 0
