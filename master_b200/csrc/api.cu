@@ -138,6 +138,7 @@ struct dsmc_ctx {
     DevBuf<unsigned long long> cursor;
     DevBuf<double> io_r, io_v;
     DevBuf<int> io_cell;
+    DevBuf<double> cells_out;  // dsmc_cells_get's arrays
     DevBuf<double> cell_energy;  // dsmc_tallies_get: per-cell kinetic-energy sums
     // launch shape of the cell pass
     int block = 256;
@@ -162,12 +163,20 @@ struct dsmc_ctx {
     double cap_factor = 2.0;
     int cap_pad = 24;
     // The production pass as CUDA graphs, one per pass configuration (buffer
-    // parity, occupancy set, sorted bottoms, collide, sample); every buffer
-    // pointer is baked into the graphs, so any (re)allocation drops them.
+    // parity, occupancy set, sorted bottoms, collide, sample).  Parameters and
+    // grids are baked into a graph: it is launched for a pass with the same
+    // ones only, and captured anew for others (a reallocated buffer, another
+    // launch shape).  Dropped at every re-layout, the six graphs of a new state cost its
+    // first steps 0.08 ms each.
+    struct PassGraph {
+        PassParams P;
+        int grids[5];
+        cudaGraphExec_t x;
+    };
     bool use_graphs = true;
-    std::map<int, cudaGraphExec_t> graphs;
+    std::map<int, PassGraph> graphs;
     void drop_graphs() {
-        for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
+        for (auto &kv : graphs) cudaGraphExecDestroy(kv.second.x);
         graphs.clear();
     }
 
@@ -196,6 +205,7 @@ bool is_fp64(const dsmc_ctx *ctx) { return ctx->precision == DSMC_PREC_FP64; }
 
 CellArrays cell_arrays(dsmc_ctx *ctx) {
     CellArrays c;
+    std::memset(&c, 0, sizeof(c));  // the padding too
     c.num_cells = ctx->num_cells;
     c.meta = ctx->meta.p;
     c.state = ctx->state.p;
@@ -211,6 +221,7 @@ CellArrays cell_arrays(dsmc_ctx *ctx) {
 
 ParticleArrays particle_arrays(dsmc_ctx *ctx) {
     ParticleArrays p;
+    std::memset(&p, 0, sizeof(p));
     for (int b = 0; b < 2; ++b) {
         p.A[b] = ctx->rec[b].p;
         p.B[b] = ctx->rec[b].p ? ctx->rec[b].p + ctx->rec_half() : nullptr;
@@ -260,7 +271,6 @@ void apply_launch_shape(dsmc_ctx *ctx) {
 }
 
 int relayout(dsmc_ctx *ctx, long long total) {
-    ctx->drop_graphs();  // slot buffers and grids may change
     const int C = ctx->num_cells;
     // Capacity per cell: twice the larger of the expected and the present
     // occupancy plus 24 slots by default (Poisson tails beyond it are below
@@ -391,7 +401,14 @@ int flush_pending(dsmc_ctx *ctx);
 cudaError_t launch_fused_graph(dsmc_ctx *ctx, const PassParams &P) {
     const int key = P.cur | (P.cin << 1) | (P.sorted_in << 3) | (P.do_collide << 4) | (P.do_sample << 5) |
                     (P.do_move << 6) | (P.any_cl << 7);
+    static_assert(sizeof(ctx->fused_grids) == sizeof(dsmc_ctx::PassGraph::grids), "five grids");
     auto it = ctx->graphs.find(key);
+    if (it != ctx->graphs.end() && (std::memcmp(&it->second.P, &P, sizeof(P)) != 0 ||
+                                    std::memcmp(it->second.grids, ctx->fused_grids, sizeof(it->second.grids)) != 0)) {
+        cudaGraphExecDestroy(it->second.x);
+        ctx->graphs.erase(it);
+        it = ctx->graphs.end();
+    }
     if (it == ctx->graphs.end()) {
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
@@ -402,17 +419,20 @@ cudaError_t launch_fused_graph(dsmc_ctx *ctx, const PassParams &P) {
             if (g) cudaGraphDestroy(g);
             return el != cudaSuccess ? el : e;
         }
-        cudaGraphExec_t x = nullptr;
-        e = cudaGraphInstantiate(&x, g, 0);
+        dsmc_ctx::PassGraph pg;
+        std::memcpy(&pg.P, &P, sizeof(P));
+        std::memcpy(pg.grids, ctx->fused_grids, sizeof(pg.grids));
+        e = cudaGraphInstantiate(&pg.x, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return e;
-        it = ctx->graphs.emplace(key, x).first;
+        it = ctx->graphs.emplace(key, pg).first;
     }
-    return cudaGraphLaunch(it->second, ctx->stream);
+    return cudaGraphLaunch(it->second.x, ctx->stream);
 }
 
 PassParams pass_params(dsmc_ctx *ctx, int do_collide, int do_move, int do_sample, int advance) {
     PassParams P;
+    std::memset(&P, 0, sizeof(P));  // compared bytewise (launch_fused_graph)
     P.sys = ctx->sys_dev.p;
     P.tally = ctx->tally.p;
     P.status = ctx->status.p;
@@ -972,6 +992,19 @@ int dsmc_system_info_get(dsmc_ctx *ctx, int sys_id, dsmc_system_info *info) {
     return DSMC_OK;
 }
 
+// The stream that state is copied on while ctx->stream converts.
+static cudaError_t io_stream_ready(dsmc_ctx *ctx) {
+    if (ctx->io_stream) return cudaSuccess;
+    cudaError_t e = cudaStreamCreateWithFlags(&ctx->io_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->io_event, cudaEventDisableTiming);
+    return e;
+}
+
+// Ranges of ids that a state of n particles is copied and converted in: none of
+// less than half a million, whose copies take 0.2 ms each way, and eight at most
+// (each download range reads every record again).
+static int io_pieces(long long n) { return (int)std::min(8ll, std::max(1ll, n >> 19)); }
+
 static int place_particles(dsmc_ctx *ctx, int sys_id, long long n, const double *r, const double *v) {
     cudaSetDevice(ctx->device);
     int rc = flush_pending(ctx);
@@ -989,13 +1022,33 @@ static int place_particles(dsmc_ctx *ctx, int sys_id, long long n, const double 
         CK(ctx->io_r.ensure(3 * std::max<long long>(n, 1)));
         CK(ctx->io_v.ensure(3 * std::max<long long>(n, 1)));
         if (n) {
-            CK(cudaMemcpyAsync(ctx->io_r.p, r, 3 * n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-            CK(cudaMemcpyAsync(ctx->io_v.p, v, 3 * n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-            e = is_fp64(ctx) ? fp64::launch_from_fp64(ctx->sys_dev.p, sys_id, ctx->io_r.p, ctx->io_v.p, 0, n, A, B, key,
-                                                      ctx->hist.p, &ctx->status.p->error, ctx->stream)
-                             : split32::launch_from_fp64(ctx->sys_dev.p, sys_id, ctx->io_r.p, ctx->io_v.p, 0, n, A, B,
-                                                         key, ctx->hist.p, &ctx->status.p->error, ctx->stream);
+            // by ranges: one is converted while the next is copied (the whole call at
+            // 3.9e6 particles 4.39 -> 4.2 ms, the copies alone 3.44)
+            CK(io_stream_ready(ctx));
+            CK(cudaEventRecord(ctx->io_event, ctx->stream));  // earlier work on io_r and io_v
+            CK(cudaStreamWaitEvent(ctx->io_stream, ctx->io_event, 0));
+            const int pieces = io_pieces(n);
+            e = cudaSuccess;
+            for (int k = 0; k < pieces && e == cudaSuccess; ++k) {
+                const long long lo = n * k / pieces, m = n * (k + 1) / pieces - lo;
+                double *dr = ctx->io_r.p + 3 * lo, *dv = ctx->io_v.p + 3 * lo;
+                e = cudaMemcpyAsync(dr, r + 3 * lo, 3 * m * sizeof(double), cudaMemcpyHostToDevice, ctx->io_stream);
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(dv, v + 3 * lo, 3 * m * sizeof(double), cudaMemcpyHostToDevice, ctx->io_stream);
+                if (e == cudaSuccess) e = cudaEventRecord(ctx->io_event, ctx->io_stream);
+                if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, ctx->io_event, 0);
+                if (e == cudaSuccess)
+                    e = is_fp64(ctx) ? fp64::launch_from_fp64(ctx->sys_dev.p, sys_id, dr, dv, (uint32_t)lo, m,
+                                                              A + lo * half, B + lo * half, key + lo, ctx->hist.p,
+                                                              &ctx->status.p->error, ctx->stream)
+                                     : split32::launch_from_fp64(ctx->sys_dev.p, sys_id, dr, dv, (uint32_t)lo, m,
+                                                                 A + lo * half, B + lo * half, key + lo, ctx->hist.p,
+                                                                 &ctx->status.p->error, ctx->stream);
+            }
+            // the copies are done with the caller's buffers before this returns
+            const cudaError_t e1 = cudaStreamSynchronize(ctx->io_stream);
             CK(e);
+            CK(e1);
         }
     } else if (n) {
         e = is_fp64(ctx) ? fp64::launch_init(ctx->sys_dev.p, sys_id, h.sqrt_t_over_m, n, A, B, key, ctx->hist.p,
@@ -1494,30 +1547,31 @@ int dsmc_particles_get(dsmc_ctx *ctx, int sys_id, int64_t cap, double *r, double
     CK(ctx->io_cell.ensure(std::max<long long>(N, 1)));
     if (N == 0) return DSMC_OK;
     if (h.slab) CK(cudaMemsetAsync(ctx->io_cell.p, 0xff, N * sizeof(int), ctx->stream));
-    if (!ctx->io_stream) {
-        CK(cudaStreamCreateWithFlags(&ctx->io_stream, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&ctx->io_event, cudaEventDisableTiming));
+    CK(io_stream_ready(ctx));
+    // Each record's values go to its id's place, a scatter, by ranges of ids: a
+    // range is copied out on io_stream while the next ones are converted
+    // (ms with positions and
+    // velocities as two halves -> by ranges: 3.9e6 particles 3.57 -> 3.45, 3.1e7 29.8
+    // -> 27.2; the copies alone 3.31 and 26.4).
+    cudaError_t e = cudaSuccess;
+    const int pieces = io_pieces(N);
+    for (int k = 0; k < pieces && e == cudaSuccess; ++k) {
+        const long long lo = N * k / pieces, hi = N * (k + 1) / pieces, m = hi - lo;
+        e = is_fp64(ctx) ? fp64::launch_to_fp64(ctx->sys_dev.p, sys_id, cell_arrays(ctx), particle_arrays(ctx), ctx->cur,
+                                                ctx->cphase, N, lo, hi, ctx->io_r.p, ctx->io_v.p, ctx->io_cell.p,
+                                                &ctx->status.p->error, ctx->stream)
+                         : split32::launch_to_fp64(ctx->sys_dev.p, sys_id, cell_arrays(ctx), particle_arrays(ctx),
+                                                   ctx->cur, ctx->cphase, N, lo, hi, ctx->io_r.p, ctx->io_v.p,
+                                                   ctx->io_cell.p, &ctx->status.p->error, ctx->stream);
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->io_event, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->io_stream, ctx->io_event, 0);
+        auto copy = [&](void *to, const void *from, size_t bytes) {
+            if (e == cudaSuccess) e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, ctx->io_stream);
+        };
+        copy(r + 3 * lo, ctx->io_r.p + 3 * lo, 3 * m * sizeof(double));
+        copy(v + 3 * lo, ctx->io_v.p + 3 * lo, 3 * m * sizeof(double));
+        if (cell) copy(cell + lo, ctx->io_cell.p + lo, m * sizeof(int32_t));
     }
-    // Each record's values go to its id's place, a scatter: the positions
-    // (and cells) first, copied out on io_stream while the velocities are
-    // converted, so that one conversion overlaps the other's copy.
-    auto to_fp64 = [&](double *ro, double *vo, int *co) {
-        return is_fp64(ctx) ? fp64::launch_to_fp64(ctx->sys_dev.p, sys_id, cell_arrays(ctx), particle_arrays(ctx),
-                                                   ctx->cur, ctx->cphase, 0, N, ro, vo, co, &ctx->status.p->error,
-                                                   ctx->stream)
-                            : split32::launch_to_fp64(ctx->sys_dev.p, sys_id, cell_arrays(ctx), particle_arrays(ctx),
-                                                      ctx->cur, ctx->cphase, 0, N, ro, vo, co, &ctx->status.p->error,
-                                                      ctx->stream);
-    };
-    CK(to_fp64(ctx->io_r.p, nullptr, ctx->io_cell.p));
-    CK(cudaEventRecord(ctx->io_event, ctx->stream));
-    CK(cudaStreamWaitEvent(ctx->io_stream, ctx->io_event, 0));
-    cudaError_t e = cudaMemcpyAsync(r, ctx->io_r.p, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, ctx->io_stream);
-    if (e == cudaSuccess && cell)
-        e = cudaMemcpyAsync(cell, ctx->io_cell.p, N * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->io_stream);
-    if (e == cudaSuccess) e = to_fp64(nullptr, ctx->io_v.p, nullptr);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(v, ctx->io_v.p, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
     // both streams are done with the caller's buffers before this returns
     const cudaError_t e1 = cudaStreamSynchronize(ctx->io_stream);
     const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
@@ -1827,33 +1881,25 @@ int dsmc_cells_get(dsmc_ctx *ctx, int sys_id, int cap, int32_t *global_index, in
     const int a0 = h.active_begin;
     if (global_index) std::memcpy(global_index, h.cell_global.data(), C * sizeof(int32_t));
     if (volume) std::memcpy(volume, h.volume_cell.data(), C * sizeof(double));
-    std::vector<unsigned> nb, nt;
-    if (count) {
-        nb.resize(C);
-        nt.resize(C);
-        CK(cudaMemcpyAsync(nb.data(), ctx->bot[ctx->cphase].p + a0, C * sizeof(unsigned), cudaMemcpyDeviceToHost,
-                           ctx->stream));
-        CK(cudaMemcpyAsync(nt.data(), ctx->top[ctx->cphase].p + a0, C * sizeof(unsigned), cudaMemcpyDeviceToHost,
-                           ctx->stream));
+    // the caller's arrays are laid out on the device: each is one copy, and no
+    // staging array of the host's has to be allocated, filled and walked (at
+    // 2.2e5 cells 8.3 -> 0.9 ms into arrays in use, 2.6 into new ones)
+    const size_t n = (size_t)C;
+    if (vr_max || rest || count) {
+        CK(ctx->cells_out.ensure(3 * n));
+        CK(launch_cells_out(ctx->meta.p, ctx->bot[ctx->cphase].p, ctx->top[ctx->cphase].p, ctx->state.p, a0, C,
+                            ctx->cells_out.p, ctx->stream));
     }
-    std::vector<double4> st(C);
-    std::vector<int4> mt(count ? C : 0);
-    if (count) CK(cudaMemcpyAsync(mt.data(), ctx->meta.p + a0, C * sizeof(int4), cudaMemcpyDeviceToHost, ctx->stream));
-    if (vr_max || rest)
-        CK(cudaMemcpyAsync(st.data(), ctx->state.p + a0, C * sizeof(double4), cudaMemcpyDeviceToHost, ctx->stream));
-    if (moments)
-        CK(cudaMemcpyAsync(moments, ctx->mom.p + 8 * (size_t)a0, 8 * (size_t)C * sizeof(double), cudaMemcpyDeviceToHost,
-                           ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    for (int q = 0; q < C; ++q) {
-        if (vr_max) vr_max[q] = st[q].x;
-        if (rest) rest[q] = st[q].y;
-        if (count) {
-            const unsigned cap = (unsigned)mt[q].y;
-            const unsigned b = std::min(nb[q], cap);
-            count[q] = (int32_t)(b + std::min(nt[q], cap - b));
-        }
-    }
+    auto copy = [&](void *to, const double *from, size_t bytes) {
+        return to ? cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, ctx->stream) : cudaSuccess;
+    };
+    cudaError_t e = copy(vr_max, ctx->cells_out.p, n * sizeof(double));
+    if (e == cudaSuccess) e = copy(rest, ctx->cells_out.p + n, n * sizeof(double));
+    if (e == cudaSuccess) e = copy(count, ctx->cells_out.p + 2 * n, n * sizeof(int32_t));
+    if (e == cudaSuccess) e = copy(moments, ctx->mom.p + 8 * (size_t)a0, 8 * n * sizeof(double));
+    const cudaError_t e1 = cudaStreamSynchronize(ctx->stream);
+    CK(e);
+    CK(e1);
     return DSMC_OK;
 }
 

@@ -101,7 +101,26 @@ __global__ void __launch_bounds__(LB) k_bases(int4 *meta, int C, const unsigned 
     if (a < C) meta[a].x = (int)(bsum[blockIdx.x] + incl - cap);  // the host refuses totals of 2^31 or more
 }
 
+// vr_max, rest and the particle count of cells [a0, a0 + C), each an array.
+__global__ void __launch_bounds__(256) k_cells_out(const int4 *meta, const unsigned *bot, const unsigned *top,
+                                                   const double4 *state, int a0, int C, double *out) {
+    const int q = blockIdx.x * 256 + threadIdx.x;
+    if (q >= C) return;
+    const int a = a0 + q;
+    const unsigned cap = (unsigned)meta[a].y, b = min(bot[a], cap);
+    const double4 st = state[a];
+    out[q] = st.x;
+    out[(size_t)C + q] = st.y;
+    reinterpret_cast<int *>(out + 2 * (size_t)C)[q] = (int)(b + min(top[a], cap - b));
+}
+
 }  // namespace
+
+cudaError_t launch_cells_out(const int4 *meta, const unsigned *bot, const unsigned *top, const double4 *state, int a0,
+                             int C, double *out, cudaStream_t st) {
+    k_cells_out<<<(C + 255) / 256, 256, 0, st>>>(meta, bot, top, state, a0, C, out);
+    return cudaGetLastError();
+}
 
 int cell_layout_blocks(int C) { return (C + LB - 1) / LB; }
 

@@ -32,8 +32,8 @@ namespace dsmc {
     cudaError_t launch_insert(const CellArrays &cells, const ParticleArrays &parts, int cur, int cin, long long n, \
                               const void *A, const void *B, const int *key, unsigned *err, cudaStream_t st);    \
     cudaError_t launch_to_fp64(const SysDev *sys, int s, const CellArrays &cells, const ParticleArrays &parts, \
-                               int cur, int cin, uint32_t id_base, long long cap, double *r, double *v, int *cell, \
-                               unsigned *err, cudaStream_t st);                                                 \
+                               int cur, int cin, long long cap, long long lo, long long hi, double *r, double *v, \
+                               int *cell, unsigned *err, cudaStream_t st);                                      \
     cudaError_t launch_cell_energy(const CellArrays &cells, const ParticleArrays &parts, int cur, int cin, int c0,  \
                                    int c1,                                                                      \
                                    double *out, cudaStream_t st);                                               \
@@ -75,6 +75,11 @@ cudaError_t launch_put(const SysDev *sys, int s, const CellArrays &cells, const 
 int cell_layout_blocks(int C);
 cudaError_t launch_cell_layout(int4 *meta, const int *pix, const unsigned *present, const double2 *np, double factor,
                                double pad, int C, unsigned long long *bsum, unsigned long long *out, cudaStream_t st);
+
+// What a caller reads of cells [a0, a0 + C), as consecutive arrays: vr_max[C],
+// rest[C], then the particle counts.
+cudaError_t launch_cells_out(const int4 *meta, const unsigned *bot, const unsigned *top, const double4 *state, int a0,
+                             int C, double *out, cudaStream_t st);
 
 // Pass modes (engine.cuh PassMode).
 enum { PASS_FUSED = 0, PASS_INPLACE = 1, PASS_SORT = 2 };

@@ -266,9 +266,11 @@ __global__ void k_insert(const CellArrays cells, const ParticleArrays parts, int
 }
 
 // Slots of one system -> fp64 state ordered by id (dsmc/dsmc_io.cpp:98-113
-// layout); r, v and cell may each be null (not written).
+// layout): the particles with ids in [lo, hi) of the cap there are; cell may be
+// null (not written).
 __global__ void k_to_fp64(const SysDev *sys, int s, const CellArrays cells, const ParticleArrays parts, int cur,
-                          int cin, uint32_t id_base, long long cap, double *r, double *v, int *cell, unsigned *err) {
+                          int cin, long long cap, long long lo, long long hi, double *r, double *v, int *cell,
+                          unsigned *err) {
     const SysDev &g = sys[s];
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -283,18 +285,16 @@ __global__ void k_to_fp64(const SysDev *sys, int s, const CellArrays cells, cons
             Particle p;
             const unsigned addr = cell_slot(m.x, m.y, nb, nt, q);
             Prec::unpack(Ain[rec_at(addr)], Bin[rec_at(addr)], p);
-            const long long i = (long long)p.id - (long long)id_base;
-            if (i < 0 || i >= cap) {
+            const long long i = (long long)p.id;
+            if (i >= cap) {
                 atomicOr(err, DSMC_EBIT_CELL);
                 continue;
             }
-            if (r) {
-                double rr[3];
-                Maker<Prec>::position(g, p, rr);
-                for (int d = 0; d < 3; ++d) r[3 * i + d] = rr[d];
-            }
-            if (v)
-                for (int d = 0; d < 3; ++d) v[3 * i + d] = (double)p.v[d];
+            if (i < lo || i >= hi) continue;
+            double rr[3];
+            Maker<Prec>::position(g, p, rr);
+            for (int d = 0; d < 3; ++d) r[3 * i + d] = rr[d];
+            for (int d = 0; d < 3; ++d) v[3 * i + d] = (double)p.v[d];
             if (cell) cell[i] = m.z;
         }
     }
@@ -430,9 +430,9 @@ cudaError_t launch_insert(const CellArrays &cells, const ParticleArrays &parts, 
 }
 
 cudaError_t launch_to_fp64(const SysDev *sys, int s, const CellArrays &cells, const ParticleArrays &parts, int cur,
-                           int cin, uint32_t id_base, long long cap, double *r, double *v, int *cell, unsigned *err,
-                           cudaStream_t st) {
-    k_to_fp64<<<148 * 8, 256, 0, st>>>(sys, s, cells, parts, cur, cin, id_base, cap, r, v, cell, err);
+                           int cin, long long cap, long long lo, long long hi, double *r, double *v, int *cell,
+                           unsigned *err, cudaStream_t st) {
+    k_to_fp64<<<148 * 8, 256, 0, st>>>(sys, s, cells, parts, cur, cin, cap, lo, hi, r, v, cell, err);
     return cudaGetLastError();
 }
 

@@ -226,3 +226,52 @@ def test_wall_flights_own_and_listed(cells, per_cell, dt_si, model):
     ta, tb = A.tallies(), B.tallies()
     assert ta.wall_collisions == tb.wall_collisions > 0 and ta.collisions == tb.collisions
     assert A.ctx.device_status()[0] & capi.EBIT_FATAL == 0
+
+
+@pytest.mark.parametrize("precision", [capi.PREC_SPLIT32, capi.PREC_FP64])
+@pytest.mark.parametrize("n", [1, 1000, (1 << 20) - 1, (1 << 20) + 3, 9 * (1 << 19) + 1])
+def test_state_in_and_out_by_ranges(n, precision):
+    """Uploads and downloads of one, two and eight ranges of ids, in an order that
+    is not the cells': velocities and cells come back exact, positions within
+    the rounding of a voxel's fp32 offset (two roundings of 2^-24), and every
+    particle is counted in its cell."""
+    w = Workload("io", n=64, radius_voxels=3.0, porosity=0.6, geometry_seed=2, cells=64,
+                 atoms_per_molecule=simulators_per_cell_weight(2.5e24, 0.1, 2, 20))
+    g = w.geometry()
+    s = w.settings(rng_seed=3, statistics_interval=10 ** 9)
+    base = System(s, g, precision=precision)
+    r0, v0, c0 = base.get_particles(with_cells=True)
+    pick = np.random.default_rng(n).integers(0, len(r0), n)
+    S = System(s, g, precision=precision, init_particles=False)
+    S.set_particles(r0[pick], v0[pick])
+    r, v, c = S.get_particles(with_cells=True)
+    assert np.abs(r - r0[pick]).max() <= 2.0 ** -22 * r0.max() / 64
+    assert np.array_equal(v, v0[pick]) and np.array_equal(c, c0[pick])
+    cells = S.cells()
+    want = np.bincount(c, minlength=64 ** 3)
+    assert np.array_equal(cells["count"], want[cells["global_index"]])
+
+
+def test_steps_after_new_states_of_other_sizes():
+    """A context's captured passes outlive a new state: the same steps follow
+    from the same state whether the context held as many particles before,
+    five times as many, or few (its buffers and launch shape then change)."""
+    w = Workload("again", n=32, radius_voxels=3.0, porosity=0.6, geometry_seed=5, cells=16,
+                 atoms_per_molecule=simulators_per_cell_weight(2.5e24, 0.1, 2, 40))
+    g = w.geometry()
+    s = w.settings(rng_seed=11, statistics_interval=10 ** 9)
+    base = System(s, g)
+    r, v = base.get_particles()
+    out = []
+    for k in (1, 5, 0):
+        S = System(s, g, init_particles=False)
+        first = (np.tile(r, (k, 1)), np.tile(v, (k, 1))) if k else (r[:100], v[:100])
+        S.set_particles(*first)
+        S.step(7)
+        S.set_particles(r, v)
+        c = S.cells()
+        S.set_cell_state(np.full(len(c["count"]), 3.0), np.zeros(len(c["count"])))
+        S.step(9)
+        out.append(S.get_particles())
+    for r1, v1 in out[1:]:
+        assert np.array_equal(r1, out[0][0]) and np.array_equal(v1, out[0][1])
