@@ -930,6 +930,16 @@ template <int CIB> cudaError_t launch_wgrad_plane(const WgradArgs &w, int ci0, i
     return cudaGetLastError();
 }
 
+// Additions per accumulator up to which the plane kernel takes a weight
+// gradient. The tensor core's fp32 sums truncate: one of n additions is off by about
+// 1.3e-8 n of its size, more or less by the order of the voxels. Up to here the
+// two kernels agree within 2e-5 (64^3 x 8: 6e-6 at 880 additions, 1.2e-5 at 1550,
+// 2.7e-5 at 3100, 4.1e-5 at 4650, each nearer to the exact sum than wgrad_kernel);
+// longer sums, of 48 output channels and more over a million voxels, keep
+// wgrad_kernel's order and bits, at its time (64^3 x 8, 32 -> 64 channels: 4070 us
+// against 391).
+constexpr long long kWgradPlaneAdds = 1800;
+
 cudaError_t launch_wgrad_planes(const WgradArgs &w, cudaStream_t st) {
     const int b32 = w.cin / 32;
     cudaError_t e = b32 ? launch_wgrad_plane<32>(w, 0, b32, st) : cudaSuccess;
@@ -1063,7 +1073,8 @@ int dsmc_sg_conv3_wgrad(void *stream, int batch, int S, const uint16_t *dy, int 
     a.rows = (long long)batch << (3 * lg);
     a.kv = 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (S >= kPlaneEdge && (cin == 16 || cin == 32 || cin == 48 || cin == 64 || cin == 96))
+    if (S >= kPlaneEdge && (cin == 16 || cin == 32 || cin == 48 || cin == 64 || cin == 96) &&
+        wgrad_voxels(a) / 16 <= kWgradPlaneAdds)
         return cuda_rc(launch_wgrad_planes(a, st));
     switch (cin) {
     case 16: return cuda_rc(launch_wgrad<16>(a, st));

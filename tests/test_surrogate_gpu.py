@@ -256,6 +256,26 @@ def test_loss_and_head_backward_rows(B, S):
     close_bf16(de, (dout @ wh.double()) * (ed > 0))
 
 
+@pytest.mark.parametrize("B,S,ci,co", [(24, 32, 16, 96), (25, 32, 16, 96), (8, 64, 16, 48), (5, 64, 32, 48)])
+def test_wgrad_at_the_longest_sums(B, S, ci, co):
+    """Weight gradients on both sides of the number of additions per
+    accumulator at which the gathering kernel takes over, against fp64 sums:
+    an accumulator of n additions that each truncate by half an ulp on average is off by at
+    most n 2^-24 of its size."""
+    g = torch.Generator(device=DEV).manual_seed(B)
+    x = torch.relu(torch.randn((B, S, S, S, ci), generator=g, device=DEV)).to(torch.bfloat16)
+    dy = torch.randn((B, S, S, S, co), generator=g, device=DEV).to(torch.bfloat16)
+    dw = torch.zeros((co, 27, ci), device=DEV)
+    capi.check(lib().dsmc_sg_conv3_wgrad(stream(), B, S, P(dy), co, 0, co, P(x), ci, 0, ci, P(dw)))
+    rows = B * S ** 3
+    adds = rows * ((27 * co + 127) // 128) / (148 * 4) / 16
+    dyd = dy.reshape(-1, co).double()
+    for t in (0, 4, 13, 22, 26):
+        d = (t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1)
+        ref = dyd.T @ torch.roll(x, (-d[0], -d[1], -d[2]), (1, 2, 3)).reshape(-1, ci).double()
+        assert ((dw[:, t].double() - ref).norm() / ref.norm()).item() <= adds * 2.0 ** -24, t
+
+
 def test_pool_and_upsample_forward_and_backward():
     g = torch.Generator().manual_seed(11)
     B, S, Cc = 2, 16, 32
