@@ -21,7 +21,11 @@
 // the measured cuBLAS rate, 42 us for its bytes), 64^3 16 -> 16 860 -> 64 us
 // (21 us for its bytes), 32^3 96 -> 32 653 -> 62 us, 16^3 64 -> 64 78 -> 19
 // us.  The one-tap-at-a-time gather was bound by its 27 reads of every voxel
-// from L2.
+// from L2.  Timed without its loads and its epilogue the 64^3 16 -> 16 kernel
+// still takes 57 of 64 us, without the MMAs 33: in the kernel an MMA of N = 48
+// takes about 60 cycles.  Two CTAs per SM (half the TMEM columns and epilogue warps
+// each) ran that forward in 58 us but its gradient in 79 for 74, 64^3 48 -> 16 in 135
+// for 127 and 32^3 32 -> 32 in 30 for 24.
 //
 // Per output value the taps and channels are accumulated in the order tap
 // 0..26, channels within a tap, as conv3_kernel (surrogate.cu) does: the two

@@ -17,8 +17,8 @@
 //   wgrad:    D[(tap,co)][ci] = sum_u dY[u - off(tap)][co] X[u][ci]
 // Edges of 16 and more (every layer of the network on boxes of 64 and more)
 // take conv_plane.cuh and wgrad_plane.cuh, which stage each voxel plane once;
-// the kernels here serve smaller edges and other channel counts: M tiles of
-// 128 rows, operands gathered tap by tap in shared memory by cp.async in a
+// the kernels here serve smaller edges, other channel counts and weight
+// gradients of very long sums: M tiles of 128 rows, operands gathered tap by tap in shared memory by cp.async in a
 // three-stage ring, one elected thread issuing the MMAs, completion tracked
 // by tcgen05.commit on an mbarrier per stage.  The epilogue (bias, ReLU, the
 // ReLU mask of a gradient, bf16 rounding) runs on the TMEM read-back.
