@@ -1,4 +1,4 @@
-// 3x3x3 periodic convolution for edges of 16 and more, on tcgen05.mma with
+// 3x3x3 periodic convolution for edges of 8 and more, on tcgen05.mma with
 // each input plane staged once per tile.
 //
 // A CTA walks tiles of 16 x 8 voxels (axes 1 and 2: the 128 rows of an MMA)
@@ -42,7 +42,7 @@ using bf16 = __nv_bfloat16;
 
 constexpr int kLines = 16, kRow = 8;             // voxels of a tile along axes 1 and 2
 constexpr int kHLines = kLines + 2, kHRow = kRow + 2;
-constexpr int kHalo = kHLines * kHRow;           // staged rows of a plane
+constexpr int kHalo = kHLines * kHRow;           // staged rows of a plane of a tile
 constexpr int kEpiWarps = 8, kLoadWarps = 4;     // two warps per TMEM lane quarter; then the loaders, then the issuer
 constexpr int kPlaneThreads = 32 * (kEpiWarps + kLoadWarps + 1);
 constexpr uint32_t kTmemCols = 512;
@@ -64,6 +64,12 @@ __device__ __forceinline__ PlaneItem plane_item(int item, int lg, int lgL) {
     return p;
 }
 
+// The same for pairs of samples (edge 8).
+__device__ __forceinline__ PlaneItem pair_item(int item, int lg, int lgL) {
+    const int nz = lg - lgL;
+    return PlaneItem{(item >> nz) << 1, 0, 0, (item & ((1 << nz) - 1)) << lgL};
+}
+
 // ---- forward (and input gradient) --------------------------------------------
 
 struct PlaneArgs {
@@ -80,9 +86,17 @@ struct PlaneArgs {
     int nb;             // output channels per CTA
     int nsplit;         // CTAs per item: cout / nb
     int items;          // tiles x plane segments
+    int batch;
 };
 
-template <int CIN> struct PlaneShape {
+// PAIR (edge 8): a tile is the whole planes of two samples, their lines
+// interleaved (the second sample's a line after the first's, so the groups of 8
+// rows stay one staged line apart and a tap along axis 1 is two lines). conv3_kernel
+// and this kernel, us, forward: 1 sample of 16 -> 16 channels 9.9 -> 5.7, 64 -> 64 38
+// -> 10; 16 of 96 -> 32 49 -> 14.5; 64 of 64 -> 64 77 -> 19.5, 96 -> 96 124 -> 37.
+template <int CIN, bool PAIR> struct PlaneShape {
+    static constexpr int kLineStep = PAIR ? 2 : 1;
+    static constexpr int kHalo = (kLines + 2 * kLineStep) * kHRow;  // staged rows of a plane
     static constexpr int kCpt = CIN / 8;                        // 16-byte channel chunks
     static constexpr int kChunk = kHalo * 16 + 16;              // bytes between chunks (odd in 16 bytes: no bank conflicts)
     static constexpr int kPlane = kCpt * kChunk;
@@ -90,7 +104,7 @@ template <int CIN> struct PlaneShape {
     // tensor pipe (nothing is queued behind an MMA that could start), as much
     // as two or three MMAs, so planes of few MMAs share one
     static constexpr int kGroup = CIN <= 32 ? 3 : CIN == 48 ? 2 : 1;
-    static constexpr int kGroups = CIN == 16 ? 4 : CIN <= 48 ? 3 : 4;
+    static constexpr int kGroups = CIN == 16 ? 4 : CIN <= 48 || (CIN == 96 && PAIR) ? 3 : 4;
     static constexpr int kStages = kGroup * kGroups;            // planes in flight
     static constexpr int kLoads = (kHalo * kCpt + 32 * kLoadWarps - 1) / (32 * kLoadWarps);
     static constexpr int kBars = 2 * kGroups + kMaxSlots + 2;
@@ -101,9 +115,10 @@ template <int CIN> struct PlaneShape {
 
 // Roles: warps 0-7 epilogue, 8-11 load planes, 12 issues the MMAs.  Every
 // wait is bounded (a wait that runs out sets bit 0 of the error flags).
-template <int CIN>
+template <int CIN, bool PAIR>
 __global__ void __launch_bounds__(kPlaneThreads, 1) conv_plane_kernel(const __grid_constant__ PlaneArgs a) {
-    using Sh = PlaneShape<CIN>;
+    using Sh = PlaneShape<CIN, PAIR>;
+    constexpr int kHalo = Sh::kHalo;
     extern __shared__ __align__(128) unsigned char smem[];
     const int nb = a.nb, nb3 = 3 * nb;
     unsigned char *Ws = smem + Sh::kStages * Sh::kPlane;
@@ -160,14 +175,17 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) conv_plane_kernel(const __gr
         bool lapped = false;  // every group has been filled once
         bool ok = true;
         for (int item = first; item < a.items; item += stride) {
-            const PlaneItem p = plane_item(item, lg, a.lgL);
+            const PlaneItem p = PAIR ? pair_item(item, lg, a.lgL) : plane_item(item, lg, a.lgL);
             int off[Sh::kLoads];
 #pragma unroll
             for (int i = 0; i < Sh::kLoads; ++i) {
                 const int idx = lt + 32 * kLoadWarps * i;
                 const int r = idx / Sh::kCpt, c = idx - r * Sh::kCpt;
                 const int line = r / kHRow, x = r - line * kHRow;
-                off[i] = (((((p.x1 - 1 + line) & msk) << lg) + ((p.x2 - 1 + x) & msk)) * a.in_cs) + a.in_coff + c * 8;
+                // (the last sample of an odd batch is its own pair)
+                const int second = PAIR && p.b + 1 < a.batch ? (line & 1) << lg3 : 0;
+                const int l1 = PAIR ? (line >> 1) - 1 : p.x1 - 1 + line;
+                off[i] = (second + ((l1 & msk) << lg) + ((p.x2 - 1 + x) & msk)) * a.in_cs + a.in_coff + c * 8;
             }
             for (int z = p.z0 - 1; z <= p.z0 + L; ++z) {
                 if (in_g == 0 && lapped) ok &= tc05::mbar_wait(&empty[s], ph ^ 1u);
@@ -239,14 +257,14 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) conv_plane_kernel(const __gr
                     for (int k = 0; k < 9 * (CIN / 16); ++k) {
                         const int t = k / (CIN / 16), c = k % (CIN / 16);
                         if (k >= k0)
-                            tc05::mma_bf16_warp(lead, d0, alo + (uint32_t)((t / 3) * kHRow + t % 3 + ((2 * c * Sh::kChunk) >> 4)),
+                            tc05::mma_bf16_warp(lead, d0, alo + (uint32_t)((t / 3) * Sh::kLineStep * kHRow + t % 3 + ((2 * c * Sh::kChunk) >> 4)),
                                                 ahi, blo + (uint32_t)((t * Sh::kCpt + 2 * c) * nb3), bhi, i0, 1u);
                     }
                 } else {
                     const uint32_t i1 = idesc(n1);
                     for (int k = k0; k < 9 * (CIN / 16); ++k) {
                         const int t = k / (CIN / 16), c = k % (CIN / 16);
-                        const uint32_t ad = alo + (uint32_t)((t / 3) * kHRow + t % 3 + ((2 * c * Sh::kChunk) >> 4));
+                        const uint32_t ad = alo + (uint32_t)((t / 3) * Sh::kLineStep * kHRow + t % 3 + ((2 * c * Sh::kChunk) >> 4));
                         const uint32_t bd = blo + (uint32_t)((t * Sh::kCpt + 2 * c) * nb3);
                         tc05::mma_bf16_warp(lead, d0, ad, ahi, bd, bhi, i0, 1u);
                         tc05::mma_bf16_warp(lead, tmem, ad, ahi, bd + (uint32_t)(n0 * nb), bhi, i1, 1u);
@@ -287,14 +305,15 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) conv_plane_kernel(const __gr
         uint32_t use = 0;
         bool ok = true;
         for (int item = first; item < a.items; item += stride) {
-            const PlaneItem p = plane_item(item, lg, a.lgL);
-            const long long row0 = ((long long)p.b << lg3) + ((long long)p.z0 << lg2) + ((long long)(p.x1 + line) << lg) +
-                                   p.x2 + x;
+            const PlaneItem p = PAIR ? pair_item(item, lg, a.lgL) : plane_item(item, lg, a.lgL);
+            const int b = PAIR ? p.b + (line & 1) : p.b, x1 = PAIR ? line >> 1 : p.x1 + line;
+            const bool here = !PAIR || b < a.batch;
+            const long long row0 = here ? ((long long)b << lg3) + ((long long)p.z0 << lg2) + ((long long)x1 << lg) + p.x2 + x : 0;
             for (int rel = 0; rel < L; ++rel, ++k) {
                 if ((k & 1) == (warp >> 2)) {
                     const long long row = row0 + ((long long)rel << lg2);
                     bf16 *dst = a.out + row * a.out_cs + a.out_coff + co0;
-                    const bf16 *mk = a.mask ? a.mask + row * a.mask_cs + a.mask_coff + co0 : nullptr;
+                    const bf16 *mk = a.mask ? a.mask + row * a.mask_cs + a.mask_coff + co0 : nullptr;  // (row 0's where not here)
                     uint4 mw[Sh::kMaxNb / 8];  // the mask's row, in flight during the wait
                     if (mk) {
 #pragma unroll
@@ -334,8 +353,10 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) conv_plane_kernel(const __gr
                             h0[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
                             h1[i] = __floats2bfloat162_rn(v[8 + 2 * i], v[8 + 2 * i + 1]);
                         }
-                        *reinterpret_cast<uint4 *>(dst + c0) = o0;
-                        *reinterpret_cast<uint4 *>(dst + c0 + 8) = o1;
+                        if (here) {
+                            *reinterpret_cast<uint4 *>(dst + c0) = o0;
+                            *reinterpret_cast<uint4 *>(dst + c0 + 8) = o1;
+                        }
                     }
                     tc05::fence_before_sync();
                     __syncwarp();

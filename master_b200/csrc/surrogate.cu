@@ -15,7 +15,8 @@
 //   dgrad:    the forward kernel on the flipped, transposed weights
 //             Wd[ci][tap][co] = W[co][26 - tap][ci]
 //   wgrad:    D[(tap,co)][ci] = sum_u dY[u - off(tap)][co] X[u][ci]
-// Edges of 16 and more (every layer of the network on boxes of 64 and more)
+// Edges of 16 and more (every layer of the network on boxes of 64 and more), and
+// of 8 for the forward kernel,
 // take conv_plane.cuh and wgrad_plane.cuh, which stage each voxel plane once;
 // the kernels here serve smaller edges, other channel counts and weight
 // gradients of very long sums: M tiles of 128 rows, operands gathered tap by tap in shared memory by cp.async in a
@@ -843,7 +844,7 @@ int sm_count() {
     return sms;
 }
 
-// The plane kernels' tiles are 16 x 8 voxels.
+// The plane kernels' tiles are 16 x 8 voxels (conv_plane_kernel: or the 8 x 8 of two samples).
 constexpr int kPlaneEdge = 16;
 
 // Output channels per CTA and planes per item of conv_plane_kernel: the split
@@ -851,17 +852,17 @@ constexpr int kPlaneEdge = 16;
 // largest of its MMAs (32 cycles to read A, or N / 2), its staged bytes and
 // its epilogue; an item stages two planes more than it writes; every CTA
 // loads its weights once.
-template <int CIN> void plane_split(PlaneArgs &a, int cout, long long rows, int sms) {
-    const long long tiles = rows >> (a.lg + 7);
+template <int CIN, bool PAIR> void plane_split(PlaneArgs &a, int cout, long long rows, int sms) {
+    const long long tiles = PAIR ? (a.batch + 1) / 2 : rows >> (a.lg + 7);
     double best = 1e300;
-    for (int nb = 16; nb <= PlaneShape<CIN>::kMaxNb; nb += 16) {
+    for (int nb = 16; nb <= PlaneShape<CIN, PAIR>::kMaxNb; nb += 16) {
         if (cout % nb) continue;
         const int nsplit = cout / nb;
         for (int lgL = 0; lgL <= a.lg; ++lgL) {
             const long long items = tiles << (a.lg - lgL);
             const long long ctas = std::max(1ll, std::min<long long>(items, sms / nsplit));
             const double mma = 9.0 * (CIN / 16) * std::max(32.0, 1.5 * nb);
-            const double plane = std::max(std::max(mma, kHalo * CIN * 2 / 25.0), 16.0 * nb);
+            const double plane = std::max(std::max(mma, PlaneShape<CIN, PAIR>::kHalo * CIN * 2 / 25.0), 16.0 * nb);
             const double t = (double)((items + ctas - 1) / ctas) * (((1 << lgL) + 2) * plane + 300.0) + 27.0 * CIN * nb * 2 / 40.0;
             if (t < best) {
                 best = t;
@@ -874,18 +875,18 @@ template <int CIN> void plane_split(PlaneArgs &a, int cout, long long rows, int 
     }
 }
 
-template <int CIN> cudaError_t launch_conv_plane(const ConvArgs &c, int cout, cudaStream_t st) {
-    using Sh = PlaneShape<CIN>;
+template <int CIN, bool PAIR> cudaError_t launch_conv_plane(const ConvArgs &c, int cout, cudaStream_t st) {
+    using Sh = PlaneShape<CIN, PAIR>;
     PlaneArgs a{c.in.p, c.in.cs, c.in.coff, c.w, c.bias, c.out.p, c.out.cs, c.out.coff, c.mask.p, c.mask.cs, c.mask.coff,
-                c.relu, c.S, c.lg, 0, 0, 0, 0};
+                c.relu, c.S, c.lg, 0, 0, 0, 0, (int)(c.rows >> (3 * c.lg))};
     const int sms = sm_count();
-    plane_split<CIN>(a, cout, c.rows, sms);
+    plane_split<CIN, PAIR>(a, cout, c.rows, sms);
     const int smem = Sh::smem(a.nb);
-    cudaError_t e = cudaFuncSetAttribute(conv_plane_kernel<CIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(conv_plane_kernel<CIN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Sh::smem(Sh::kMaxNb));
     if (e != cudaSuccess) return e;
     const int grid = (int)std::min<long long>(a.items, std::max(1, sms / a.nsplit)) * a.nsplit;
-    conv_plane_kernel<CIN><<<grid, kPlaneThreads, smem, st>>>(a);
+    conv_plane_kernel<CIN, PAIR><<<grid, kPlaneThreads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -1033,13 +1034,14 @@ int dsmc_sg_conv3(void *stream, int batch, int S, const uint16_t *in, int in_cs,
     a.lg = lg;
     a.rows = (long long)batch << (3 * lg);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (S >= kPlaneEdge && (cout == 16 || cout == 32 || cout == 48 || cout == 64 || cout == 96)) {
+    if (S >= kPlaneEdge / 2 && (cout == 16 || cout == 32 || cout == 48 || cout == 64 || cout == 96)) {
+        const bool pair = S < kPlaneEdge;
         switch (cin) {
-        case 16: return cuda_rc(launch_conv_plane<16>(a, cout, st));
-        case 32: return cuda_rc(launch_conv_plane<32>(a, cout, st));
-        case 48: return cuda_rc(launch_conv_plane<48>(a, cout, st));
-        case 64: return cuda_rc(launch_conv_plane<64>(a, cout, st));
-        case 96: return cuda_rc(launch_conv_plane<96>(a, cout, st));
+        case 16: return cuda_rc(pair ? launch_conv_plane<16, true>(a, cout, st) : launch_conv_plane<16, false>(a, cout, st));
+        case 32: return cuda_rc(pair ? launch_conv_plane<32, true>(a, cout, st) : launch_conv_plane<32, false>(a, cout, st));
+        case 48: return cuda_rc(pair ? launch_conv_plane<48, true>(a, cout, st) : launch_conv_plane<48, false>(a, cout, st));
+        case 64: return cuda_rc(pair ? launch_conv_plane<64, true>(a, cout, st) : launch_conv_plane<64, false>(a, cout, st));
+        case 96: return cuda_rc(pair ? launch_conv_plane<96, true>(a, cout, st) : launch_conv_plane<96, false>(a, cout, st));
         default: break;
         }
     }

@@ -173,8 +173,7 @@ def test_conv_edges_of_the_plane_kernels(B, S, cin, cout):
     """Forward, masked input gradient and weight gradient at the smallest edge
     of the plane kernels (16: one tile line block, every halo wraps), odd
     batches, several planes per tile, each accumulator ring (16, 32 and 48
-    channels per block) past its first lap, and the edge below (8: the
-    per-tap kernels).  bf16 results are held to the rounding of the output
+    channels per block) past its first lap, and the edge below (8).  bf16 results are held to the rounding of the output
     (2^-8) plus fp32 summation, as the module's other tests."""
     g = torch.Generator().manual_seed(1000 * S + cin + cout)
     x = rnd_bf16((B, S, S, S, cin), g)
@@ -206,6 +205,39 @@ def test_conv_edges_of_the_plane_kernels(B, S, cin, cout):
     close_bf16(y, torch.relu(ry).cpu())
     close_bf16(dx, (rdx * (xd > 0)).cpu())
     assert rel_l2(dw.cpu().numpy(), rdw.cpu().numpy()) <= 1e-4
+
+
+@pytest.mark.parametrize("B,cin,cout", [(1, 16, 16), (1, 96, 64), (2, 48, 48), (3, 64, 96), (5, 32, 32), (41, 96, 32)])
+def test_conv_of_pairs_of_samples(B, cin, cout):
+    """Edge 8, two samples per tile: even and odd batches, one and several
+    planes per item, reads and writes through views of wider tensors, and the
+    volume behind the last sample untouched.  bf16 results held to the
+    rounding of the output, as the module's other tests."""
+    S = 8
+    g = torch.Generator().manual_seed(100 * B + cin + cout)
+    xw = rnd_bf16((B, S, S, S, cin + 16), g)
+    x = xw[..., 8:8 + cin]
+    mask = rnd_bf16((B, S, S, S, cout), g)
+    w32 = torch.randn((cout, 27, cin), generator=g) * (2.0 / (27 * cin)) ** 0.5
+    bias = torch.randn(cout, generator=g) * 0.1
+    wf = torch.empty(cout * 27 * cin, dtype=torch.int16, device=DEV)
+    wd = torch.empty_like(wf)
+    d_w32, d_xw, d_m, d_b = w32.to(DEV), xw.to(DEV), mask.to(DEV), bias.to(DEV)
+    y = torch.full((B + 1, S, S, S, cout + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    ym = torch.full((B + 1, S, S, S, cout), 7.0, dtype=torch.bfloat16, device=DEV)
+    L = lib()
+    capi.check(L.dsmc_sg_pack_weights(stream(), P(d_w32), cout, cin, P(wf), P(wd)))
+    capi.check(L.dsmc_sg_conv3(stream(), B, S, P(d_xw), cin + 16, 8, cin, P(wf), P(d_b), cout, P(y), cout + 8, 8, 1, None, 0, 0))
+    capi.check(L.dsmc_sg_conv3(stream(), B, S, P(d_xw), cin + 16, 8, cin, P(wf), None, cout, P(ym), cout, 0, 0, P(d_m), cout, 0))
+    sync_ok()
+    xd, wb = x.to(DEV).double(), d_w32.to(torch.bfloat16).double()
+    ref = torch.zeros((B, S, S, S, cout), dtype=torch.float64, device=DEV)
+    for t in range(27):
+        off = (t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1)
+        ref += torch.roll(xd, tuple(-o for o in off), (1, 2, 3)) @ wb[:, t].T
+    close_bf16(y[:B, ..., 8:], torch.relu(ref + d_b.double()).cpu())
+    close_bf16(ym[:B], (ref * (d_m > 0)).cpu())
+    assert (y[B] == 7.0).all() and (y[..., :8] == 7.0).all() and (ym[B] == 7.0).all()
 
 
 @pytest.mark.parametrize("B,S,c,cs,off", [(1, 4, 16, 16, 0), (3, 8, 48, 64, 16), (2, 16, 128, 128, 0), (1, 16, 8, 24, 8),
