@@ -15,8 +15,7 @@
 //   dgrad:    the forward kernel on the flipped, transposed weights
 //             Wd[ci][tap][co] = W[co][26 - tap][ci]
 //   wgrad:    D[(tap,co)][ci] = sum_u dY[u - off(tap)][co] X[u][ci]
-// Edges of 16 and more (every layer of the network on boxes of 64 and more), and
-// of 8 for the forward kernel,
+// Edges of 8 and more (every layer of the network on boxes of 32 and more)
 // take conv_plane.cuh and wgrad_plane.cuh, which stage each voxel plane once;
 // the kernels here serve smaller edges, other channel counts and weight
 // gradients of very long sums: M tiles of 128 rows, operands gathered tap by tap in shared memory by cp.async in a
@@ -844,7 +843,7 @@ int sm_count() {
     return sms;
 }
 
-// The plane kernels' tiles are 16 x 8 voxels (conv_plane_kernel: or the 8 x 8 of two samples).
+// The plane kernels' tiles are 16 x 8 voxels (edge 8: the 8 x 8 of two samples).
 constexpr int kPlaneEdge = 16;
 
 // Output channels per CTA and planes per item of conv_plane_kernel: the split
@@ -901,10 +900,10 @@ long long wgrad_voxels(const WgradArgs &a) {
 }
 
 // One launch over the input channels [ci0, ci0 + ciblocks * CIB).
-template <int CIB> cudaError_t launch_wgrad_plane(const WgradArgs &w, int ci0, int ciblocks, cudaStream_t st) {
-    using Sh = PlaneWgradShape<CIB>;
+template <int CIB, bool PAIR> cudaError_t launch_wgrad_plane(const WgradArgs &w, int ci0, int ciblocks, cudaStream_t st) {
+    using Sh = PlaneWgradShape<CIB, PAIR>;
     PlaneWgradArgs a{w.dy.p, w.dy.cs, w.dy.coff, w.x.p, w.x.cs, w.x.coff, w.dw, w.cin, ci0, ciblocks,
-                     0, 0, w.S, w.lg, 0, 0, 1};
+                     0, 0, w.S, w.lg, 0, 0, 1, (int)(w.rows >> (3 * w.lg))};
     const int sms = sm_count();
     // an accumulator takes as many additions of 16 voxels as wgrad_kernel's
     // would: more would cost precision, fewer cost flushes
@@ -919,15 +918,15 @@ template <int CIB> cudaError_t launch_wgrad_plane(const WgradArgs &w, int ci0, i
     const int groups = ciblocks * a.coblocks;
     const int ctas = std::max(1, sms / groups);
     // planes per item: 16, fewer while items are short of two per CTA
-    const long long tiles = w.rows >> (w.lg + 7);
+    const long long tiles = PAIR ? (a.batch + 1) / 2 : w.rows >> (w.lg + 7);
     a.lgL = std::min(4, w.lg);
     while (a.lgL > 1 && (tiles << (w.lg - a.lgL)) < 2 * ctas) --a.lgL;
     a.items = (int)(tiles << (w.lg - a.lgL));
     a.flush = (int)std::max(1ll, adds / (8 << a.lgL));
-    cudaError_t e = cudaFuncSetAttribute(wgrad_plane_kernel<CIB>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::smem(48));
+    cudaError_t e = cudaFuncSetAttribute(wgrad_plane_kernel<CIB, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::smem(48));
     if (e != cudaSuccess) return e;
     const int grid = (int)std::min<long long>(a.items, ctas) * groups;
-    wgrad_plane_kernel<CIB><<<grid, kPlaneThreads, Sh::smem(a.cob), st>>>(a);
+    wgrad_plane_kernel<CIB, PAIR><<<grid, kPlaneThreads, Sh::smem(a.cob), st>>>(a);
     return cudaGetLastError();
 }
 
@@ -941,10 +940,10 @@ template <int CIB> cudaError_t launch_wgrad_plane(const WgradArgs &w, int ci0, i
 // against 391).
 constexpr long long kWgradPlaneAdds = 1800;
 
-cudaError_t launch_wgrad_planes(const WgradArgs &w, cudaStream_t st) {
+template <bool PAIR> cudaError_t launch_wgrad_planes(const WgradArgs &w, cudaStream_t st) {
     const int b32 = w.cin / 32;
-    cudaError_t e = b32 ? launch_wgrad_plane<32>(w, 0, b32, st) : cudaSuccess;
-    if (e == cudaSuccess && w.cin % 32) e = launch_wgrad_plane<16>(w, 32 * b32, 1, st);
+    cudaError_t e = b32 ? launch_wgrad_plane<32, PAIR>(w, 0, b32, st) : cudaSuccess;
+    if (e == cudaSuccess && w.cin % 32) e = launch_wgrad_plane<16, PAIR>(w, 32 * b32, 1, st);
     return e;
 }
 
@@ -1075,9 +1074,9 @@ int dsmc_sg_conv3_wgrad(void *stream, int batch, int S, const uint16_t *dy, int 
     a.rows = (long long)batch << (3 * lg);
     a.kv = 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (S >= kPlaneEdge && (cin == 16 || cin == 32 || cin == 48 || cin == 64 || cin == 96) &&
+    if (S >= kPlaneEdge / 2 && (cin == 16 || cin == 32 || cin == 48 || cin == 64 || cin == 96) &&
         wgrad_voxels(a) / 16 <= kWgradPlaneAdds)
-        return cuda_rc(launch_wgrad_planes(a, st));
+        return cuda_rc(S < kPlaneEdge ? launch_wgrad_planes<true>(a, st) : launch_wgrad_planes<false>(a, st));
     switch (cin) {
     case 16: return cuda_rc(launch_wgrad<16>(a, st));
     case 32: return cuda_rc(launch_wgrad<32>(a, st));

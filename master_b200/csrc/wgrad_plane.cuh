@@ -1,4 +1,4 @@
-// Weight gradient of the 3x3x3 periodic convolution for edges of 16 and more,
+// Weight gradient of the 3x3x3 periodic convolution for edges of 8 and more,
 // on tcgen05.mma with the planes of both operands staged once per tile: the
 // tiles, the staging and the roles of conv_plane.cuh.
 //
@@ -27,9 +27,16 @@ struct PlaneWgradArgs {
     int S, lg, lgL;
     int items;
     int flush;           // items between two flushes of the accumulators
+    int batch;
 };
 
-template <int CIB> struct PlaneWgradShape {
+// PAIR (edge 8): a tile is the whole planes of two samples, the second one's
+// lines behind the first's. wgrad_kernel and this kernel, us: 1 sample of 16 -> 16
+// channels 11.6 -> 6.2, 64 -> 64 17.9 -> 8.8; 16 of 96 -> 32 23 -> 9.7; 64 of 64 -> 64
+// 104 -> 20.5, 96 -> 96 123 -> 32.
+template <int CIB, bool PAIR> struct PlaneWgradShape {
+    static constexpr int kHLines = PAIR ? 20 : kLines + 2;
+    static constexpr int kHalo = kHLines * kHRow;
     static constexpr int kCpt = CIB / 8;
     static constexpr int kLine = kCpt * kHRow * 16;   // staged bytes of a line of X: [chunk][10 voxels]
     static constexpr int kX = kHLines * kLine;
@@ -49,9 +56,10 @@ template <int CIB> struct PlaneWgradShape {
 // 128 holds the 3 x CIB of them (the rest is not used); B's columns are three planes of dY (the
 // axis-0 taps) x cob; the axis-2 taps are three start addresses of A with an
 // accumulator each.  The accumulators are added to dW every `flush` items.
-template <int CIB>
+template <int CIB, bool PAIR>
 __global__ void __launch_bounds__(kPlaneThreads, 1) wgrad_plane_kernel(const __grid_constant__ PlaneWgradArgs a) {
-    using Sh = PlaneWgradShape<CIB>;
+    using Sh = PlaneWgradShape<CIB, PAIR>;
+    constexpr int kHalo = Sh::kHalo;
     extern __shared__ __align__(128) unsigned char smem[];
     const int cob = a.cob, cpy = cob >> 3;
     const int ystep = cpy * 128;              // bytes of one slot in a line of dY: [slot][chunk][8 voxels]
@@ -99,22 +107,31 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) wgrad_plane_kernel(const __g
         bool ok = true;
         const int ym = lt >> 3, yx = lt & 7;  // this thread's voxel of dY
         for (int item = first; item < a.items; item += stride) {
-            const PlaneItem p = plane_item(item, lg, a.lgL);
+            const PlaneItem p = PAIR ? pair_item(item, lg, a.lgL) : plane_item(item, lg, a.lgL);
+            // PAIR: an odd batch's last tile has one sample, its other lines are zero
+            const bool two = !PAIR || p.b + 1 < a.batch;
             int off[Sh::kXLoads];
 #pragma unroll
             for (int i = 0; i < Sh::kXLoads; ++i) {
                 const int idx = lt + 32 * kLoadWarps * i;
                 const int r = idx / Sh::kCpt, c = idx - r * Sh::kCpt;
                 const int line = r / kHRow, x = r - line * kHRow;
-                off[i] = (((((p.x1 - 1 + line) & msk) << lg) + ((p.x2 - 1 + x) & msk)) * a.x_cs) + a.x_coff + ci0 + c * 8;
+                const int second = PAIR && two && line >= 10 ? 1 << lg3 : 0;
+                const int l1 = PAIR && line >= 10 ? line - 10 : line;
+                off[i] = (second + (((p.x1 - 1 + l1) & msk) << lg) + ((p.x2 - 1 + x) & msk)) * a.x_cs + a.x_coff + ci0 + c * 8;
             }
-            const int yoff = (((p.x1 + ym) << lg) + p.x2 + yx) * a.dy_cs + a.dy_coff + co0;
+            const int yv = PAIR ? (two ? (ym >> 3) << lg3 : 0) + ((ym & 7) << lg) + yx : ((p.x1 + ym) << lg) + p.x2 + yx;
+            const int yoff = yv * a.dy_cs + a.dy_coff + co0;
+            const uint32_t ybytes = two || ym < 8 ? 16u : 0u;
             for (int u = 0; u < L + 2; ++u) {  // unit u: planes z0 - 1 + u of dY and, inside the item, of X
                 if (!(u & 1) && n >= Sh::kSlots) ok &= tc05::mbar_wait(&empty[s >> 1], ph ^ 1u);
                 const long long plane = ((long long)p.b << lg3) + ((long long)((p.z0 - 1 + u) & msk) << lg2);
                 const bf16 *py = a.dy + plane * a.dy_cs + yoff;
                 unsigned char *yd = Ys + ym * yline + s * ystep + yx * 16;
-                for (int c = 0; c < cpy; ++c) tc05::cp_async16(yd + c * 128, py + c * 8);
+                for (int c = 0; c < cpy; ++c) {
+                    if (PAIR) tc05::cp_async16_zfill(yd + c * 128, py + c * 8, ybytes);
+                    else tc05::cp_async16(yd + c * 128, py + c * 8);
+                }
                 if (u >= 1 && u <= L) {
                     const bf16 *px = a.x + plane * a.x_cs;
                     unsigned char *xd = smem + s * Sh::kX;
@@ -124,7 +141,9 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) wgrad_plane_kernel(const __g
                         if (idx < kHalo * Sh::kCpt) {
                             const int r = idx / Sh::kCpt, c = idx - r * Sh::kCpt;
                             const int line = r / kHRow, x = r - line * kHRow;
-                            tc05::cp_async16(xd + line * Sh::kLine + c * (kHRow * 16) + x * 16, px + off[i]);
+                            unsigned char *to = xd + line * Sh::kLine + c * (kHRow * 16) + x * 16;
+                            if (PAIR) tc05::cp_async16_zfill(to, px + off[i], two || line < 10 ? 16u : 0u);
+                            else tc05::cp_async16(to, px + off[i]);
                         }
                     }
                 }
@@ -176,7 +195,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) wgrad_plane_kernel(const __g
                         const uint32_t add = kk > 0 || !start ? 1u : 0u;
 #pragma unroll
                         for (int t2 = 0; t2 < 3; ++t2) {
-                            const uint32_t ad = alo + (uint32_t)((2 * kk * Sh::kLine) >> 4) + (uint32_t)t2;
+                            const uint32_t ad = alo + (uint32_t)(((2 * kk + (PAIR && kk >= 4 ? 2 : 0)) * Sh::kLine) >> 4) + (uint32_t)t2;
                             tc05::mma_bf16_warp(lead, col + t2 * 3 * cob, ad, ahi, blo + ys, bhi, i0, add);
                             if (n1 > 0)
                                 tc05::mma_bf16_warp(lead, col + (t2 * 3 + n0) * cob, ad, ahi, blo0 + ys, bhi, i1, add);

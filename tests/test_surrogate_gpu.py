@@ -240,6 +240,30 @@ def test_conv_of_pairs_of_samples(B, cin, cout):
     assert (y[B] == 7.0).all() and (y[..., :8] == 7.0).all() and (ym[B] == 7.0).all()
 
 
+@pytest.mark.parametrize("B,cin,cout", [(1, 16, 16), (2, 96, 64), (3, 48, 96), (5, 64, 48), (41, 32, 32), (8, 16, 160)])
+def test_wgrad_of_pairs_of_samples(B, cin, cout):
+    """Edge 8, two samples per tile: even and odd batches (what lies behind
+    the last sample is NaN), both blocks of input channels, each width of output
+    channels, through views.  Accumulators of at most 64 truncating additions
+    (64 x 2^-24) and at most 21 partial sums added in fp32: 1e-5."""
+    S = 8
+    g = torch.Generator().manual_seed(10 * B + cin + cout)
+    x = torch.full((B + 1, S, S, S, cin + 8), float("nan"), dtype=torch.bfloat16)
+    dy = torch.full((B + 1, S, S, S, cout + 16), float("nan"), dtype=torch.bfloat16)
+    x[:B] = rnd_bf16((B, S, S, S, cin + 8), g)
+    dy[:B] = rnd_bf16((B, S, S, S, cout + 16), g)
+    d_x, d_dy = x.to(DEV), dy.to(DEV)
+    dw = torch.zeros((cout, 27, cin), device=DEV)
+    capi.check(lib().dsmc_sg_conv3_wgrad(stream(), B, S, P(d_dy), cout + 16, 16, cout, P(d_x), cin + 8, 8, cin, P(dw)))
+    sync_ok()
+    xd, dyd = d_x[:B, ..., 8:].double(), d_dy[:B, ..., 16:].double().reshape(-1, cout)
+    ref = torch.zeros((cout, 27, cin), dtype=torch.float64, device=DEV)
+    for t in range(27):
+        off = (t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1)
+        ref[:, t] = dyd.T @ torch.roll(xd, tuple(-o for o in off), (1, 2, 3)).reshape(-1, cin)
+    assert ((dw.double() - ref).norm() / ref.norm()).item() <= 1e-5
+
+
 @pytest.mark.parametrize("B,S,c,cs,off", [(1, 4, 16, 16, 0), (3, 8, 48, 64, 16), (2, 16, 128, 128, 0), (1, 16, 8, 24, 8),
                                           (2, 8, 20, 24, 1), (1, 2, 128, 128, 0)])
 def test_bias_gradient_shapes(B, S, c, cs, off):
