@@ -231,7 +231,10 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) conv_plane_kernel(const __gr
             for (int zi = 0; zi < L + 2; ++zi) {
                 const int jb = zi < 2 ? 2 - zi : 0, je = zi < L ? 3 : L + 2 - zi;
                 const bool fresh = je == 3;  // the plane's newest block starts an accumulator
-                if (fresh && lapped && (slot == 0 || slot == H)) ok &= tc05::mbar_wait(&accfree[slot ? 1 : 0], use ^ 1u);
+                if (fresh && lapped && (slot == 0 || slot == H)) {
+                    ok &= tc05::mbar_wait(&accfree[slot ? 1 : 0], use ^ 1u);
+                    tc05::fence_after_sync();  // the epilogue's reads, before the MMAs that start these slots again
+                }
                 if (in_g == 0) {
                     ok &= tc05::mbar_wait(&full[s], ph);
                     tc05::fence_proxy_async_smem();  // the loaders' copies, for the MMAs' reads
