@@ -1502,14 +1502,16 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
         const bool collide = P.do_collide && MODE != MODE_SORT;
         bool sample = P.do_sample && MODE != MODE_SORT && g.sample_interval > 0 && step > 0 &&
                       (step % (uint32_t)g.sample_interval) == 0 && step >= (uint32_t)g.sample_begin;
-        // Cell::prepare, on every lane; the candidate pairs run below
+        // Cell::prepare, on the lane that runs the candidate pairs below and
+        // writes the cell's state back: no other lane touches it
         double4 cs = make_double4(0, 0, 0, 0);
         int pairs = 0;
-        if (collide) {
+        if (collide && lane == 0) {
             cs = P.cells.state[a];
             pairs = ntc_select(cs.z, n, cs.x, cs.y);
             if (n < 2) pairs = 0;
         }
+        pairs = __shfl_sync(0xffffffffu, pairs, 0);
         const bool staged = pairs > 0 || sample;  // members needed in id order
 
         // Stage velocities (and ids) in shared memory.

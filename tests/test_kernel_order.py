@@ -39,3 +39,20 @@ def test_tensor_memory_is_touched_only_after_a_fence_behind_the_wait(name, waits
                 pytest.fail(f"{name}: {t.group()} after the wait on {m.group(1)} without a fence between")
         else:
             pytest.fail(f"{name}: no fence after the wait on {m.group(1)}")
+
+
+def test_one_lane_reads_and_writes_a_cells_state():
+    """The generic cell pass: a cell's collision state is read, selected on and
+    written by one lane, and the warp learns the pair count from it. (Read
+    by every lane, the state could be written before a late lane had read it.)"""
+    text = source("engine.cuh")
+    body = text[text.index("pass_kernel(PassParams P)"):text.index("pass_walls_kernel(PassParams P)")]
+    uses = [m.start() for m in re.finditer(r"P\.cells\.state\[a\]", body)]
+    assert len(uses) == 2
+    for at in uses:
+        opened, depth = at, 0  # the innermost block that is open here
+        while depth <= 0:
+            opened -= 1
+            depth += {"{": 1, "}": -1}.get(body[opened], 0)
+        assert re.search(r"if \(collide && lane == 0\) $", body[:opened]), body[opened - 60:at]
+    assert re.search(r"pairs = __shfl_sync\(0xffffffffu, pairs, 0\)", body[uses[0]:uses[1]])
