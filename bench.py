@@ -413,7 +413,7 @@ def main():
 
     import ctypes as C
     import torch
-    from master_b200 import autotune, capi, workloads
+    from master_b200 import capi, workloads
     from master_b200.system import System
 
     torch.cuda.set_device(local)
@@ -434,6 +434,7 @@ def main():
     # untimed timesteps of this workload; the cache is applied when present)
     tuning = None
     if not args.no_tune and system.ctx.pass_info()["pipelined"] == 1:
+        from master_b200 import autotune
         cached = autotune.apply_cached(system.ctx)
         if cached is not None:
             tuning = {"source": "cache", "choice": cached["choice"]}
@@ -469,10 +470,7 @@ def main():
     # ---- per-kernel durations (CUDA events around each kernel of each pass,
     # recorded by the library on its stream), after the timed region -------
     pipelined = system.ctx.pass_info()["pipelined"] == 1
-    tuned, most = autotune.get(system.ctx)
-    place_blocks = tuned.blocks_per_sm[2] or most.blocks_per_sm[2]
-    place_warps = 4 * max(1, place_blocks * torch.cuda.get_device_properties(local).multi_processor_count // 2)
-    own_walls = settings.surface_model != 2 and system.info().num_active_cells <= 4 * 32 * place_warps
+    launches_step, launches_sample = system.ctx.pass_launches()
     kernels = None
     if pipelined:
         k_t = max(3, min(args.steps, 20))
@@ -586,14 +584,11 @@ def main():
                      "h2d_bytes_per_step": 48 * N / k_long, "d2h_bytes_per_step": (48 * N + 64 * k_long) / k_long},
         "cadence": cadence,
         "tuning": tuning,
-        # collide_cells + move_cells + place_movers (+ place_walls, unless
-        # place_movers' warps move their own wall flights: thermal or specular
-        # walls and at most four chunks of 32 cells per warp) per step
-        # (production pass) and sample_cells on the sampled steps the timed
-        # passes collide; one pass kernel per step otherwise
-        "gpu_launches": args.steps * ((3 if own_walls else 4) if pipelined else 1) + (sum(
-            1 for st in range(step_before, step_after)
-            if st > 0 and st % settings.statistics_interval == 0) if pipelined else 0),
+        # as the library reports them (production pass: collide_cells,
+        # move_cells, place_movers and, for listed wall flights, place_walls per
+        # step, sample_cells on the sampled steps the timed passes collide)
+        "gpu_launches": args.steps * launches_step + launches_sample * sum(
+            1 for st in range(step_before, step_after) if st > 0 and st % settings.statistics_interval == 0),
         "clocks": clocks,
         "device_status": {"error_bits": err, "spill": spill},
         "pass": system.ctx.pass_info(),

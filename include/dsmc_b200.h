@@ -408,6 +408,13 @@ int dsmc_ctx_set_capacity(dsmc_ctx *ctx, double factor, int pad);
  * block of move_cells, and the particles of a group that its warps stage. */
 int dsmc_pass_info(dsmc_ctx *ctx, int *pipelined, int *grid, int *block, int *stage_capacity);
 
+/* Kernels that dsmc_step launches for one timestep with the present layout
+ * and tuning, and further ones on a step whose collide samples. (Three or
+ * four per step in the production pass: with few cells and no
+ * Cercignani-Lampis walls place_movers moves the wall flights itself and
+ * place_walls does not run.) */
+int dsmc_pass_launches(dsmc_ctx *ctx, int *per_step, int *per_sample);
+
 /* Launch tuning of the production pass, for the autotuner
  * (master_b200/autotune.py): the reference has no counterpart (its stages are
  * loops over particles on one core).  blocks_per_sm: resident blocks per SM of

@@ -41,7 +41,7 @@ EXPORTED = [
     "dsmc_particles_count", "dsmc_particles_get", "dsmc_step", "dsmc_stage_move", "dsmc_stage_sort",
     "dsmc_stage_collide", "dsmc_stage_sample", "dsmc_tallies_get", "dsmc_tallies_reset", "dsmc_cells_get",
     "dsmc_cells_set_state", "dsmc_device_status", "dsmc_stream", "dsmc_counters_get", "dsmc_cells_layout",
-    "dsmc_ctx_set_capacity", "dsmc_pass_info", "dsmc_geometry_finish_gpu_noalloc", "dsmc_ctx_set_timing",
+    "dsmc_ctx_set_capacity", "dsmc_pass_info", "dsmc_pass_launches", "dsmc_geometry_finish_gpu_noalloc", "dsmc_ctx_set_timing",
     "dsmc_pass_times_get", "dsmc_state_file_read", "dsmc_state_file_write", "dsmc_tocontinue_read",
     "dsmc_tocontinue_write", "dsmc_continue_from", "dsmc_checkpoint_save", "dsmc_checkpoint_load",
     "dsmc_profile_sums_get", "dsmc_profiles_finish", "dsmc_profiles_get", "dsmc_measures_get",
@@ -173,6 +173,7 @@ def load() -> C.CDLL:
         "dsmc_stream": [_P],
         "dsmc_counters_get": [_P, C.c_int, C.POINTER(C.c_int64)],
         "dsmc_ctx_set_capacity": [_P, C.c_double, C.c_int],
+        "dsmc_pass_launches": [_P, C.POINTER(C.c_int), C.POINTER(C.c_int)],
         "dsmc_pass_info": [_P, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)],
         "dsmc_ctx_set_timing": [_P, C.c_int],
         "dsmc_pass_times_get": [_P, _D, C.POINTER(C.c_int64)],

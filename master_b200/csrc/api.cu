@@ -430,6 +430,12 @@ cudaError_t launch_fused_graph(dsmc_ctx *ctx, const PassParams &P) {
     return cudaGraphLaunch(it->second.x, ctx->stream);
 }
 
+int any_cl(const dsmc_ctx *ctx) {
+    for (const auto &s : ctx->systems)
+        if (s->dev.wall_model == DSMC_WALL_CL) return 1;
+    return 0;
+}
+
 PassParams pass_params(dsmc_ctx *ctx, int do_collide, int do_move, int do_sample, int advance) {
     PassParams P;
     std::memset(&P, 0, sizeof(P));  // compared bytewise (launch_fused_graph)
@@ -450,8 +456,7 @@ PassParams pass_params(dsmc_ctx *ctx, int do_collide, int do_move, int do_sample
     P.advance_step = advance;
     P.ring = ctx->tune_ring;
     P.claim = ctx->tune_claim;
-    P.any_cl = 0;
-    for (const auto &s : ctx->systems) P.any_cl |= s->dev.wall_model == DSMC_WALL_CL ? 1 : 0;
+    P.any_cl = any_cl(ctx);
     return P;
 }
 
@@ -1955,6 +1960,16 @@ int dsmc_pass_info(dsmc_ctx *ctx, int *pipelined, int *grid, int *block, int *st
     if (grid) *grid = pipe ? ctx->fused_grids[1] : ctx->grid;
     if (block) *block = pipe ? split32::fused_block() : ctx->block;
     if (stage_capacity) *stage_capacity = pipe ? split32::fused_capacity(ctx->smem_cap) : ctx->smem_cap;
+    return DSMC_OK;
+}
+
+int dsmc_pass_launches(dsmc_ctx *ctx, int *per_step, int *per_sample) {
+    if (!ctx) return DSMC_ERR_ARG;
+    const bool pipe = ctx->use_pipelined && ctx->fused_grids[1] > 0;
+    // collide_cells, move_cells, place_movers and, for listed flights,
+    // place_walls; sample_cells.  The generic pass: its cells, then its wall flights
+    if (per_step) *per_step = !pipe ? 2 : split32::own_walls(ctx->num_cells, any_cl(ctx), ctx->fused_grids) ? 3 : 4;
+    if (per_sample) *per_sample = pipe ? 1 : 0;
     return DSMC_OK;
 }
 

@@ -55,6 +55,9 @@ int fused_block();                  // threads per block of the production kerne
 // and sample_cells; 0 when one of them cannot be resident.
 // ring: as ring_for.  max_bps (may be null): the most blocks per SM of each.
 int fused_grids(int smem_cap, int num_sms, int grids[5], int ring = 0, int max_bps[5] = nullptr);
+// Whether place_movers' warps move their own wall flights with these grids
+// (place_walls then does not run).  any_cl: as PassParams.
+bool own_walls(int num_cells, int any_cl, const int grids[5]);
 // ev: null, or five events recorded before each kernel and after the last
 // (the sampler, on sampled steps, falls in the collide interval)
 cudaError_t launch_fused(const PassParams &P, const int grids[5], cudaStream_t st, cudaEvent_t *ev = nullptr);

@@ -128,6 +128,15 @@ static void launch_collide_cells(const PassParams &P0, int grid, cudaStream_t st
         pass3::collide_cells_kernel<false><<<grid, 32 * pass3::C_WARPS, 0, st>>>(P);
 }
 
+// place_movers' blocks when its warps move their own wall flights: half the
+// blocks of the listing kernel fit
+static int own_walls_grid(const int grids[5]) { return std::max(1, grids[2] / 2); }
+
+// They do up to four chunks of 32 cells per warp (place_movers_kernel's comment).
+bool own_walls(int num_cells, int any_cl, const int grids[5]) {
+    return !any_cl && num_cells <= 4ll * 32 * own_walls_grid(grids) * pass3::P_WARPS;
+}
+
 cudaError_t launch_fused(const PassParams &P, const int grids[5], cudaStream_t st, cudaEvent_t *ev) {
     if (ev) cudaEventRecord(ev[0], st);
     if (P.do_collide || P.do_sample) {
@@ -151,12 +160,10 @@ cudaError_t launch_fused(const PassParams &P, const int grids[5], cudaStream_t s
     }
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[2], st);
-    // each warp its own wall flights, up to four chunks of cells per warp (its
-    // comment); half the blocks of the listing kernel fit
-    const int own_grid = std::max(1, grids[2] / 2);
-    const long long own_warps = (long long)own_grid * pass3::P_WARPS;
-    if (!P.any_cl && P.cells.num_cells <= 4 * 32 * own_warps) {
-        pass3::place_movers_kernel<true><<<own_grid, 32 * pass3::P_WARPS, 0, st>>>(with_chunk(P, own_warps));
+    if (own_walls(P.cells.num_cells, P.any_cl, grids)) {
+        const int own_grid = own_walls_grid(grids);
+        pass3::place_movers_kernel<true><<<own_grid, 32 * pass3::P_WARPS, 0, st>>>(
+            with_chunk(P, (long long)own_grid * pass3::P_WARPS));
         e = cudaGetLastError();
         if (ev) cudaEventRecord(ev[3], st);
     } else {

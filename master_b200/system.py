@@ -297,6 +297,12 @@ class Context:
         self.check(self.lib.dsmc_pass_info(self.handle, *(C.byref(v) for v in vals)))
         return dict(zip(("pipelined", "grid", "block", "stage_capacity"), (v.value for v in vals)))
 
+    def pass_launches(self) -> tuple[int, int]:
+        """Kernels launched per timestep, and further ones on a sampled step."""
+        step, sample = C.c_int(), C.c_int()
+        self.check(self.lib.dsmc_pass_launches(self.handle, C.byref(step), C.byref(sample)))
+        return step.value, sample.value
+
     def checkpoint_save(self, path) -> None:
         """Exact checkpoint of every system of the context."""
         self.check(self.lib.dsmc_checkpoint_save(self.handle, str(path).encode()))

@@ -43,6 +43,21 @@ def test_any_launch_shape_gives_the_same_trajectory(bps, ring, claim):
     assert B.ctx.device_status()[0] & capi.EBIT_FATAL == 0
 
 
+def test_launches_follow_the_grid_of_place_movers():
+    """1.6e5 active cells: place_movers' warps move their own wall flights
+    (three kernels a step) unless its grid is too small for that; walls of the
+    Cercignani-Lampis model always have a kernel of their own."""
+    w = workloads.Workload("own", n=64, radius_voxels=3.0, porosity=0.6, geometry_seed=5, cells=64,
+                           atoms_per_molecule=workloads.simulators_per_cell_weight(2.5e24, 0.1, 1, 3))
+    s = w.settings()
+    S = System(s, w.geometry())
+    assert S.ctx.pass_launches() == (3, 1)
+    autotune.set_tuning(S.ctx, (0, 0, 1, 0, 0))
+    assert S.ctx.pass_launches() == (4, 1)
+    s.surface_model = 2
+    assert System(s, w.geometry()).ctx.pass_launches() == (4, 1)
+
+
 def test_tuning_arguments_are_checked():
     A, _ = pair()
     with pytest.raises(capi.DsmcError):
