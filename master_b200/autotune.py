@@ -1,12 +1,15 @@
 """Autotuner of the production pass's launch shape, with a JSON cache.
 
-The production pass is four persistent kernels per step (collide_cells,
+The production pass is three or four persistent kernels per step (collide_cells,
 move_cells, place_movers, place_walls; sample_cells on sampled steps), each a
 grid of resident blocks.  Their shapes are searched on the workload itself:
 
 * blocks per SM of each kernel, from one up to the most that are resident;
   the kernels run one after another, so each is timed alone by the library's
-  per-kernel CUDA events (dsmc_ctx_set_timing) while the others keep theirs;
+  per-kernel CUDA events (dsmc_ctx_set_timing) while the others keep theirs,
+  but place_movers with place_walls: the number of its blocks also decides
+  whether it moves the wall flights itself or hands them on, and place_walls'
+  blocks are then searched behind the chosen place_movers, if it runs at all;
 * move_cells' staging ring: the smallest that holds the largest cell, and
   the next larger rings (more staging per warp, fewer resident blocks);
 * collide_cells' chunk claims: a fixed stride or a pass-wide counter.
@@ -34,7 +37,7 @@ from pathlib import Path
 from . import capi
 
 KERNELS = ("collide_cells", "move_cells", "place_movers", "place_walls")
-RINGS = (64, 96, 128, 160, 192, 224, 256, 320, 384, 448, 512)
+RINGS = (128, 160, 192, 224, 256, 320, 384, 448, 512)
 
 
 def cache_path() -> Path:
@@ -175,16 +178,20 @@ def tune(ctx, steps: int = 10, repeats: int = 3, extra_rings: int = 2, store: bo
             if t["collide_cells"] < best_col[0]:
                 best_col = (t["collide_cells"], b, claim)
     best["bps"][0], best["claim"] = best_col[1], best_col[2]
-    # place_movers and place_walls
-    for k, name in ((2, "place_movers"), (3, "place_walls")):
-        bk = (default[name], 0)
-        for b in range(1, max_bps[k] + 1):
-            bps = [0] * 5
-            bps[k] = b
-            t = run(bps, 0, 0, f"{name} bps {b}")
-            if t[name] < bk[0]:
-                bk = (t[name], b)
-        best["bps"][k] = bk[1]
+    # place_movers, with the flights it hands on
+    best_place, flights = (default["place_movers"] + default["place_walls"], 0), default["place_walls"]
+    for b in range(1, max_bps[2] + 1):
+        t = run([0, 0, b, 0, 0], 0, 0, f"place_movers bps {b}")
+        if t["place_movers"] + t["place_walls"] < best_place[0]:
+            best_place, flights = (t["place_movers"] + t["place_walls"], b), t["place_walls"]
+    best["bps"][2] = best_place[1]
+    # place_walls behind it
+    set_tuning(ctx, [0, 0, best["bps"][2], 0, 0])
+    if ctx.pass_launches()[0] == 4:
+        for b in range(1, max_bps[3] + 1):
+            t = run([0, 0, best["bps"][2], b, 0], 0, 0, f"place_walls bps {b}")
+            if t["place_walls"] < flights:
+                best["bps"][3], flights = b, t["place_walls"]
     # the combination, against the default on the whole step
     chosen = run(best["bps"], best["ring"], best["claim"], "chosen")
     set_tuning(ctx)
