@@ -412,7 +412,7 @@ int dsmc_pass_info(dsmc_ctx *ctx, int *pipelined, int *grid, int *block, int *st
  * and tuning, and further ones on a step whose collide samples. (Three or
  * four per step in the production pass: with few cells and no
  * Cercignani-Lampis walls place_movers moves the wall flights itself and
- * place_walls does not run.) */
+ * place_walls does not run. One or two in the generic pass, likewise.) */
 int dsmc_pass_launches(dsmc_ctx *ctx, int *per_step, int *per_sample);
 
 /* Launch tuning of the production pass, for the autotuner

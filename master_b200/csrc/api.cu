@@ -143,6 +143,8 @@ struct dsmc_ctx {
     // launch shape of the cell pass
     int block = 256;
     int grid = 0;
+    int walls_grid = 0;          // of the wall flights that the cell pass lists
+    bool own_flights = false;    // the cell pass moves them itself instead
     int fused_grids[5] = {0, 0, 0, 0, 0};  // production pass (collide, move, place, walls, sample); 0 = not usable
     int fused_max_bps[5] = {0, 0, 0, 0, 0};  // the most resident blocks per SM of each at the current ring
     // launch tuning (dsmc_tuning_set): blocks per SM of each production
@@ -270,6 +272,24 @@ void apply_launch_shape(dsmc_ctx *ctx) {
             ctx->fused_grids[k] = std::min(ctx->tune_bps[k], ctx->fused_max_bps[k]) * ctx->num_sms;
 }
 
+// Whether the cell pass moves its wall flights where it finds them, which
+// saves a launch and the list's turn-around but has a warp's flights follow one
+// another: while each warp makes few turns (32 members of a cell; a quarter
+// above the mean, where cells of more than 32 are many), fewer with walls that
+// leave flights longer.  us per step in fp64, own / listed: thermal walls
+// 336 cells (4.4e3 particles) 23 / 34, 2944 36 / 47, 5920 49 / 55, 10256 (five
+// turns) 64 / 65 and with twice the particles (ten) 91 / 82, 16152 85 / 76, 24128 111 / 92; Cercignani-Lampis 336 136 / 147,
+// 4336 (two turns) 253 / 260, 10256 307 / 291; specular 1176 69 / 86, 1960 (one turn) 88 / 91,
+// 2944 130 / 99, 10256 267 / 123.
+bool pass_owns_flights(const dsmc_ctx *ctx, long long total) {
+    const long long warps = (long long)ctx->grid * (ctx->block / 32), C = std::max(ctx->num_cells, 1);
+    const long long turns = ((C + warps - 1) / warps) * ((total + total / 4 + 32 * C - 1) / (32 * C));
+    int most = 5;
+    for (const auto &s : ctx->systems)
+        most = std::min(most, s->dev.wall_model == DSMC_WALL_SPECULAR ? 1 : s->dev.wall_model == DSMC_WALL_CL ? 2 : 5);
+    return turns <= most;
+}
+
 int relayout(dsmc_ctx *ctx, long long total) {
     const int C = ctx->num_cells;
     // Capacity per cell: twice the larger of the expected and the present
@@ -323,13 +343,19 @@ int relayout(dsmc_ctx *ctx, long long total) {
     // Launch shape of the cell pass: a persistent grid at full occupancy.
     const int bps = is_fp64(ctx) ? fp64::pass_blocks_per_sm(PASS_FUSED, ctx->block, ctx->smem_cap)
                                  : split32::pass_blocks_per_sm(PASS_FUSED, ctx->block, ctx->smem_cap);
-    if (bps <= 0) return fail(ctx, DSMC_ERR_CUDA, "cell pass cannot be resident (shared memory)");
+    const int bps_own = is_fp64(ctx) ? fp64::pass_blocks_per_sm(PASS_FUSED_OWN, ctx->block, ctx->smem_cap)
+                                     : split32::pass_blocks_per_sm(PASS_FUSED_OWN, ctx->block, ctx->smem_cap);
+    const int bps_walls = is_fp64(ctx) ? fp64::pass_walls_blocks_per_sm() : split32::pass_walls_blocks_per_sm();
+    if (bps <= 0 || bps_own <= 0 || bps_walls <= 0)
+        return fail(ctx, DSMC_ERR_CUDA, "cell pass cannot be resident (shared memory)");
     const int bps_in = is_fp64(ctx) ? fp64::pass_blocks_per_sm(PASS_INPLACE, ctx->block, ctx->smem_cap)
                                     : split32::pass_blocks_per_sm(PASS_INPLACE, ctx->block, ctx->smem_cap);
     const int bps_so = is_fp64(ctx) ? fp64::pass_blocks_per_sm(PASS_SORT, ctx->block, ctx->smem_cap)
                                     : split32::pass_blocks_per_sm(PASS_SORT, ctx->block, ctx->smem_cap);
     if (bps_in <= 0 || bps_so <= 0) return fail(ctx, DSMC_ERR_CUDA, "stage passes cannot be resident (shared memory)");
     ctx->grid = bps * ctx->num_sms;
+    ctx->walls_grid = bps_walls * ctx->num_sms;
+    ctx->own_flights = pass_owns_flights(ctx, total);
     apply_launch_shape(ctx);
     Status st;
     cudaError_t e;
@@ -490,8 +516,9 @@ int launch(dsmc_ctx *ctx, int mode, int do_collide, int do_move, int do_sample, 
     } else {
         P.top_only = 1;
         if (mode != PASS_INPLACE) ctx->sorted = false;  // the generic passes fill top segments only
-        e = is_fp64(ctx) ? fp64::launch_pass(mode, P, ctx->grid, ctx->block, ctx->stream)
-                         : split32::launch_pass(mode, P, ctx->grid, ctx->block, ctx->stream);
+        if (mode == PASS_FUSED && ctx->own_flights) mode = PASS_FUSED_OWN;
+        e = is_fp64(ctx) ? fp64::launch_pass(mode, P, ctx->grid, ctx->walls_grid, ctx->block, ctx->stream)
+                         : split32::launch_pass(mode, P, ctx->grid, ctx->walls_grid, ctx->block, ctx->stream);
     }
     CK(e);
     // a re-binning pass rotates the occupancy sets
@@ -1967,8 +1994,11 @@ int dsmc_pass_launches(dsmc_ctx *ctx, int *per_step, int *per_sample) {
     if (!ctx) return DSMC_ERR_ARG;
     const bool pipe = ctx->use_pipelined && ctx->fused_grids[1] > 0;
     // collide_cells, move_cells, place_movers and, for listed flights,
-    // place_walls; sample_cells.  The generic pass: its cells, then its wall flights
-    if (per_step) *per_step = !pipe ? 2 : split32::own_walls(ctx->num_cells, any_cl(ctx), ctx->fused_grids) ? 3 : 4;
+    // place_walls; sample_cells.  The generic pass: its cells, then its wall
+    // flights if it lists them
+    if (per_step)
+        *per_step = pipe ? (split32::own_walls(ctx->num_cells, any_cl(ctx), ctx->fused_grids) ? 3 : 4)
+                         : (ctx->own_flights ? 1 : 2);
     if (per_sample) *per_sample = pipe ? 1 : 0;
     return DSMC_OK;
 }

@@ -23,7 +23,7 @@
 
 namespace dsmc {
 
-enum PassMode { MODE_FUSED = 0, MODE_INPLACE = 1, MODE_SORT = 2 };
+enum PassMode { MODE_FUSED = 0, MODE_INPLACE = 1, MODE_SORT = 2, MODE_FUSED_OWN = 3 };
 
 __device__ __forceinline__ float one_minus_ulp() { return __int_as_float(0x3f7fffff); }
 
@@ -1429,7 +1429,8 @@ __device__ __forceinline__ void end_pass(const PassParams &P) {
 
 // The cell pass.  MODE_FUSED (the whole step) moves the flights that end in an
 // empty voxel and lists the others, a few in a thousand, for
-// pass_walls_kernel: with the general mover inline one lane's reflections kept
+// pass_walls_kernel (MODE_FUSED_OWN, for few cells, moves them too: the rule is
+// api.cu's pass_owns_flights): with the general mover inline one lane's reflections kept
 // its warp's other cells waiting, and the kernel ran at half the resident
 // warps.  Members are staged and ranked only in cells that collide or sample,
 // and the next cell's header is loaded ahead.  At 3.9e5 particles in fp64 a step
@@ -1583,7 +1584,7 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
                 if (a == g.active_begin) atomicAdd(&P.tally[sys].samples, 1ull);
             }
         }
-        if (MODE == MODE_FUSED || MODE == MODE_SORT) {
+        if (MODE != MODE_INPLACE) {
             // this pass writes only top slots; clear the set the pass after next fills
             if (lane == 0) {
                 P.cells.bot[P.cclear][a] = 0;
@@ -1673,7 +1674,7 @@ __global__ void __launch_bounds__(256) pass_kernel(PassParams P) {
         nt = next_nt;
     }
     if (wt.sys >= 0) flush_tally(P, wt, lane);
-    if (MODE != MODE_FUSED) end_pass(P);  // a fused pass ends with its wall flights
+    if (MODE != MODE_FUSED) end_pass(P);  // that pass ends with its wall flights
 }
 
 // The general mover for the wall flights that a fused pass listed, then their

@@ -10,8 +10,10 @@ namespace dsmc {
 
 #define DSMC_DECLARE_LAUNCHERS(NS)                                                                              \
     namespace NS {                                                                                              \
-    cudaError_t launch_pass(int mode, const PassParams &P, int grid, int block, cudaStream_t st);               \
+    /* walls_grid: of the wall flights that a fused pass lists */                                               \
+    cudaError_t launch_pass(int mode, const PassParams &P, int grid, int walls_grid, int block, cudaStream_t st); \
     int pass_blocks_per_sm(int mode, int block, int smem_cap);                                                  \
+    int pass_walls_blocks_per_sm();                                                                             \
     size_t record_bytes();                                                                                      \
     cudaError_t launch_from_fp64(const SysDev *sys, int s, const double *r, const double *v, uint32_t id_base, \
                                  long long n, void *A, void *B, int *key, unsigned *hist, unsigned *err,        \
@@ -85,6 +87,6 @@ cudaError_t launch_cells_out(const int4 *meta, const unsigned *bot, const unsign
                              int C, double *out, cudaStream_t st);
 
 // Pass modes (engine.cuh PassMode).
-enum { PASS_FUSED = 0, PASS_INPLACE = 1, PASS_SORT = 2 };
+enum { PASS_FUSED = 0, PASS_INPLACE = 1, PASS_SORT = 2, PASS_FUSED_OWN = 3 };
 
 }  // namespace dsmc

@@ -326,25 +326,17 @@ __global__ void k_cell_energy(const CellArrays cells, const ParticleArrays parts
 // ---- launchers --------------------------------------------------------------
 static size_t stage_bytes(int cap) { return WarpStage<Prec>::bytes(cap); }
 
-// The wall flights of a fused pass: a grid of the most resident blocks.
-static cudaError_t launch_pass_walls(const PassParams &P, cudaStream_t st) {
-    int dev = 0, sms = 0, nb = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pass_walls_kernel<Prec>, 32 * G_WARPS, 0);
-    if (e != cudaSuccess) return e;
-    pass_walls_kernel<Prec><<<std::max(1, nb * sms), 32 * G_WARPS, 0, st>>>(P);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pass(int mode, const PassParams &P, int grid, int block, cudaStream_t st) {
+cudaError_t launch_pass(int mode, const PassParams &P, int grid, int walls_grid, int block, cudaStream_t st) {
     const size_t smem = stage_bytes(P.smem_cap) * (block / 32);
     switch (mode) {
+        case MODE_FUSED_OWN:
+            pass_kernel<Prec, MODE_FUSED_OWN><<<grid, block, smem, st>>>(P);
+            break;
         case MODE_FUSED:
             pass_kernel<Prec, MODE_FUSED><<<grid, block, smem, st>>>(P);
             if (cudaError_t e = cudaGetLastError()) return e;
-            return launch_pass_walls(P, st);
+            pass_walls_kernel<Prec><<<walls_grid, 32 * G_WARPS, 0, st>>>(P);
+            break;
         case MODE_INPLACE:
             pass_kernel<Prec, MODE_INPLACE><<<grid, block, smem, st>>>(P);
             break;
@@ -374,10 +366,13 @@ template <class K> static int blocks_per_sm(K kernel, int block, size_t smem) {
 
 int pass_blocks_per_sm(int mode, int block, int smem_cap) {
     const size_t smem = stage_bytes(smem_cap) * (block / 32);
+    if (mode == MODE_FUSED_OWN) return blocks_per_sm(pass_kernel<Prec, MODE_FUSED_OWN>, block, smem);
     if (mode == MODE_FUSED) return blocks_per_sm(pass_kernel<Prec, MODE_FUSED>, block, smem);
     if (mode == MODE_INPLACE) return blocks_per_sm(pass_kernel<Prec, MODE_INPLACE>, block, smem);
     return blocks_per_sm(pass_kernel<Prec, MODE_SORT>, block, smem);
 }
+
+int pass_walls_blocks_per_sm() { return blocks_per_sm(pass_walls_kernel<Prec>, 32 * G_WARPS, 0); }
 
 size_t record_bytes() { return sizeof(RecA) + sizeof(RecB); }
 

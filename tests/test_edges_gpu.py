@@ -275,3 +275,23 @@ def test_steps_after_new_states_of_other_sizes():
         out.append(S.get_particles())
     for r1, v1 in out[1:]:
         assert np.array_equal(r1, out[0][0]) and np.array_equal(v1, out[0][1])
+
+
+@pytest.mark.parametrize("n,cells,per_cell,model,launches", [
+    (8, 4, 20, 0, 1), (24, 12, 20, 1, 1), (32, 16, 20, 1, 2), (32, 8, 60, 1, 2), (32, 16, 20, 2, 1), (48, 24, 20, 2, 2),
+    (40, 20, 20, 0, 1), (64, 32, 20, 0, 2)])
+def test_generic_pass_moves_or_lists_its_wall_flights(n, cells, per_cell, model, launches):
+    """fp64 steps on both sides of the rule by which the cell pass moves its
+    wall flights itself (one kernel a step) or lists them (two), for each wall model
+    and for cells of more than 32 members: bit for bit the stage kernels."""
+    w = Workload("walls", n=n, radius_voxels=3.0, porosity=0.6, geometry_seed=5, cells=cells,
+                 atoms_per_molecule=simulators_per_cell_weight(2.5e24, 0.1, n // cells, per_cell), dt_si=2e-11)
+    g = w.geometry()
+    s = w.settings(rng_seed=11, statistics_interval=2)
+    s.surface_model = model
+    if model == 2:
+        s.alpha_n, s.alpha_t = 0.8, 0.8
+    A, B = System(s, g, precision=capi.PREC_FP64), System(s, g, precision=capi.PREC_FP64)
+    assert A.ctx.pass_launches() == (launches, 0)
+    run_both(A, B, 5)
+    assert A.tallies().wall_collisions > 0
