@@ -145,6 +145,11 @@ struct dsmc_ctx {
     int grid = 0;
     int walls_grid = 0;          // of the wall flights that the cell pass lists
     bool own_flights = false;    // the cell pass moves them itself instead
+    // Resident blocks per SM of the generic passes with smem_cap slots per
+    // warp, asked of the driver again only for another cap.
+    struct {
+        int smem_cap = 0, fused = 0, own = 0, walls = 0, inplace = 0, sort = 0;
+    } resident;
     int fused_grids[5] = {0, 0, 0, 0, 0};  // production pass (collide, move, place, walls, sample); 0 = not usable
     int fused_max_bps[5] = {0, 0, 0, 0, 0};  // the most resident blocks per SM of each at the current ring
     // launch tuning (dsmc_tuning_set): blocks per SM of each production
@@ -341,20 +346,25 @@ int relayout(dsmc_ctx *ctx, long long total) {
         CK(e);
     }
     // Launch shape of the cell pass: a persistent grid at full occupancy.
-    const int bps = is_fp64(ctx) ? fp64::pass_blocks_per_sm(PASS_FUSED, ctx->block, ctx->smem_cap)
-                                 : split32::pass_blocks_per_sm(PASS_FUSED, ctx->block, ctx->smem_cap);
-    const int bps_own = is_fp64(ctx) ? fp64::pass_blocks_per_sm(PASS_FUSED_OWN, ctx->block, ctx->smem_cap)
-                                     : split32::pass_blocks_per_sm(PASS_FUSED_OWN, ctx->block, ctx->smem_cap);
-    const int bps_walls = is_fp64(ctx) ? fp64::pass_walls_blocks_per_sm() : split32::pass_walls_blocks_per_sm();
-    if (bps <= 0 || bps_own <= 0 || bps_walls <= 0)
+    auto &res = ctx->resident;
+    if (res.smem_cap != ctx->smem_cap) {
+        auto blocks = [&](int mode) {
+            return is_fp64(ctx) ? fp64::pass_blocks_per_sm(mode, ctx->block, ctx->smem_cap)
+                                : split32::pass_blocks_per_sm(mode, ctx->block, ctx->smem_cap);
+        };
+        res.fused = blocks(PASS_FUSED);
+        res.own = blocks(PASS_FUSED_OWN);
+        res.walls = is_fp64(ctx) ? fp64::pass_walls_blocks_per_sm() : split32::pass_walls_blocks_per_sm();
+        res.inplace = blocks(PASS_INPLACE);
+        res.sort = blocks(PASS_SORT);
+        res.smem_cap = ctx->smem_cap;
+    }
+    if (res.fused <= 0 || res.own <= 0 || res.walls <= 0)
         return fail(ctx, DSMC_ERR_CUDA, "cell pass cannot be resident (shared memory)");
-    const int bps_in = is_fp64(ctx) ? fp64::pass_blocks_per_sm(PASS_INPLACE, ctx->block, ctx->smem_cap)
-                                    : split32::pass_blocks_per_sm(PASS_INPLACE, ctx->block, ctx->smem_cap);
-    const int bps_so = is_fp64(ctx) ? fp64::pass_blocks_per_sm(PASS_SORT, ctx->block, ctx->smem_cap)
-                                    : split32::pass_blocks_per_sm(PASS_SORT, ctx->block, ctx->smem_cap);
-    if (bps_in <= 0 || bps_so <= 0) return fail(ctx, DSMC_ERR_CUDA, "stage passes cannot be resident (shared memory)");
-    ctx->grid = bps * ctx->num_sms;
-    ctx->walls_grid = bps_walls * ctx->num_sms;
+    if (res.inplace <= 0 || res.sort <= 0)
+        return fail(ctx, DSMC_ERR_CUDA, "stage passes cannot be resident (shared memory)");
+    ctx->grid = res.fused * ctx->num_sms;
+    ctx->walls_grid = res.walls * ctx->num_sms;
     ctx->own_flights = pass_owns_flights(ctx, total);
     apply_launch_shape(ctx);
     Status st;
@@ -1026,9 +1036,9 @@ int dsmc_system_info_get(dsmc_ctx *ctx, int sys_id, dsmc_system_info *info) {
 
 // The stream that state is copied on while ctx->stream converts.
 static cudaError_t io_stream_ready(dsmc_ctx *ctx) {
-    if (ctx->io_stream) return cudaSuccess;
-    cudaError_t e = cudaStreamCreateWithFlags(&ctx->io_stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->io_event, cudaEventDisableTiming);
+    cudaError_t e = cudaSuccess;
+    if (!ctx->io_stream) e = cudaStreamCreateWithFlags(&ctx->io_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess && !ctx->io_event) e = cudaEventCreateWithFlags(&ctx->io_event, cudaEventDisableTiming);
     return e;
 }
 
@@ -1055,20 +1065,24 @@ static int place_particles(dsmc_ctx *ctx, int sys_id, long long n, const double 
         CK(ctx->io_v.ensure(3 * std::max<long long>(n, 1)));
         if (n) {
             // by ranges: one is converted while the next is copied (the whole call at
-            // 3.9e6 particles 4.39 -> 4.2 ms, the copies alone 3.44)
-            CK(io_stream_ready(ctx));
-            CK(cudaEventRecord(ctx->io_event, ctx->stream));  // earlier work on io_r and io_v
-            CK(cudaStreamWaitEvent(ctx->io_stream, ctx->io_event, 0));
+            // 3.9e6 particles 4.39 -> 4.2 ms, the copies alone 3.44); a single range
+            // needs no other stream
             const int pieces = io_pieces(n);
             e = cudaSuccess;
+            if (pieces > 1) {
+                CK(io_stream_ready(ctx));
+                CK(cudaEventRecord(ctx->io_event, ctx->stream));  // earlier work on io_r and io_v
+                CK(cudaStreamWaitEvent(ctx->io_stream, ctx->io_event, 0));
+            }
+            const cudaStream_t up = pieces > 1 ? ctx->io_stream : ctx->stream;
             for (int k = 0; k < pieces && e == cudaSuccess; ++k) {
                 const long long lo = n * k / pieces, m = n * (k + 1) / pieces - lo;
                 double *dr = ctx->io_r.p + 3 * lo, *dv = ctx->io_v.p + 3 * lo;
-                e = cudaMemcpyAsync(dr, r + 3 * lo, 3 * m * sizeof(double), cudaMemcpyHostToDevice, ctx->io_stream);
+                e = cudaMemcpyAsync(dr, r + 3 * lo, 3 * m * sizeof(double), cudaMemcpyHostToDevice, up);
                 if (e == cudaSuccess)
-                    e = cudaMemcpyAsync(dv, v + 3 * lo, 3 * m * sizeof(double), cudaMemcpyHostToDevice, ctx->io_stream);
-                if (e == cudaSuccess) e = cudaEventRecord(ctx->io_event, ctx->io_stream);
-                if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, ctx->io_event, 0);
+                    e = cudaMemcpyAsync(dv, v + 3 * lo, 3 * m * sizeof(double), cudaMemcpyHostToDevice, up);
+                if (e == cudaSuccess && pieces > 1) e = cudaEventRecord(ctx->io_event, up);
+                if (e == cudaSuccess && pieces > 1) e = cudaStreamWaitEvent(ctx->stream, ctx->io_event, 0);
                 if (e == cudaSuccess)
                     e = is_fp64(ctx) ? fp64::launch_from_fp64(ctx->sys_dev.p, sys_id, dr, dv, (uint32_t)lo, m,
                                                               A + lo * half, B + lo * half, key + lo, ctx->hist.p,
@@ -1077,8 +1091,9 @@ static int place_particles(dsmc_ctx *ctx, int sys_id, long long n, const double 
                                                                  A + lo * half, B + lo * half, key + lo, ctx->hist.p,
                                                                  &ctx->status.p->error, ctx->stream);
             }
-            // the copies are done with the caller's buffers before this returns
-            const cudaError_t e1 = cudaStreamSynchronize(ctx->io_stream);
+            // the copies are done with the caller's buffers before this returns (a
+            // single range's by the read of the status below)
+            const cudaError_t e1 = pieces > 1 || e != cudaSuccess ? cudaStreamSynchronize(up) : cudaSuccess;
             CK(e);
             CK(e1);
         }
