@@ -905,11 +905,12 @@ template <int CIB, bool PAIR> cudaError_t launch_wgrad_plane(const WgradArgs &w,
     PlaneWgradArgs a{w.dy.p, w.dy.cs, w.dy.coff, w.x.p, w.x.cs, w.x.coff, w.dw, w.cin, ci0, ciblocks,
                      0, 0, w.S, w.lg, 0, 0, 1, (int)(w.rows >> (3 * w.lg))};
     const int sms = sm_count();
-    // an accumulator takes as many additions of 16 voxels as wgrad_kernel's
-    // would: more would cost precision, fewer cost flushes
+    // an accumulator takes at most as many additions of 16 voxels as
+    // wgrad_kernel's would: more would cost precision, fewer cost flushes
     const long long adds = wgrad_voxels(w) / 16;
     // the widest block of output channels, unless a CTA would then see far
-    // fewer additions where they are many and the fp32 sums' rounding counts
+    // fewer additions where they are many: the result would move from
+    // wgrad_kernel's by more than it may (kWgradPlaneAdds), though towards the exact sum
     for (a.cob = 48; a.cob > 16; a.cob -= 16)
         if (w.cout % a.cob == 0 &&
             (adds < 1500 || w.rows / 16 / std::max(1, sms / (ciblocks * (w.cout / a.cob))) >= adds * 3 / 4))
@@ -922,10 +923,11 @@ template <int CIB, bool PAIR> cudaError_t launch_wgrad_plane(const WgradArgs &w,
     a.lgL = std::min(4, w.lg);
     while (a.lgL > 1 && (tiles << (w.lg - a.lgL)) < 2 * ctas) --a.lgL;
     a.items = (int)(tiles << (w.lg - a.lgL));
-    // (whole items, up to a sixteenth more: at 64^3 x 8 and 16 channels 896 for
-    // 885; 768 left the trained network's gradients 1.8e-5 from wgrad_kernel's, 896
-    // 1.3e-5, at no larger an error)
-    a.flush = (int)std::max(1ll, (adds + adds / 16) / (8 << a.lgL));
+    // whole items of 8 additions a plane (a sixteenth more may round up to one), cut to that limit: at 64^3 x 8
+    // and 16 channels 7 items of 16 planes to 111 planes, 888 additions. (With 6 items, 768, the trained
+    // network's gradients lay 1.8e-5 from wgrad_kernel's; with 7 1.3e-5, but at a larger error on some inputs.)
+    const long long whole = std::max(1ll, (adds + adds / 16) / (8 << a.lgL)) << a.lgL;
+    a.flush = (int)std::min(whole, adds / 8);
     cudaError_t e = cudaFuncSetAttribute(wgrad_plane_kernel<CIB, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::smem(48));
     if (e != cudaSuccess) return e;
     const int grid = (int)std::min<long long>(a.items, ctas) * groups;
@@ -935,12 +937,13 @@ template <int CIB, bool PAIR> cudaError_t launch_wgrad_plane(const WgradArgs &w,
 
 // Additions per accumulator up to which the plane kernel takes a weight
 // gradient. The tensor core's fp32 sums truncate: one of n additions is off by about
-// 1.3e-8 n of its size, more or less by the order of the voxels. Up to here the
-// two kernels agree within 2e-5 (64^3 x 8: 6e-6 at 880 additions, 1.2e-5 at 1550,
-// 2.7e-5 at 3100, 4.1e-5 at 4650, each nearer to the exact sum than wgrad_kernel);
-// longer sums, of 48 output channels and more over a million voxels, keep
-// wgrad_kernel's order and bits, at its time (64^3 x 8, 32 -> 64 channels: 4070 us
-// against 391).
+// 1.3e-8 n of its size, so a kernel of shorter accumulators moves the result by
+// as much as wgrad_kernel is off. Up to here the results stay within 2e-5 of
+// wgrad_kernel's (64^3 x 8: 6e-6 at 880 additions, 1.3e-5 at 1550); beyond, at
+// 2.7e-5 for 3100 and 4.1e-5 for 4650, they would leave the 2e-5 that fp32
+// results are held to from one version to the next. That is the only reason: the plane
+// kernel's are the nearer ones to the exact sums there too, and wgrad_kernel takes ten
+// times as long (64^3 x 8, 32 -> 64 channels 4070 us against 391).
 constexpr long long kWgradPlaneAdds = 1800;
 
 template <bool PAIR> cudaError_t launch_wgrad_planes(const WgradArgs &w, cudaStream_t st) {

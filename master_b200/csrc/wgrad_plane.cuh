@@ -26,7 +26,7 @@ struct PlaneWgradArgs {
     int coblocks;        // cout / cob
     int S, lg, lgL;
     int items;
-    int flush;           // items between two flushes of the accumulators
+    int flush;           // planes between two flushes of the accumulators
     int batch;
 };
 
@@ -55,7 +55,7 @@ template <int CIB, bool PAIR> struct PlaneWgradShape {
 // the next tap's chunks follow at the same distance and M = 64 (CIB = 16) or
 // 128 holds the 3 x CIB of them (the rest is not used); B's columns are three planes of dY (the
 // axis-0 taps) x cob; the axis-2 taps are three start addresses of A with an
-// accumulator each.  The accumulators are added to dW every `flush` items.
+// accumulator each.  The accumulators are added to dW every `flush` planes.
 template <int CIB, bool PAIR>
 __global__ void __launch_bounds__(kPlaneThreads, 1) wgrad_plane_kernel(const __grid_constant__ PlaneWgradArgs a) {
     using Sh = PlaneWgradShape<CIB, PAIR>;
@@ -166,12 +166,11 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) wgrad_plane_kernel(const __g
         auto idesc = [&](int planes) { return tc05::idesc_bf16_f32(Sh::kM, planes * cob, 1, 1); };
         int s = 0;          // slot of the newest plane waited for
         uint32_t ph = 0;
-        int acc = 0, flushes = 0, since = 0;  // accumulator; flushes so far; items since the last
+        int acc = 0, flushes = 0, since = 0;  // accumulator; flushes so far; planes since the last
         uint32_t aph = 0;
         bool ok = true;
         auto prev = [&](int q, int d) { return q >= d ? q - d : q - d + Sh::kSlots; };
         for (int item = first; item < a.items; item += stride) {
-            const bool last = since + 1 == a.flush || item + stride >= a.items;
             for (int u = 0; u < L + 2; ++u) {
                 if (!(u & 1)) {
                     ok &= tc05::mbar_wait(&full[s >> 1], ph);
@@ -180,7 +179,8 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) wgrad_plane_kernel(const __g
                 }
                 if (u >= 2) {
                     // plane u - 1 of X against planes u - 2 .. u of dY
-                    const bool start = u == 2 && since == 0;
+                    const bool start = since == 0;
+                    const bool last = ++since == a.flush || (u == L + 1 && item + stride >= a.items);
                     if (start && flushes >= nacc) ok &= tc05::mbar_wait(&accfree[acc], aph ^ 1u);
                     tc05::fence_after_sync();
                     const int y0 = prev(s, 2), xs = prev(s, 1);
@@ -203,23 +203,20 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) wgrad_plane_kernel(const __g
                     }
                     // (L is even: planes go in pairs) the pair u - 3, u - 2 has served its last step
                     if (u & 1) tc05::mma_commit_warp(lead, &empty[prev(s, 3) >> 1]);
-                    if (u == L + 1) {
-                        tc05::mma_commit_warp(lead, &empty[s >> 1]);
-                        if (last) tc05::mma_commit_warp(lead, &accfull[acc]);
+                    if (u == L + 1) tc05::mma_commit_warp(lead, &empty[s >> 1]);
+                    if (last) {
+                        tc05::mma_commit_warp(lead, &accfull[acc]);
+                        since = 0;
+                        ++flushes;
+                        if (++acc == nacc) {
+                            acc = 0;
+                            aph ^= 1u;
+                        }
                     }
                 }
                 if (++s == Sh::kSlots) {
                     s = 0;
                     ph ^= 1u;
-                }
-            }
-            ++since;
-            if (last) {
-                since = 0;
-                ++flushes;
-                if (++acc == nacc) {
-                    acc = 0;
-                    aph ^= 1u;
                 }
             }
         }
@@ -234,10 +231,8 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) wgrad_plane_kernel(const __g
         int acc = 0;
         uint32_t aph = 0;
         bool ok = true;
-        int since = 0;
-        for (int item = first; item < a.items; item += stride) {
-            if (++since < a.flush && item + stride < a.items) continue;
-            since = 0;
+        // this CTA's planes, `flush` at a time
+        for (long long planes = (long long)((a.items - first + stride - 1) / stride) << a.lgL; planes > 0; planes -= a.flush) {
             ok &= tc05::mbar_wait(&accfull[acc], aph);
             tc05::fence_after_sync();
             const uint32_t col = tmem + ((uint32_t)(quarter * 32) << 16) + acc * ncol;

@@ -456,3 +456,32 @@ def test_training_on_one_batch_lowers_the_loss():
     sync_ok()
     assert np.isfinite(losses).all()
     assert losses[-1] < 0.2 * losses[0], losses[::10]
+
+
+@pytest.mark.parametrize("B,S,ci,co", [(50, 16, 96, 16), (7, 32, 96, 16), (49, 16, 48, 16), (41, 8, 96, 16), (8, 64, 16, 16)])
+def test_wgrad_accumulators_take_no_more_additions_than_the_gathering_kernels(B, S, ci, co):
+    """Positive data: every addition of an accumulator truncates by half an ulp
+    on average and nothing cancels, so the sums' mean shortfall is proportional
+    to the additions per accumulator. The same values as many boxes of edge
+    4, which the gathering kernel takes, are split into accumulators by the same
+    rule; the plane kernels' shortfall is at most that one (a tenth is left for
+    the accumulators that end early in either). The lengths cover a whole item of planes longer
+    than the limit (88, 100 and 44 additions) and limits of several items."""
+    g = torch.Generator(device=DEV).manual_seed(S * B)
+    rows = B * S ** 3
+    x = (torch.rand((rows, ci), generator=g, device=DEV) + 0.5).to(torch.bfloat16)
+    dy = (torch.rand((rows, co), generator=g, device=DEV) + 0.5).to(torch.bfloat16)
+    short = []
+    for b, s in ((B, S), (rows // 64, 4)):
+        dw = torch.zeros((co, 27, ci), device=DEV)
+        capi.check(lib().dsmc_sg_conv3_wgrad(stream(), b, s, P(dy), co, 0, co, P(x), ci, 0, ci, P(dw)))
+        sync_ok()
+        total, n = 0.0, 0
+        for t in (0, 5, 13, 22):
+            d = (t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1)
+            xs = torch.roll(x.reshape(b, s, s, s, ci), tuple(-o for o in d), (1, 2, 3)).reshape(-1, ci)
+            ref = sum(dy[k:k + 65536].double().T @ xs[k:k + 65536].double() for k in range(0, rows, 65536))
+            total += ((ref - dw[:, t].double()) / ref).sum().item()
+            n += ref.numel()
+        short.append(total / n)
+    assert 0.0 < short[0] <= 1.1 * short[1], short
