@@ -946,7 +946,16 @@ template <int CIB, bool PAIR> cudaError_t launch_wgrad_plane(const WgradArgs &w,
 // times as long (64^3 x 8, 32 -> 64 channels 4070 us against 391).
 constexpr long long kWgradPlaneAdds = 1800;
 
+// Blocks of 32 input channels, and of 16 for the rest in a launch of its own.
+// Where a launch is mostly its start and end, 48 channels go as three blocks of
+// 16 in one: us for 16 / 48 / 96 output channels as 32 + 16 and so, 8^3 x 1 13.3 / 21 / 22
+// and 6.0 / 10.4 / 10.5 (wgrad_kernel 14.6 / 15.5 / 15.1), 16^3 x 8 15.6 / 25 / 30
+// and 10 / 21 / 28, 32^3 x 3 (9.8e4 voxels) 23 / 35 / 49 and 17 / 32 / 49, but
+// 32^3 x 8 (2.6e5) 38 / 58 / 94 and 37 / 65 / 114.
+constexpr long long kSplit48Rows = 1 << 17;
+
 template <bool PAIR> cudaError_t launch_wgrad_planes(const WgradArgs &w, cudaStream_t st) {
+    if (w.cin == 48 && w.rows <= kSplit48Rows) return launch_wgrad_plane<16, PAIR>(w, 0, 3, st);
     const int b32 = w.cin / 32;
     cudaError_t e = b32 ? launch_wgrad_plane<32, PAIR>(w, 0, b32, st) : cudaSuccess;
     if (e == cudaSuccess && w.cin % 32) e = launch_wgrad_plane<16, PAIR>(w, 32 * b32, 1, st);

@@ -485,3 +485,24 @@ def test_wgrad_accumulators_take_no_more_additions_than_the_gathering_kernels(B,
             n += ref.numel()
         short.append(total / n)
     assert 0.0 < short[0] <= 1.1 * short[1], short
+
+
+@pytest.mark.parametrize("B,S,co", [(1, 8, 48), (3, 32, 16), (4, 32, 96), (5, 32, 16), (65, 16, 32)])
+def test_wgrad_of_48_input_channels_in_one_launch_and_two(B, S, co):
+    """Three blocks of 16 input channels in one launch (up to 131072 voxels) and
+    blocks of 32 and 16 in two (above), the largest one-launch size included,
+    through views.  Truncating sums of at most 304 additions (x 2^-24) and
+    as many partial sums added in fp32: 3e-5."""
+    ci = 48
+    g = torch.Generator(device=DEV).manual_seed(B + S)
+    rows = B * S ** 3
+    x = torch.relu(torch.randn((B, S, S, S, ci + 16), generator=g, device=DEV)).to(torch.bfloat16)
+    dy = torch.randn((B, S, S, S, co + 8), generator=g, device=DEV).to(torch.bfloat16)
+    dw = torch.ones((co, 27, ci), device=DEV)  # accumulated
+    capi.check(lib().dsmc_sg_conv3_wgrad(stream(), B, S, P(dy), co + 8, 8, co, P(x), ci + 16, 16, ci, P(dw)))
+    sync_ok()
+    dyd = dy[..., 8:].reshape(rows, co).double()
+    for t in range(27):
+        d = (t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1)
+        ref = 1.0 + dyd.T @ torch.roll(x[..., 16:], tuple(-o for o in d), (1, 2, 3)).reshape(rows, ci).double()
+        assert ((dw[:, t].double() - ref).norm() / ref.norm()).item() <= 3e-5, t
