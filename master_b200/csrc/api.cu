@@ -279,20 +279,29 @@ void apply_launch_shape(dsmc_ctx *ctx) {
 
 // Whether the cell pass moves its wall flights where it finds them, which
 // saves a launch and the list's turn-around but has a warp's flights follow one
-// another: while each warp makes few turns (32 members of a cell; a quarter
-// above the mean, where cells of more than 32 are many), fewer with walls that
-// leave flights longer.  us per step in fp64, own / listed: thermal walls
-// 336 cells (4.4e3 particles) 23 / 34, 2944 36 / 47, 5920 49 / 55, 10256 (five
-// turns) 64 / 65 and with twice the particles (ten) 91 / 82, 16152 85 / 76, 24128 111 / 92; Cercignani-Lampis 336 136 / 147,
-// 4336 (two turns) 253 / 260, 10256 307 / 291; specular 1176 69 / 86, 1960 (one turn) 88 / 91,
-// 2944 130 / 99, 10256 267 / 123.
+// another: while a warp takes few cells, or makes few turns (32 members of a
+// cell; a quarter above the mean, where cells of more are many), fewer with walls
+// that leave flights longer.  Measured, us per step own / listed (warps: 2368):
+//   thermal, fp64: 336 cells 23 / 34, 2944 36 / 47, 5920 (three cells a warp) 49 / 55,
+//     10256 64 / 65 and with twice the particles 91 / 82, 24128 111 / 92; of 190 particles
+//     each 1728 cells 130 / 148, 2744 179 / 200, of 95 7576 172 / 158; split, of 238 512
+//     cells 97 / 124, of 180 5832 204 / 209, 8000 264 / 245
+//   Cercignani-Lampis, fp64: 336 136 / 147, 4336 (two turns) 250 / 252, 10256 307 / 291, of 95
+//     particles 3856 486 / 451; split, of 238 512 cells 222 / 267, of 180 4096 (two cells a
+//     warp) 340 / 349, 8000 533 / 488
+//   specular, fp64: 1176 69 / 86, 1960 (one turn) 88 / 91, 2944 130 / 99, 10256 267 / 123
 bool pass_owns_flights(const dsmc_ctx *ctx, long long total) {
     const long long warps = (long long)ctx->grid * (ctx->block / 32), C = std::max(ctx->num_cells, 1);
-    const long long turns = ((C + warps - 1) / warps) * ((total + total / 4 + 32 * C - 1) / (32 * C));
-    int most = 5;
-    for (const auto &s : ctx->systems)
-        most = std::min(most, s->dev.wall_model == DSMC_WALL_SPECULAR ? 1 : s->dev.wall_model == DSMC_WALL_CL ? 2 : 5);
-    return turns <= most;
+    const long long cells = (C + warps - 1) / warps;  // of a warp
+    const long long turns = cells * ((total + total / 4 + 32 * C - 1) / (32 * C));
+    int most_cells = 3, most_turns = 4;
+    for (const auto &s : ctx->systems) {
+        if (s->dev.wall_model == DSMC_WALL_THERMAL) continue;
+        const bool cl = s->dev.wall_model == DSMC_WALL_CL;
+        most_cells = std::min(most_cells, cl && !is_fp64(ctx) ? 2 : 0);
+        most_turns = std::min(most_turns, cl ? 2 : 1);
+    }
+    return cells <= most_cells || turns <= most_turns;
 }
 
 int relayout(dsmc_ctx *ctx, long long total) {

@@ -295,3 +295,22 @@ def test_generic_pass_moves_or_lists_its_wall_flights(n, cells, per_cell, model,
     assert A.ctx.pass_launches() == (launches, 0)
     run_both(A, B, 5)
     assert A.tallies().wall_collisions > 0
+
+
+@pytest.mark.parametrize("n,per_cell,model,launches", [(32, 400, 0, 1), (64, 400, 2, 1), (32, 400, 1, 2), (160, 300, 0, 2)])
+def test_generic_pass_of_large_cells_moves_or_lists_its_wall_flights(n, per_cell, model, launches):
+    """Cells of more particles than the production pass stages (the generic pass in
+    split precision), on both sides of the same rule: bit for bit the stage
+    kernels."""
+    w = Workload("walls", n=n, radius_voxels=4.0, porosity=0.6, geometry_seed=1, cells=n // 8,
+                 atoms_per_molecule=simulators_per_cell_weight(2.5e24, 0.1, 8, per_cell))
+    g = w.geometry()
+    s = w.settings(rng_seed=11, statistics_interval=2)
+    s.surface_model = model
+    if model == 2:
+        s.alpha_n, s.alpha_t = 0.8, 0.8
+    A, B = System(s, g), System(s, g)
+    assert A.ctx.pass_info()["pipelined"] == 0
+    assert A.ctx.pass_launches() == (launches, 0)
+    run_both(A, B, 3)
+    assert A.tallies().wall_collisions > 0
