@@ -161,8 +161,8 @@ struct dsmc_ctx {
     // per-kernel timers of the production pass (dsmc_ctx_set_timing)
     bool timing = false;
     cudaEvent_t tev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    // dsmc_particles_get: positions are copied out on io_stream while the
-    // velocities are converted on `stream`
+    // dsmc_particles_get and _set: a range of ids is copied on io_stream while
+    // another is converted on `stream`
     cudaStream_t io_stream = nullptr;
     cudaEvent_t io_event = nullptr;
     double tms[4] = {0, 0, 0, 0};

@@ -14,7 +14,7 @@
 // (N = 3 x output channels).  The bound is shared memory feeding the MMAs: one
 // of M = 128 and K = 16 takes 34 + N / 4 cycles here (measured for N <= 128;
 // 4 KB of A and 32 N bytes of B at 128 bytes a cycle), so at 16 output
-// channels one of N = 48 does in 46 cycles what three of N = 16 do in 122.
+// channels one of N = 48 does in 46 cycles what three of N = 16 do in 114.
 //
 // Measured (batch 8, back to back), conv3_kernel of surrogate.cu before and
 // this kernel: 64^3 48 -> 16 channels 2479 -> 127 us (0.69 PFLOP/s; 53 us at

@@ -1350,7 +1350,9 @@ __device__ __forceinline__ void end_split_pass(const PassParams &P) {
 // 45.2 and 46.8 us per step against 44.9 at 64^3), which costs the placing of
 // many movers more than a launch and the list's turn-around: us per step, both
 // kernels, list -> own: 64^3 (2e4 cells) 39 -> 28, 128^3 (2e5) 60 -> 49, 160^3
-// (3.5e5) 76 -> 68 in all 226 -> 223, 192^3 (6e5) 92 -> 99, 256^3 162 -> 193.
+// (3.5e5) 76 -> 68 in all 226 -> 223, 192^3 (6e5) 92 -> 99, 256^3 162 -> 193. The
+// rule (four chunks per warp, 3.0e5 cells on 148 SMs) lies below that crossing:
+// 160^3 is listed.
 // Cercignani-Lampis flights are always listed: their warps share the rejection
 // trials, so equal claims matter more (64^3 69 -> 182, 128^3 119 -> 393).
 template <bool OWN>
@@ -1477,9 +1479,9 @@ __global__ void __launch_bounds__(32 * W_WARPS) place_walls_kernel(const __grid_
     int tsys = -1;
     // Warps claim entries from a counter: flights differ widely in length, so
     // a warp that finishes early takes more.  A claim is 32 entries, or fewer
-    // when the list would not fill the grid's warps: a turn of the flights'
-    // state machine runs every state that some lane is in, so a warp of few
-    // lanes finishes its flights sooner.
+    // when the list would not fill the grid's warps: a warp's lanes wait for one
+    // another where their flights part (and, with Cercignani-Lampis walls, take turns
+    // in the state machine), so a warp of few lanes finishes its flights sooner.
     const unsigned nw = gridDim.x * W_WARPS;
     const unsigned claim = min(32u, max(1u, (nwalls + nw - 1u) / nw));
     for (;;) {

@@ -847,10 +847,16 @@ int sm_count() {
 constexpr int kPlaneEdge = 16;
 
 // Output channels per CTA and planes per item of conv_plane_kernel: the split
-// with the least estimated time, in cycles of an SM.  A plane costs the
-// largest of its MMAs (32 cycles to read A, or N / 2), its staged bytes and
-// its epilogue; an item stages two planes more than it writes; every CTA
-// loads its weights once.
+// with the least estimated time, in cycles of an SM.  A plane is taken to cost the
+// largest of its MMAs (32 cycles to read A, or N / 2), its staged bytes (25 a cycle) and
+// its epilogue (16 cycles a channel); an item stages two planes more than it
+// writes and costs 300 cycles to begin; every CTA loads its weights once, 40 bytes a
+// cycle. These are estimates that order the splits, not the kernel's own rates (an MMA of
+// N <= 128 takes 34 + N / 4 cycles): of 414 layers (edges 8 to 64, 16 to 96 channels,
+// one sample to the training batch and beyond) the chosen split is within 4 % of
+// the fastest in 394 and up to 1.5 times it in the others, nearly all with 16 or
+// 32 input channels (32^3 x 20, 16 -> 48: 63 us, 41 with 48 channels a CTA). With 34 + 3/4 nb for the MMAs alone 395 are, but others lose up to 1.3
+// (16^3 x 8, 64 -> 32).
 template <int CIN, bool PAIR> void plane_split(PlaneArgs &a, int cout, long long rows, int sms) {
     const long long tiles = PAIR ? (a.batch + 1) / 2 : rows >> (a.lg + 7);
     double best = 1e300;
